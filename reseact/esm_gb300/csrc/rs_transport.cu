@@ -58,17 +58,14 @@ __device__ __forceinline__ void limit(double a, double& aL, double& aR) {
     else if (-(dA * dA) > dA * a6) aR = 3.0 * a - 2.0 * aL;
   }
 }
-// ---- production-build forms of slope_u / slope_n / limit.  The same slopes, edges and limiter
-// decisions, with the sign tests and the exact power-of-two scalings done on the sign and
-// exponent bits in the integer pipes (FP64 issues at ~2 lanes per SM per clock on this GPU):
+// ---- production-build forms of the slopes: the same slopes, with the sign tests and the exact
+// power-of-two scalings done on the sign and exponent bits in the integer pipes (FP64 issues at
+// ~2 lanes per SM per clock on this GPU):
 //   d1*d0 > 0            <=>  d0, d1 nonzero with equal signs       (unless the product underflows)
 //   0.5*s, 2*m           =    exponent field -1 / +1                 (normal operands)
 //   fmin of magnitudes   =    integer min of the magnitude bits
-// so slopes and the extremum test are bit-identical to the FP forms for normal operands (where a
-// product of differences could underflow, or an operand is subnormal, the FP form decides).  The
-// steepening tests dA*a6 > dA*dA and -(dA*dA) > dA*a6 become sign tests of dA and a6 -+ dA,
-// which can differ from the FP forms only where a6 = +-dA to roundoff -- where the limiter is
-// continuous (the steepened edge equals the unsteepened one), so a face moves by roundoff only.
+// bit-identical to the FP forms for normal operands (where a product of differences could
+// underflow, or an operand is subnormal, the FP form decides).
 // copysign(min(|da|, 2 min(|d0|, |d1|)), da), or 0 where d0, d1 are not nonzero with equal
 // signs, on the 32-bit halves of the bit patterns.  (Written on 64-bit masks of reinterpreted
 // doubles, the same arithmetic was partly emitted as FP64 adds -- three per slope, measured with
@@ -86,63 +83,6 @@ __device__ __forceinline__ double slope_pick32(double d0, double d1, double da, 
                     ((h1 | l1) != 0u);
   return __hiloint2double(live ? (int)hr : 0, live ? (int)lr : 0);
 }
-__device__ __forceinline__ double slope_u_fast(double am, double a, double ap) {
-  const double d0 = a - am, d1 = ap - a;
-  if (prod_may_underflow(d0, d1)) return slope_u(am, a, ap);
-  return slope_pick32(d0, d1, ap - am, true);  // nonzero span where live; |da| = |ap - am| / 2
-}
-__device__ __forceinline__ double slope_n_fast(double am, double a, double ap, double sA, double sB) {
-  const double d0 = a - am, d1 = ap - a;
-  if (prod_may_underflow(d0, d1)) return slope_n(am, a, ap, sA, sB);
-  return slope_pick32(d0, d1, sA * d1 + sB * d0, false);
-}
-// Branch-free: every lane issues the same six FP64 instructions (dA, a6, one steepened edge) and
-// picks its result with integer selects -- with the limiter's data-dependent branches, a warp
-// issued both sides and the FP64 pipe (16 cycles per warp instruction) ran with about half its
-// lanes idle.
-__device__ __forceinline__ void limit_fast(double a, double& aL, double& aR) {
-  if (tiny_operand(a) || tiny_operand(aL) || tiny_operand(aR)) {
-    limit(a, aL, aR);
-    return;
-  }
-  const long long ka = ord_key(a), kl = ord_key(aL), kr = ord_key(aR);
-  // extremum: (aR - a)(a - aL) <= 0
-  const bool flat = !((kr > ka && ka > kl) || (kr < ka && ka < kl));
-  const double dA = aR - aL;
-  const double a6 = 6.0 * (a - 0.5 * (aL + aR));
-  const long long kd = ord_key(dA), k6 = ord_key(a6);
-  // dA (a6 - dA) > 0 and dA (a6 + dA) < 0 as comparisons of a6 with +-dA
-  const bool stl = (kd > 0 && k6 > kd) || (kd < 0 && k6 < kd);             // aL <- 3a - 2aR
-  const bool str = !stl && ((kd > 0 && k6 < -kd) || (kd < 0 && k6 > -kd));  // aR <- 3a - 2aL
-  const double st = fma(-2.0, sel_d(stl, aR, aL), 3.0 * a);
-  const double nL = sel_d(stl, st, aL), nR = sel_d(str, st, aR);
-  aL = sel_d(flat, a, nL);
-  aR = sel_d(flat, a, nR);
-}
-// the forms the transport kernels use: the oracle's in the strict build, the integer-pipe forms
-// in the production build
-__device__ __forceinline__ double slope_u_p(double am, double a, double ap) {
-#if RS_STRICT
-  return slope_u(am, a, ap);
-#else
-  return slope_u_fast(am, a, ap);
-#endif
-}
-__device__ __forceinline__ double slope_n_p(double am, double a, double ap, double sA, double sB) {
-#if RS_STRICT
-  return slope_n(am, a, ap, sA, sB);
-#else
-  return slope_n_fast(am, a, ap, sA, sB);
-#endif
-}
-__device__ __forceinline__ void limit_p(double a, double& aL, double& aR) {
-#if RS_STRICT
-  limit(a, aL, aR);
-#else
-  limit_fast(a, aL, aR);
-#endif
-}
-
 // slopes from the neighbour differences d0 = a - am, d1 = ap - a (computed once per cell by the
 // pencil kernels) -- the same operations as slope_u / slope_n, so bit-identical to them
 __device__ __forceinline__ double slope_ud(double d0, double d1, double am, double ap) {
@@ -162,7 +102,7 @@ __device__ __forceinline__ double slope_ud(double d0, double d1, double am, doub
     }
     return 0.0;
   }
-  return slope_pick32(d0, d1, ap - am, true);
+  return slope_pick32(d0, d1, d0 + d1, true);
 #endif
 }
 __device__ __forceinline__ double slope_nd(double d0, double d1, double sA, double sB) {
@@ -186,14 +126,69 @@ __device__ __forceinline__ double slope_nd(double d0, double d1, double sA, doub
 #endif
 }
 
+#if !RS_STRICT
+// ---- production form of edges, limiter and face value, on deviations from the cell's own value.
+// With D_p = v(p+1) - v(p) and S_p the limited slope, the deviation of cell p's right edge is
+// eR = D_p/2 - (S_{p+1} - S_p)/6 and that of its left edge eL = E_{p-1} - D_{p-1} (E the right
+// deviations).  On these the CW84 limiter (eq. 1.10) needs no arithmetic: it flattens unless eL
+// and eR have strictly opposite signs, and
+//   dA a6 >  dA^2  <=>  |eL| > 2 |eR|   (eL <- -2 eR)
+//   dA a6 < -dA^2  <=>  |eR| > 2 |eL|   (eR <- -2 eL),
+// so the limited deviation of one edge is its own sign with min(|e|, 2 |the other|): sign tests,
+// magnitude compares and an exact doubling on the integer pipes.  The uniform directions carry
+// 6 E (no division): 6 E_p = 3 D_p - (S_{p+1} - S_p), 6 eL = 6 E_{p-1} - 6 D_{p-1}, and the face
+// value is a + dev6 / 6 in one FMA.  FP64 operations per face: 7 (x, y) and 9 (vertical) where
+// the edge values with the limiter's dA, a6 and 3a - 2e took 12 and 13; FP64 issues one warp
+// instruction per 64 cycles and SM sub-partition here, so the count is the time.  A deviation
+// is formed from differences alone, so it carries less rounding than aR - a did; a uniform field
+// gives exactly 0.  Measured on 144x91x47 with 12 tracers: lon rows 202 -> 125 us, lat plus
+// vertical pencils 400 -> 275 us.
+__device__ __forceinline__ double edge6_u(double D, double S0, double S1) {
+  return fma(3.0, D, -(S1 - S0));
+}
+__device__ __forceinline__ double left6_u(double Em, double Dm) { return fma(-6.0, Dm, Em); }
+__device__ __forceinline__ double edge_nd(double D, double S0, double S1, double ab, double c,
+                                          double d) {
+  return fma(d, S0, fma(c, S1, ab * D));
+}
+// The face value of upwind cell value a with edge deviations eL, eR (times 6 if UNI).  Where the
+// product of the deviations could underflow (the limiter's extremum test in FP64 then sees 0),
+// the FP form decides, as before.
+template <bool UNI>
+__device__ __forceinline__ double face_value(double a, double eL, double eR, bool right) {
+  if (prod_may_underflow(eL, eR)) {
+    double aL = UNI ? fma(eL, kOneSixth, a) : a + eL, aR = UNI ? fma(eR, kOneSixth, a) : a + eR;
+    limit(a, aL, aR);
+    return right ? aR : aL;
+  }
+  const int hL = __double2hiint(eL), hR = __double2hiint(eR);
+  const unsigned lL = (unsigned)__double2loint(eL), lR = (unsigned)__double2loint(eR);
+  const unsigned mL = (unsigned)hL & 0x7fffffffu, mR = (unsigned)hR & 0x7fffffffu;
+  const unsigned ms = right ? mR : mL, ls = right ? lR : lL;                // the edge itself
+  const unsigned mo = (right ? mL : mR) + (1u << 20), lo = right ? lL : lR;  // 2 |the other|
+  const bool binds = mag_lt(mo, lo, ms, ls);
+  const unsigned sg = (unsigned)(right ? hR : hL) & 0x80000000u;
+  const bool opp = ((hL ^ hR) < 0) & ((mL | lL) != 0u) & ((mR | lR) != 0u);
+  const double dev = __hiloint2double(opp ? (int)((binds ? mo : ms) | sg) : 0,
+                                      opp ? (int)(binds ? lo : ls) : 0);
+  return UNI ? fma(dev, kOneSixth, a) : a + dev;
+}
+#endif
 __device__ __forceinline__ double ppm_face_u(const double* v, bool right) {
-  double dm1 = slope_u_p(v[0], v[1], v[2]);
-  double d0 = slope_u_p(v[1], v[2], v[3]);
-  double dp1 = slope_u_p(v[2], v[3], v[4]);
+#if RS_STRICT
+  double dm1 = slope_u(v[0], v[1], v[2]);
+  double d0 = slope_u(v[1], v[2], v[3]);
+  double dp1 = slope_u(v[2], v[3], v[4]);
   double aL = v[1] + 0.5 * (v[2] - v[1]) - (d0 - dm1) * kOneSixth;
   double aR = v[2] + 0.5 * (v[3] - v[2]) - (dp1 - d0) * kOneSixth;
-  limit_p(v[2], aL, aR);
+  limit(v[2], aL, aR);
   return right ? aR : aL;
+#else
+  const double d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3];
+  const double sm = slope_ud(d0, d1, v[0], v[2]), sc = slope_ud(d1, d2, v[1], v[3]),
+               sp = slope_ud(d2, d3, v[2], v[4]);
+  return face_value<true>(v[2], left6_u(edge6_u(d1, sm, sc), d1), edge6_u(d2, sc, sp), right);
+#endif
 }
 
 // split a double into hi + lo floats (used only for boundary ghosts in the flux kernels)
@@ -377,13 +372,22 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_z(DevTransport<double> T,
     const double* q = Q + (size_t)s * nc + col;
     double v[5];
     for (int o = 0; o < 5; ++o) v[o] = q[(size_t)kk[o] * ncol];
-    double dm1 = slope_n_p(v[0], v[1], v[2], sA0, sB0);
-    double d0 = slope_n_p(v[1], v[2], v[3], sA1, sB1);
-    double dp1 = slope_n_p(v[2], v[3], v[4], sA2, sB2);
+#if RS_STRICT
+    double dm1 = slope_n(v[0], v[1], v[2], sA0, sB0);
+    double d0 = slope_n(v[1], v[2], v[3], sA1, sB1);
+    double dp1 = slope_n(v[2], v[3], v[4], sA2, sB2);
     double aL = v[1] + eLab * (v[2] - v[1]) + eLc * d0 + eLd * dm1;
     double aR = v[2] + eRab * (v[3] - v[2]) + eRc * dp1 + eRd * d0;
-    limit_p(v[2], aL, aR);
-    T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * (right ? aR : aL);
+    limit(v[2], aL, aR);
+    const double face = right ? aR : aL;
+#else
+    const double e0 = v[1] - v[0], e1 = v[2] - v[1], e2 = v[3] - v[2], e3 = v[4] - v[3];
+    const double sm = slope_nd(e0, e1, sA0, sB0), sc = slope_nd(e1, e2, sA1, sB1),
+                 sp = slope_nd(e2, e3, sA2, sB2);
+    const double face = face_value<false>(v[2], edge_nd(e1, sm, sc, eLab, eLc, eLd) - e1,
+                                          edge_nd(e2, sc, sp, eRab, eRc, eRd), right);
+#endif
+    T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * face;
   }
 }
 
@@ -403,7 +407,8 @@ __global__ void __launch_bounds__(256) k_flux_x_fused(DevTransport<double> T, St
   double* V = smx;            // V[p+3], p in [-3, n+2]
   double* Dd = smx + L;       // Dd[p+3] = v(p+1) - v(p), p in [-3, n+1]
   double* D = smx + 2 * L;    // D[p+3], slopes p in [-2, n+1]
-  double* E = smx + 3 * L;    // E[f+3], edge between f-1 and f, f in [-1, n+1]
+  double* E = smx + 3 * L;    // strict: E[f+3], edge between f-1 and f, f in [-1, n+1];
+                              // production: E[p+3] = 6 x right-edge deviation of cell p
   double* Mf = smx + 4 * L;   // Mf[f], the face's air-mass flux g*mx (shared by all tracers)
   const int row = blockIdx.x;  // (k, j)
   const int j = row % T.nlat, k = row / T.nlat;
@@ -430,16 +435,27 @@ __global__ void __launch_bounds__(256) k_flux_x_fused(DevTransport<double> T, St
     for (int p = threadIdx.x - 2; p <= n + 1; p += blockDim.x)
       D[bck(T, p + 3, L)] = slope_ud(Dd[bck(T, p + 2, L)], Dd[bck(T, p + 3, L)], V[bck(T, p + 2, L)], V[bck(T, p + 4, L)]);
     __syncthreads();
+#if RS_STRICT
     for (int f = threadIdx.x - 1; f <= n + 1; f += blockDim.x)
       E[bck(T, f + 3, L)] = V[bck(T, f + 2, L)] + 0.5 * Dd[bck(T, f + 2, L)] - (D[bck(T, f + 3, L)] - D[bck(T, f + 2, L)]) * kOneSixth;
+#else
+    for (int p = threadIdx.x - 2; p <= n; p += blockDim.x)  // 6 E of cells -2 .. n
+      E[bck(T, p + 3, L)] = edge6_u(Dd[bck(T, p + 3, L)], D[bck(T, p + 3, L)], D[bck(T, p + 4, L)]);
+#endif
     __syncthreads();
     for (int f = threadIdx.x; f <= n; f += blockDim.x) {
       const double M = Mf[bck(T, f, nf)];
       const bool right = __double_as_longlong(M) > 0;  // M > 0 for every non-NaN M
       int up = right ? f - 1 : f;
+#if RS_STRICT
       double aL = E[bck(T, up + 3, L)], aR = E[bck(T, up + 4, L)];
-      limit_p(V[bck(T, up + 3, L)], aL, aR);
-      T.fx[((size_t)s * T.nlev * T.nlat + (size_t)k * T.nlat + j) * nf + f] = M * (right ? aR : aL);
+      limit(V[bck(T, up + 3, L)], aL, aR);
+      const double face = right ? aR : aL;
+#else
+      const double face = face_value<true>(V[bck(T, up + 3, L)], left6_u(E[bck(T, up + 2, L)], Dd[bck(T, up + 2, L)]),
+                                           E[bck(T, up + 3, L)], right);
+#endif
+      T.fx[((size_t)s * T.nlev * T.nlat + (size_t)k * T.nlat + j) * nf + f] = M * face;
     }
     __syncthreads();
   }
@@ -491,8 +507,13 @@ __global__ void __launch_bounds__(512) k_flux_y_fused(DevTransport<double> T, St
     for (int p = (int)ty - 2; p <= n + 1; p += blockDim.y)
       RS_P(D, p) = slope_ud(RS_P(Dd, p - 1), RS_P(Dd, p), RS_P(V, p - 1), RS_P(V, p + 1));
     __syncthreads();
+#if RS_STRICT
     for (int f = (int)ty - 1; f <= n + 1; f += blockDim.y)
       RS_P(E, f) = RS_P(V, f - 1) + 0.5 * RS_P(Dd, f - 1) - (RS_P(D, f) - RS_P(D, f - 1)) * kOneSixth;
+#else
+    for (int p = (int)ty - 2; p <= n; p += blockDim.y)
+      RS_P(E, p) = edge6_u(RS_P(Dd, p), RS_P(D, p), RS_P(D, p + 1));
+#endif
     __syncthreads();
     if (live) {
       for (int f = ty; f <= n; f += blockDim.y) {
@@ -504,9 +525,14 @@ __global__ void __launch_bounds__(512) k_flux_y_fused(DevTransport<double> T, St
         const double M = Mf[bck(T, f * kPencil + tx, (long long)(n + 1) * kPencil)];
         const bool right = __double_as_longlong(M) > 0;
         int up = right ? f - 1 : f;
+#if RS_STRICT
         double aL = RS_P(E, up), aR = RS_P(E, up + 1);
-        limit_p(RS_P(V, up), aL, aR);
-        T.fy[(size_t)s * fplane + fb] = M * (right ? aR : aL);
+        limit(RS_P(V, up), aL, aR);
+        const double face = right ? aR : aL;
+#else
+        const double face = face_value<true>(RS_P(V, up), left6_u(RS_P(E, up - 1), RS_P(Dd, up - 1)), RS_P(E, up), right);
+#endif
+        T.fy[(size_t)s * fplane + fb] = M * face;
       }
     }
     __syncthreads();
@@ -558,7 +584,11 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
       double eab = live ? T.veAB[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
       double ec = live ? T.veC[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
       double ed = live ? T.veD[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
+#if RS_STRICT
       RS_P(E, e) = RS_P(V, e - 1) + eab * RS_P(Dd, e - 1) + ec * RS_P(D, e) + ed * RS_P(D, e - 1);
+#else
+      RS_P(E, e - 1) = edge_nd(RS_P(Dd, e - 1), RS_P(D, e - 1), RS_P(D, e), eab, ec, ed);  // of cell e-1
+#endif
     }
     __syncthreads();
     if (live) {
@@ -570,9 +600,14 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
         const double M = Mf[bck(T, kf * kPencil + tx, (long long)(n + 1) * kPencil)];
         const bool right = __double_as_longlong(M) > 0;
         int up = right ? kf - 1 : kf;
+#if RS_STRICT
         double aL = RS_P(E, up), aR = RS_P(E, up + 1);
-        limit_p(RS_P(V, up), aL, aR);
-        T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * (right ? aR : aL);
+        limit(RS_P(V, up), aL, aR);
+        const double face = right ? aR : aL;
+#else
+        const double face = face_value<false>(RS_P(V, up), RS_P(E, up - 1) - RS_P(Dd, up - 1), RS_P(E, up), right);
+#endif
+        T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * face;
       }
     }
     __syncthreads();
