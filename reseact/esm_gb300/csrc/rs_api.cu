@@ -326,7 +326,7 @@ struct rs_handle {
   std::vector<DevBuf<double>> dtabs;
   DevBuf<int> slot_row, slot_col;
   // state and scratch
-  DevBuf<double> U[2], S1, S2, S3, fx, fy, fz, partial, krates, T, P, emis, io, io2;
+  DevBuf<double> U[2], S1, S2, S3, fx, fy, fz, mx6, myn6, mys6, partial, krates, T, P, emis, io, io2;
   DevBuf<double> mx, my, mz, qw, qe, qs, qn, gx, gylo, gyhi, vsA, vsB, veAB, veC, veD, dtcell,
       stepcell, totals;
   DevBuf<float> qhi, qlo;  // mixed-precision transport: split planes
@@ -403,6 +403,7 @@ struct rs_handle {
     int pc_regcap = 0;  // 1: the table-walking per-cell kernel capped at 32 registers
     int pencil = 32, rows = 8, xthreads = 128;        // transport pencil kernels
     int xgroups = 1, yzgroups = 1;                    // their tracer groups
+    int yzline = 0;                                   // thread per lat / vertical line
     int mpencil = 16, mrows = 16, mxthreads = 128;    // mixed-precision pencil kernels
     int msper_x = 1 << 20, msper_yz = 1;             // tracers per block (clamped to ntr)
     int mbulk_x = 1, mbulk_yz = 1;                    // bulk-copy staging per direction
@@ -553,6 +554,24 @@ void make_flux_pairs(rs_handle* h) {
   CK(cudaGetLastError());
 }
 
+// The production FP64 kernels' scaled fluxes (after every flux change).
+void scale_fluxes(rs_handle* h) {
+#if !RS_STRICT
+  h->mx6.alloc(h->mx.n);
+  h->myn6.alloc(h->my.n);
+  h->mys6.alloc(h->my.n);
+  rs::DevTransport<double> T{};
+  T.nlon = h->nlon; T.nlat = h->nlat; T.nlev = h->nlev;
+  T.lat_bc = h->cfg.grid.lat_bc;
+  T.gx = h->gx.p; T.gylo = h->gylo.p; T.gyhi = h->gyhi.p;
+  T.mx = h->mx.p; T.my = h->my.p;
+  rs::launch_scale_fluxes(h->st, T, h->mx6.p, h->myn6.p, h->mys6.p);
+  CK(cudaGetLastError());
+#else
+  (void)h;
+#endif
+}
+
 // Lat-lon geometry on the unit sphere (same formulas and order as the CPU restatement).
 void build_geometry(rs_handle* h) {
   const rs_grid& g = h->cfg.grid;
@@ -642,19 +661,22 @@ void refresh_dt(rs_handle* h) {
   T.qw = h->qw.p; T.qe = h->qe.p; T.qs = h->qs.p; T.qn = h->qn.p;
   T.vsA = h->vsA.p; T.vsB = h->vsB.p; T.veAB = h->veAB.p; T.veC = h->veC.p; T.veD = h->veD.p;
   T.fx = h->fx.p; T.fy = h->fy.p; T.fz = h->fz.p;
+  T.acc64 = h->fx.p;
+  T.mx6 = h->mx6.p; T.myn6 = h->myn6.p; T.mys6 = h->mys6.p;
   T.mixed = h->cfg.precision == RS_PREC_MIXED;
   T.qhi = h->qhi.p; T.qlo = h->qlo.p;
   auto f2 = [](const DevBuf<float>& b) { return reinterpret_cast<const float2*>(b.p); };
   T.gx2 = f2(h->gx2); T.gylo2 = f2(h->gylo2); T.gyhi2 = f2(h->gyhi2);
   T.vsA2 = f2(h->vsA2); T.vsB2 = f2(h->vsB2); T.veAB2 = f2(h->veAB2); T.veC2 = f2(h->veC2);
   T.veD2 = f2(h->veD2);
-  T.acc = T.mixed ? reinterpret_cast<float2*>(h->fx.p) : nullptr;  // ntr*nc pairs fit in fx
+  T.acc = T.mixed ? reinterpret_cast<float2*>(h->fx.p) : nullptr;  // ntr*nc pairs
   T.mx2 = f2(h->mx2); T.my2 = f2(h->my2); T.mz2 = f2(h->mz2);
   T.pencil = h->tune.pencil;
   T.rows = h->tune.rows;
   T.xthreads = h->tune.xthreads;
   T.xgroups = h->tune.xgroups;
   T.yzgroups = h->tune.yzgroups;
+  T.yzline = h->tune.yzline;
   T.mpencil = h->tune.mpencil;
   T.mrows = h->tune.mrows;
   T.mxthreads = h->tune.mxthreads;
@@ -1033,9 +1055,13 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
     }
     if (cfg->do_transport) {
       h->S1.alloc(n); h->S2.alloc(n); h->S3.alloc(n);
+#if RS_STRICT
       h->fx.alloc((size_t)h->ntr * g.nlev * g.nlat * (g.nlon + 1));
       h->fy.alloc((size_t)h->ntr * g.nlev * (g.nlat + 1) * g.nlon);
       h->fz.alloc((size_t)h->ntr * (g.nlev + 1) * g.nlat * g.nlon);
+#else
+      h->fx.alloc((size_t)h->ntr * h->nc);  // the accumulator
+#endif
       h->mx.alloc((size_t)g.nlev * g.nlat * (g.nlon + 1)); h->mx.zero(h->st);
       h->my.alloc((size_t)g.nlev * (g.nlat + 1) * g.nlon); h->my.zero(h->st);
       h->mz.alloc((size_t)(g.nlev + 1) * g.nlat * g.nlon); h->mz.zero(h->st);
@@ -1054,6 +1080,7 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
       build_vertical(h);
     }
     if (cfg->do_transport && cfg->precision == RS_PREC_MIXED) make_flux_pairs(h);  // zero fluxes
+    if (cfg->do_transport) scale_fluxes(h);
     refresh_dt(h);
     if (cfg->do_transport && cfg->precision == RS_PREC_MIXED) {
       const char* why = nullptr;
@@ -1083,6 +1110,7 @@ void rs_destroy(rs_handle* h) {
                             &h->vsB2, &h->veAB2, &h->veC2, &h->veD2, &h->mx2, &h->my2, &h->mz2};
   for (auto* b : fbufs) b->release();
   DevBuf<double>* bufs[] = {&h->U[0], &h->U[1], &h->S1, &h->S2, &h->S3, &h->fx, &h->fy, &h->fz,
+                            &h->mx6, &h->myn6, &h->mys6,
                             &h->partial, &h->krates, &h->T, &h->P, &h->emis, &h->io, &h->io2,
                             &h->mx, &h->my, &h->mz, &h->qw, &h->qe, &h->qs, &h->qn, &h->gx,
                             &h->gylo, &h->gyhi, &h->vsA, &h->vsB, &h->veAB, &h->veC, &h->veD,
@@ -1202,6 +1230,7 @@ rs_status rs_set_forcing(rs_handle* h, const rs_forcing* f) {
       if (f->dps_dt) h->dpsdt_host.assign(f->dps_dt, f->dps_dt + ncol);
       if (f->dps_dt || f->hyb_b || f->mx || f->my || f->mz || f->dp) build_fixer(h);
       if (h->cfg.precision == RS_PREC_MIXED) make_flux_pairs(h);
+      if (f->mx || f->my) scale_fluxes(h);
     }
     if (f->temperature) {
       h->T.upload(f->temperature, nc, st);
@@ -2050,6 +2079,7 @@ extern "C" rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t 
     else if (k == "rows") ok = in({4, 8, 16, 32}) && (t.rows = value, true);
     else if (k == "x_tracer_groups") ok = value >= 1 && value <= ntr && (t.xgroups = value, true);
     else if (k == "yz_tracer_groups") ok = value >= 1 && value <= ntr && (t.yzgroups = value, true);
+    else if (k == "yz_line") ok = in({0, 1}) && (value == 0 || !RS_STRICT) && (t.yzline = value, true);
     else if (k == "mixed_xthreads") ok = in({64, 128, 256}) && (t.mxthreads = value, true);
     else if (k == "mixed_x_tracers") ok = value >= 1 && value <= ntr && (t.msper_x = value, true);
     else if (k == "mixed_pencil") ok = in({16, 32}) && (t.mpencil = value, true);
@@ -2529,6 +2559,7 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
       rep += "], \"pencils\": [";
       first = true;
       float byz = 1e30f;
+      T.yzline = 0;
       T.xthreads = h->tune.xthreads;
       for (int pw : {8, 16, 32})
         for (int rows : {4, 8, 16, 32}) {
@@ -2577,11 +2608,27 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
         rs::launch_flux_dir(h->st, T, Q, 1);
         rs::launch_flux_dir(h->st, T, Q, 2);
       });
+      // a thread per lat / vertical line against the best pencils (production build)
+      h->tune.yzline = 0;
+      if (!RS_STRICT) {
+        auto run = [&] {
+          rs::launch_flux_dir(h->st, T, Q, 1);
+          rs::launch_flux_dir(h->st, T, Q, 2);
+        };
+        T.yzline = 0;
+        const float mp = time_min(h->st, 3, run);
+        T.yzline = 1;
+        const float ml = time_min(h->st, 3, run);
+        h->tune.yzline = ml < mp;
+        T.yzline = h->tune.yzline;
+        std::snprintf(line, sizeof line, "], \"yz_lines\": [{\"line\": 0, \"ms\": %.4f}, {\"line\": 1, \"ms\": %.4f}", mp, ml);
+        rep += line;
+      }
       std::snprintf(line, sizeof line,
                     "], \"transport_choice\": {\"xthreads\": %d, \"pencil\": %d, \"rows\": %d, "
-                    "\"x_tracer_groups\": %d, \"yz_tracer_groups\": %d}",
+                    "\"x_tracer_groups\": %d, \"yz_tracer_groups\": %d, \"yz_line\": %d}",
                     h->tune.xthreads, h->tune.pencil, h->tune.rows, h->tune.xgroups,
-                    h->tune.yzgroups);
+                    h->tune.yzgroups, h->tune.yzline);
       rep += line;
       if (h->cfg.precision == RS_PREC_MIXED) {
         // the FP32 deviation-form pencils: threads per lon row and tracers per block for x,

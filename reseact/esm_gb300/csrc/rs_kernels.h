@@ -53,12 +53,19 @@ struct DevTransport {
   const double* veAB;  // [(nlev+1)][ncol] edge coefficients, edges 0..nlev
   const double* veC;
   const double* veD;
+  // strict build: the FP64 tracer fluxes
   R* fx;               // [ntr][nlev][nlat][nlon+1]
   R* fy;               // [ntr][nlev][nlat+1][nlon]
   R* fz;               // [ntr][nlev+1][nlat][nlon]
+  // production build: the FP64 accumulator of -m dq/dt / g per cell, and the horizontal air-mass
+  // fluxes with the cells' metric and the uniform edges' 1/6 folded in
+  double* acc64;       // [ntr][nc]
+  const double* mx6;   // shape of mx
+  const double* myn6;  // shape of my, as the cell south of the face sees it
+  const double* mys6;  // and the cell north of it
   // mixed precision (compensated FP32): the RHS input split into hi, lo planes [ntr][nc]
   // (hi + lo = q to 2^-47), the metric factors and vertical coefficients as (hi, lo) pairs, and
-  // the per-cell accumulator of m dq/dt as pairs [ntr][nc] (in the memory of fx)
+  // the per-cell accumulator of m dq/dt as pairs [ntr][nc]
   float* qhi;
   float* qlo;
   const float2* gx2;    // [nlat]
@@ -90,6 +97,7 @@ struct DevTransport {
   int rows;      // threads along the pencil (blockDim.y): 4 .. 32
   int xthreads;  // threads per lon row: 64 .. 256 in steps of 32
   int xgroups, yzgroups;  // tracer groups (blockIdx.y) of the lon / lat and vertical pencils
+  int yzline;    // 1: one thread per lat / vertical line instead of the pencils (production build)
   // launch shape of the mixed-precision pencil kernels (chosen by rs_autotune)
   int mpencil, mrows, mxthreads;
   int msper_x, msper_yz;  // tracers per block (blockIdx.y selects the group)
@@ -162,6 +170,9 @@ size_t mixed_pencil_cap();
 void mixed_tmaps_destroy(MixedTmaps* m);
 bool mixed_tmaps_dir_ok(const MixedTmaps* m, int dir);  // dir 0 lon rows, 1 lat, 2 vertical
 void launch_flux_dir(cudaStream_t st, const DevTransport<double>& T, const double* Q, int dir);
+// the scaled air-mass fluxes mx6, myn6, mys6 from mx, my (production build)
+void launch_scale_fluxes(cudaStream_t st, const DevTransport<double>& T, double* mx6, double* myn6,
+                         double* mys6);
 // (hi, lo) float pairs of n doubles (the mixed kernels' face fluxes)
 void launch_make_pairs(cudaStream_t st, const double* src, float2* dst, size_t n);
 void launch_flux_dir_mixed(cudaStream_t st, const DevTransport<double>& T, const double* Q, int dir,

@@ -26,7 +26,11 @@
 namespace rs {
 
 constexpr double kOneSixth = 1.0 / 6.0;
+#if RS_STRICT
 constexpr int kFluxThreads = 256;
+#else
+constexpr int kLineThreads = 64;
+#endif
 
 // (the limit 2 min(|d0|, |d1|) equals min(2|d0|, 2|d1|) exactly: scaling by 2 is exact)
 __device__ __forceinline__ double slope_u(double am, double a, double ap) {
@@ -83,112 +87,40 @@ __device__ __forceinline__ double slope_pick32(double d0, double d1, double da, 
                     ((h1 | l1) != 0u);
   return __hiloint2double(live ? (int)hr : 0, live ? (int)lr : 0);
 }
-// slopes from the neighbour differences d0 = a - am, d1 = ap - a (computed once per cell by the
-// pencil kernels) -- the same operations as slope_u / slope_n, so bit-identical to them
-__device__ __forceinline__ double slope_ud(double d0, double d1, double am, double ap) {
+// slopes from the neighbour differences d0 = a - am, d1 = ap - a
 #if RS_STRICT
+// (am, ap: the oracle forms the centred slope from the values)
+__device__ __forceinline__ double slope_ud(double d0, double d1, double am, double ap) {
   if (d1 * d0 > 0.0) {
     double da = 0.5 * (ap - am);
     double lim = 2.0 * fmin(fabs(d0), fabs(d1));
     return copysign(fmin(fabs(da), lim), da);
   }
   return 0.0;
+}
 #else
+__device__ __forceinline__ double slope_ud(double d0, double d1) {
   if (prod_may_underflow(d0, d1)) {
     if (d1 * d0 > 0.0) {
-      double da = 0.5 * (ap - am);
+      double da = 0.5 * (d0 + d1);
       double lim = 2.0 * fmin(fabs(d0), fabs(d1));
       return copysign(fmin(fabs(da), lim), da);
     }
     return 0.0;
   }
   return slope_pick32(d0, d1, d0 + d1, true);
-#endif
 }
+#endif
 __device__ __forceinline__ double slope_nd(double d0, double d1, double sA, double sB) {
-#if RS_STRICT
+#if !RS_STRICT
+  if (!prod_may_underflow(d0, d1)) return slope_pick32(d0, d1, sA * d1 + sB * d0, false);
+#endif
   if (d1 * d0 > 0.0) {
     double da = sA * d1 + sB * d0;
     double lim = 2.0 * fmin(fabs(d0), fabs(d1));
     return copysign(fmin(fabs(da), lim), da);
   }
   return 0.0;
-#else
-  if (prod_may_underflow(d0, d1)) {
-    if (d1 * d0 > 0.0) {
-      double da = sA * d1 + sB * d0;
-      double lim = 2.0 * fmin(fabs(d0), fabs(d1));
-      return copysign(fmin(fabs(da), lim), da);
-    }
-    return 0.0;
-  }
-  return slope_pick32(d0, d1, sA * d1 + sB * d0, false);
-#endif
-}
-
-#if !RS_STRICT
-// ---- production form of edges, limiter and face value, on deviations from the cell's own value.
-// With D_p = v(p+1) - v(p) and S_p the limited slope, the deviation of cell p's right edge is
-// eR = D_p/2 - (S_{p+1} - S_p)/6 and that of its left edge eL = E_{p-1} - D_{p-1} (E the right
-// deviations).  On these the CW84 limiter (eq. 1.10) needs no arithmetic: it flattens unless eL
-// and eR have strictly opposite signs, and
-//   dA a6 >  dA^2  <=>  |eL| > 2 |eR|   (eL <- -2 eR)
-//   dA a6 < -dA^2  <=>  |eR| > 2 |eL|   (eR <- -2 eL),
-// so the limited deviation of one edge is its own sign with min(|e|, 2 |the other|): sign tests,
-// magnitude compares and an exact doubling on the integer pipes.  The uniform directions carry
-// 6 E (no division): 6 E_p = 3 D_p - (S_{p+1} - S_p), 6 eL = 6 E_{p-1} - 6 D_{p-1}, and the face
-// value is a + dev6 / 6 in one FMA.  FP64 operations per face: 7 (x, y) and 9 (vertical) where
-// the edge values with the limiter's dA, a6 and 3a - 2e took 12 and 13; FP64 issues one warp
-// instruction per 64 cycles and SM sub-partition here, so the count is the time.  A deviation
-// is formed from differences alone, so it carries less rounding than aR - a did; a uniform field
-// gives exactly 0.  Measured on 144x91x47 with 12 tracers: lon rows 202 -> 125 us, lat plus
-// vertical pencils 400 -> 275 us.
-__device__ __forceinline__ double edge6_u(double D, double S0, double S1) {
-  return fma(3.0, D, -(S1 - S0));
-}
-__device__ __forceinline__ double left6_u(double Em, double Dm) { return fma(-6.0, Dm, Em); }
-__device__ __forceinline__ double edge_nd(double D, double S0, double S1, double ab, double c,
-                                          double d) {
-  return fma(d, S0, fma(c, S1, ab * D));
-}
-// The face value of upwind cell value a with edge deviations eL, eR (times 6 if UNI).  Where the
-// product of the deviations could underflow (the limiter's extremum test in FP64 then sees 0),
-// the FP form decides, as before.
-template <bool UNI>
-__device__ __forceinline__ double face_value(double a, double eL, double eR, bool right) {
-  if (prod_may_underflow(eL, eR)) {
-    double aL = UNI ? fma(eL, kOneSixth, a) : a + eL, aR = UNI ? fma(eR, kOneSixth, a) : a + eR;
-    limit(a, aL, aR);
-    return right ? aR : aL;
-  }
-  const int hL = __double2hiint(eL), hR = __double2hiint(eR);
-  const unsigned lL = (unsigned)__double2loint(eL), lR = (unsigned)__double2loint(eR);
-  const unsigned mL = (unsigned)hL & 0x7fffffffu, mR = (unsigned)hR & 0x7fffffffu;
-  const unsigned ms = right ? mR : mL, ls = right ? lR : lL;                // the edge itself
-  const unsigned mo = (right ? mL : mR) + (1u << 20), lo = right ? lL : lR;  // 2 |the other|
-  const bool binds = mag_lt(mo, lo, ms, ls);
-  const unsigned sg = (unsigned)(right ? hR : hL) & 0x80000000u;
-  const bool opp = ((hL ^ hR) < 0) & ((mL | lL) != 0u) & ((mR | lR) != 0u);
-  const double dev = __hiloint2double(opp ? (int)((binds ? mo : ms) | sg) : 0,
-                                      opp ? (int)(binds ? lo : ls) : 0);
-  return UNI ? fma(dev, kOneSixth, a) : a + dev;
-}
-#endif
-__device__ __forceinline__ double ppm_face_u(const double* v, bool right) {
-#if RS_STRICT
-  double dm1 = slope_u(v[0], v[1], v[2]);
-  double d0 = slope_u(v[1], v[2], v[3]);
-  double dp1 = slope_u(v[2], v[3], v[4]);
-  double aL = v[1] + 0.5 * (v[2] - v[1]) - (d0 - dm1) * kOneSixth;
-  double aR = v[2] + 0.5 * (v[3] - v[2]) - (dp1 - d0) * kOneSixth;
-  limit(v[2], aL, aR);
-  return right ? aR : aL;
-#else
-  const double d0 = v[1] - v[0], d1 = v[2] - v[1], d2 = v[3] - v[2], d3 = v[4] - v[3];
-  const double sm = slope_ud(d0, d1, v[0], v[2]), sc = slope_ud(d1, d2, v[1], v[3]),
-               sp = slope_ud(d2, d3, v[2], v[4]);
-  return face_value<true>(v[2], left6_u(edge6_u(d1, sm, sc), d1), edge6_u(d2, sc, sp), right);
-#endif
 }
 
 // split a double into hi + lo floats (used only for boundary ghosts in the flux kernels)
@@ -242,7 +174,20 @@ __device__ __forceinline__ bool resolve_stage(const StageSel& s, const double*& 
   return true;
 }
 
-// ------------------------------------------------------------------ face fluxes
+// ------------------------------------------------------------------ face fluxes (strict build)
+// The oracle's flux form, expression by expression; the production build's kernels are in
+// rs_adv64.cuh.
+#if RS_STRICT
+__device__ __forceinline__ double ppm_face_u(const double* v, bool right) {
+  double dm1 = slope_u(v[0], v[1], v[2]);
+  double d0 = slope_u(v[1], v[2], v[3]);
+  double dp1 = slope_u(v[2], v[3], v[4]);
+  double aL = v[1] + 0.5 * (v[2] - v[1]) - (d0 - dm1) * kOneSixth;
+  double aR = v[2] + 0.5 * (v[3] - v[2]) - (dp1 - d0) * kOneSixth;
+  limit(v[2], aL, aR);
+  return right ? aR : aL;
+}
+
 // x faces: (i_f in 0..nlon, j, k), i_f fastest
 __global__ void __launch_bounds__(kFluxThreads) k_flux_x(DevTransport<double> T, StageSel sel) {
   const double* Q;
@@ -372,7 +317,6 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_z(DevTransport<double> T,
     const double* q = Q + (size_t)s * nc + col;
     double v[5];
     for (int o = 0; o < 5; ++o) v[o] = q[(size_t)kk[o] * ncol];
-#if RS_STRICT
     double dm1 = slope_n(v[0], v[1], v[2], sA0, sB0);
     double d0 = slope_n(v[1], v[2], v[3], sA1, sB1);
     double dp1 = slope_n(v[2], v[3], v[4], sA2, sB2);
@@ -380,13 +324,6 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_z(DevTransport<double> T,
     double aR = v[2] + eRab * (v[3] - v[2]) + eRc * dp1 + eRd * d0;
     limit(v[2], aL, aR);
     const double face = right ? aR : aL;
-#else
-    const double e0 = v[1] - v[0], e1 = v[2] - v[1], e2 = v[3] - v[2], e3 = v[4] - v[3];
-    const double sm = slope_nd(e0, e1, sA0, sB0), sc = slope_nd(e1, e2, sA1, sB1),
-                 sp = slope_nd(e2, e3, sA2, sB2);
-    const double face = face_value<false>(v[2], edge_nd(e1, sm, sc, eLab, eLc, eLd) - e1,
-                                          edge_nd(e2, sc, sp, eRab, eRc, eRd), right);
-#endif
     T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * face;
   }
 }
@@ -435,26 +372,16 @@ __global__ void __launch_bounds__(256) k_flux_x_fused(DevTransport<double> T, St
     for (int p = threadIdx.x - 2; p <= n + 1; p += blockDim.x)
       D[bck(T, p + 3, L)] = slope_ud(Dd[bck(T, p + 2, L)], Dd[bck(T, p + 3, L)], V[bck(T, p + 2, L)], V[bck(T, p + 4, L)]);
     __syncthreads();
-#if RS_STRICT
     for (int f = threadIdx.x - 1; f <= n + 1; f += blockDim.x)
       E[bck(T, f + 3, L)] = V[bck(T, f + 2, L)] + 0.5 * Dd[bck(T, f + 2, L)] - (D[bck(T, f + 3, L)] - D[bck(T, f + 2, L)]) * kOneSixth;
-#else
-    for (int p = threadIdx.x - 2; p <= n; p += blockDim.x)  // 6 E of cells -2 .. n
-      E[bck(T, p + 3, L)] = edge6_u(Dd[bck(T, p + 3, L)], D[bck(T, p + 3, L)], D[bck(T, p + 4, L)]);
-#endif
     __syncthreads();
     for (int f = threadIdx.x; f <= n; f += blockDim.x) {
       const double M = Mf[bck(T, f, nf)];
       const bool right = __double_as_longlong(M) > 0;  // M > 0 for every non-NaN M
       int up = right ? f - 1 : f;
-#if RS_STRICT
       double aL = E[bck(T, up + 3, L)], aR = E[bck(T, up + 4, L)];
       limit(V[bck(T, up + 3, L)], aL, aR);
       const double face = right ? aR : aL;
-#else
-      const double face = face_value<true>(V[bck(T, up + 3, L)], left6_u(E[bck(T, up + 2, L)], Dd[bck(T, up + 2, L)]),
-                                           E[bck(T, up + 3, L)], right);
-#endif
       T.fx[((size_t)s * T.nlev * T.nlat + (size_t)k * T.nlat + j) * nf + f] = M * face;
     }
     __syncthreads();
@@ -507,13 +434,8 @@ __global__ void __launch_bounds__(512) k_flux_y_fused(DevTransport<double> T, St
     for (int p = (int)ty - 2; p <= n + 1; p += blockDim.y)
       RS_P(D, p) = slope_ud(RS_P(Dd, p - 1), RS_P(Dd, p), RS_P(V, p - 1), RS_P(V, p + 1));
     __syncthreads();
-#if RS_STRICT
     for (int f = (int)ty - 1; f <= n + 1; f += blockDim.y)
       RS_P(E, f) = RS_P(V, f - 1) + 0.5 * RS_P(Dd, f - 1) - (RS_P(D, f) - RS_P(D, f - 1)) * kOneSixth;
-#else
-    for (int p = (int)ty - 2; p <= n; p += blockDim.y)
-      RS_P(E, p) = edge6_u(RS_P(Dd, p), RS_P(D, p), RS_P(D, p + 1));
-#endif
     __syncthreads();
     if (live) {
       for (int f = ty; f <= n; f += blockDim.y) {
@@ -525,13 +447,9 @@ __global__ void __launch_bounds__(512) k_flux_y_fused(DevTransport<double> T, St
         const double M = Mf[bck(T, f * kPencil + tx, (long long)(n + 1) * kPencil)];
         const bool right = __double_as_longlong(M) > 0;
         int up = right ? f - 1 : f;
-#if RS_STRICT
         double aL = RS_P(E, up), aR = RS_P(E, up + 1);
         limit(RS_P(V, up), aL, aR);
         const double face = right ? aR : aL;
-#else
-        const double face = face_value<true>(RS_P(V, up), left6_u(RS_P(E, up - 1), RS_P(Dd, up - 1)), RS_P(E, up), right);
-#endif
         T.fy[(size_t)s * fplane + fb] = M * face;
       }
     }
@@ -584,11 +502,7 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
       double eab = live ? T.veAB[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
       double ec = live ? T.veC[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
       double ed = live ? T.veD[bck(T, (size_t)e * ncol + col, (long long)(n + 1) * ncol)] : 0.0;
-#if RS_STRICT
       RS_P(E, e) = RS_P(V, e - 1) + eab * RS_P(Dd, e - 1) + ec * RS_P(D, e) + ed * RS_P(D, e - 1);
-#else
-      RS_P(E, e - 1) = edge_nd(RS_P(Dd, e - 1), RS_P(D, e - 1), RS_P(D, e), eab, ec, ed);  // of cell e-1
-#endif
     }
     __syncthreads();
     if (live) {
@@ -600,13 +514,9 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
         const double M = Mf[bck(T, kf * kPencil + tx, (long long)(n + 1) * kPencil)];
         const bool right = __double_as_longlong(M) > 0;
         int up = right ? kf - 1 : kf;
-#if RS_STRICT
         double aL = RS_P(E, up), aR = RS_P(E, up + 1);
         limit(RS_P(V, up), aL, aR);
         const double face = right ? aR : aL;
-#else
-        const double face = face_value<false>(RS_P(V, up), RS_P(E, up - 1) - RS_P(Dd, up - 1), RS_P(E, up), right);
-#endif
         T.fz[(size_t)s * fplane + (size_t)kf * ncol + col] = M * face;
       }
     }
@@ -614,6 +524,7 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
   }
 #undef RS_P
 }
+#endif  // RS_STRICT
 
 // ------------------------------------------------------------------ mixed precision
 // Compensated FP32 transport.  Every transport value is carried as a double-float pair
@@ -1475,20 +1386,14 @@ __device__ __forceinline__ void div_parts(const DevTransport<double>& T, int i, 
                                           double g, const CellGeo& G, double& hz, double& vz) {
   div_parts(mass_fluxes(T, i, j, k, g), G, hz, vz);
 }
-// Production form of a flux divergence, (e - w) gx + n gyhi - s gylo + (t - b), as one FMA
-// chain (five FP64 operations).  k_stage applies it to the air-mass fluxes and to every tracer's
-// fluxes alike, so a tracer whose fluxes equal the air-mass fluxes bit for bit (a uniform
-// field) still cancels exactly.
-__device__ __forceinline__ double div_chain(double w, double e, double s, double n, double b,
-                                            double t, const CellGeo& G) {
-  return fma(e - w, G.gx, fma(n, G.gyhi, fma(-s, G.gylo, t - b)));
-}
+#if RS_STRICT
 __device__ __forceinline__ double div_m(const DevTransport<double>& T, int i, int j, int k,
                                         double g, const CellGeo& G) {
   double hz, vz;
   div_parts(T, i, j, k, g, G, hz, vz);
   return hz + vz;
 }
+#endif
 // air-mass tendency: -divM, or with the pressure fixer -((divh + corr) + DzM)
 __device__ __forceinline__ double dm_dt(const DevTransport<double>& T, int i, int j, int k,
                                         double g, const CellGeo& G, size_t c) {
@@ -1536,6 +1441,7 @@ static void launch_pbl_mean(cudaStream_t st, const DevTransport<double>& T, cons
   k_pbl_mean<<<(unsigned)((n + kRedThreads - 1) / kRedThreads), kRedThreads, 0, st>>>(T, sel);
 }
 
+#if RS_STRICT
 // stage in 1..4.  Qin: the field whose fluxes were computed (RHS argument).
 //   1: S1 = U + dt/2 f(U)           2: S2 = S1 + dt/2 f(S1)
 //   3: S1 = u3 = S2 + dt/2 f(S2), S3 = u4 = 2/3 U + 1/3 u3
@@ -1577,24 +1483,11 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
     CellGeo G{T.gx[j], T.gylo[j], T.gyhi[j]};
     // the air-mass divergence, once per cell: tracers and the air-mass row
     const MassFluxes F = mass_fluxes(T, i, j, k, g);
-#if RS_STRICT
     double hz, vz;
     div_parts(F, G, hz, vz);
     const double divM = hz + vz;
     const double dmdt = T.mcorr ? -((hz + T.mcorr[c]) + vz) : -(hz + vz);  // = dm_dt(...)
-#else
-    const double divM = div_chain(F.w, F.e, F.s, F.n, F.b, F.t, G);  // the tracers' own chain
-    double dmdt = -divM;
-    if (T.mcorr) {  // the pressure fixer's -((divh + corr) + DzM)
-      double hz, vz;
-      div_parts(F, G, hz, vz);
-      dmdt = -((hz + T.mcorr[c]) + vz);
-    }
-#endif
     double m = Qin[(size_t)(T.nsp - 1) * nc + c];
-#if !RS_STRICT
-    double rm = rcp_nr(m);  // m > 0
-#endif
     const int nfx = T.nlon + 1, nfy = T.nlat + 1;
     const size_t ncol = (size_t)T.nlon * T.nlat, col = (size_t)j * T.nlon + i;
     const size_t fxp = (size_t)T.nlev * T.nlat * nfx, fyp = (size_t)T.nlev * nfy * T.nlon,
@@ -1602,9 +1495,6 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
     const size_t fxi = ((size_t)k * T.nlat + j) * nfx + i;
     const size_t fyi = ((size_t)k * nfy + j) * T.nlon + i;
     const size_t fzi = (size_t)k * ncol + col;
-#if !RS_STRICT
-    const double sc = dt_2 * rm;  // the tracer increment is (a + q divM) * sc without PBL mixing
-#endif
     for (int s = 0; s < T.nsp; ++s) {
       size_t x = (size_t)s * nc + c;
       double q = Qin[x];
@@ -1612,15 +1502,10 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
       // expression order); the production build forms it as fma(du, scale, q), folding 1/m
       // into the scale when no PBL term is added
       double du;
-#if !RS_STRICT
-      double scale = dt_2;
-      bool per_m = false;  // du is the tendency times m (1/m folded into the scale)
-#endif
       if (s < T.ntr) {
         double fw = T.fx[s * fxp + fxi], fe = T.fx[s * fxp + fxi + 1];
         double fs = T.fy[s * fyp + fyi], fn = T.fy[s * fyp + fyi + T.nlon];
         double fb = T.fz[s * fzp + fzi], ft = T.fz[s * fzp + fzi + ncol];
-#if RS_STRICT
         double Dx = (fe - fw) * G.gx;
         double Dy = fn * G.gyhi - fs * G.gylo;
         double Dz = ft - fb;
@@ -1628,26 +1513,11 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
         double b = q * divM;
         du = (a + b) / m;
         if (T.pbl) du = du + pbl_term(T, c, col, s, q);
-#else
-        const double ab = fma(q, divM, -div_chain(fw, fe, fs, fn, fb, ft, G));
-        if (T.pbl) {
-          du = fma(ab, rm, pbl_term(T, c, col, s, q));
-        } else {
-          du = ab;
-          scale = sc;
-          per_m = true;
-        }
-#endif
       } else {
         du = dmdt;
       }
-#if RS_STRICT
       const double nx = q + dt_2 * du;
       if (Fo) Fo[x] = du;
-#else
-      const double nx = fma(du, scale, q);
-      if (Fo) Fo[x] = per_m ? du * rm : du;
-#endif
       if (STAGE == 1) {
         B.S1[x] = nx;
         if (Vo) Vo[x] = nx;
@@ -1665,7 +1535,6 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
         double u0 = U[x];
         double u3 = B.S1[x];
         double un = nx;
-#if RS_STRICT
         double ut = (1.0 / 3.0) * u0 + (2.0 / 3.0) * u3;
         double err = 0.5 * (ut - un);
         double am = fmax(fabs(u0), fabs(un));
@@ -1673,27 +1542,16 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
         double at = err / den;
         e = e + at * at;
         Un[x] = clamp ? fmax(un, 0.0) : un;
-#else
-        // (1/3 u0 + 2/3 u3) - un in two FMAs; the factor 1/2 of the error goes onto the
-        // cell's sum as an exact 1/4
-        const double err = fma(2.0 / 3.0, u3, fma(1.0 / 3.0, u0, -un));
-        const double den = fma(amax_bits(u0, un), rtol, atol);
-        const double at = err * rcp_nr1(den);  // den >= atol > 0
-        e = fma(at, at, e);
-        // clamp at 0 on the sign bit (integer pipe); a NaN candidate fails the norm anyway
-        Un[x] = (clamp && __double2hiint(un) < 0) ? 0.0 : un;
-#endif
       }
     }
   }
-#if !RS_STRICT
-  if (STAGE == 4) e = 0.25 * e;
-#endif
   if (STAGE == 4) {
     double tot = block_tree256(e, sm);
     if (threadIdx.x == 0) B.partial[blockIdx.x] = tot;
   }
 }
+#endif  // RS_STRICT
+#include "rs_adv64.cuh"
 
 // Compensated-FP32 stage kernel (mixed precision).  The tracers of stages 1-3 stay pairs:
 // the stage input is the pencils' own (hi, lo) planes, the update q + dt/2 * (m dq/dt) / m is
@@ -1836,33 +1694,38 @@ __global__ void __launch_bounds__(kRedThreads) k_rhs_eval(DevTransport<double> T
   int j = (int)((c / T.nlon) % T.nlat);
   int k = (int)(c / ((size_t)T.nlon * T.nlat));
   CellGeo G{T.gx[j], T.gylo[j], T.gyhi[j]};
-  double divM = div_m(T, i, j, k, g, G);
-  const bool has_m = T.nsp > T.ntr;
-  double m = has_m ? Qin[(size_t)(T.nsp - 1) * nc + c] : 1.0;
-  const int nfx = T.nlon + 1, nfy = T.nlat + 1;
   const size_t ncol = (size_t)T.nlon * T.nlat, col = (size_t)j * T.nlon + i;
+  const double m = Qin[(size_t)(T.nsp - 1) * nc + c];
+#if RS_STRICT
+  double divM = div_m(T, i, j, k, g, G);
+  const int nfx = T.nlon + 1, nfy = T.nlat + 1;
   const size_t fxp = (size_t)T.nlev * T.nlat * nfx, fyp = (size_t)T.nlev * nfy * T.nlon,
                fzp = ncol * (T.nlev + 1);
   const size_t fxi = ((size_t)k * T.nlat + j) * nfx + i;
   const size_t fyi = ((size_t)k * nfy + j) * T.nlon + i;
   const size_t fzi = (size_t)k * ncol + col;
+#endif
   for (int s = 0; s < T.nsp; ++s) {
     size_t x = (size_t)s * nc + c;
-    if (s < T.ntr && T.mixed) {  // the pencils accumulated m dq/dt as a pair
-      const double ab = df_to_d(T.acc[x]);
-      const double adv = has_m ? ab / m : ab;
-      dU[x] = T.pbl ? adv + pbl_term(T, c, col, s, Qin[x]) : adv;
-      if (dUadv) dUadv[x] = adv;
-    } else if (s < T.ntr) {
-      double fw = T.fx[s * fxp + fxi], fe = T.fx[s * fxp + fxi + 1];
-      double fs = T.fy[s * fyp + fyi], fn = T.fy[s * fyp + fyi + T.nlon];
-      double fb = T.fz[s * fzp + fzi], ft = T.fz[s * fzp + fzi + ncol];
-      double Dx = (fe - fw) * G.gx;
-      double Dy = fn * G.gyhi - fs * G.gylo;
-      double Dz = ft - fb;
-      double a = -((Dx + Dy) + Dz);
-      double b = Qin[x] * divM;
-      const double adv = has_m ? (a + b) / m : a + b;
+    if (s < T.ntr) {
+      double adv;
+      if (T.mixed) {  // the kernels accumulated m dq/dt as a pair
+        adv = df_to_d(T.acc[x]) / m;
+      } else {
+#if RS_STRICT
+        double fw = T.fx[s * fxp + fxi], fe = T.fx[s * fxp + fxi + 1];
+        double fs = T.fy[s * fyp + fyi], fn = T.fy[s * fyp + fyi + T.nlon];
+        double fb = T.fz[s * fzp + fzi], ft = T.fz[s * fzp + fzi + ncol];
+        double Dx = (fe - fw) * G.gx;
+        double Dy = fn * G.gyhi - fs * G.gylo;
+        double Dz = ft - fb;
+        double a = -((Dx + Dy) + Dz);
+        double b = Qin[x] * divM;
+        adv = (a + b) / m;
+#else
+        adv = -(g * T.acc64[x]) / m;
+#endif
+      }
       dU[x] = T.pbl ? adv + pbl_term(T, c, col, s, Qin[x]) : adv;
       if (dUadv) dUadv[x] = adv;
     } else {
@@ -1879,6 +1742,7 @@ static void allow_big_smem() {
   static bool done = false;
   if (done) return;
   const int cap = kPencilSmemCap;
+#if RS_STRICT
   cudaFuncSetAttribute(k_flux_x_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_flux_y_fused<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_flux_y_fused<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
@@ -1886,6 +1750,15 @@ static void allow_big_smem() {
   cudaFuncSetAttribute(k_flux_z_fused<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_flux_z_fused<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_flux_z_fused<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+#else
+  cudaFuncSetAttribute(k_adv_x_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  cudaFuncSetAttribute(k_adv_pencil<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+#endif
   cudaFuncSetAttribute(k_adv_x_mixed<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_adv_x_mixed<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(k_adv_yz_mixed<1, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
@@ -1899,6 +1772,7 @@ static void allow_big_smem() {
   done = true;
 }
 
+#if RS_STRICT
 // Launch shape of the fused pencil kernels: V, Dd, D, E rows (n+6 each) plus the n+1 face fluxes,
 // per pencil.  Lat / vertical blocks are (pencil width 8, 16 or 32) x rows threads, at most 512;
 // the tuned width drops to 16 where 32 does not fit; a direction whose pencils do not fit even
@@ -1965,6 +1839,90 @@ static void launch_flux_one(cudaStream_t st, const DevTransport<double>& T, cons
     }
   }
 }
+void launch_scale_fluxes(cudaStream_t, const DevTransport<double>&, double*, double*, double*) {}
+#else
+// Launch shape of the FP64 kernels.  Lat / vertical pencil blocks are (pencil width 8, 16 or 32) x
+// up to `rows` threads, at most 512; a line of n cells takes n + 5 entries per phase, dealt evenly
+// over the passes it needs (51 entries at rows 32: two passes of 26, not 32 + 19).  The tuned
+// width drops to 8 where the pencils do not fit; lines that do not fit even then take the
+// thread-per-line kernel, lon rows that do not fit the thread-per-cell kernel -- the same bits.
+struct FluxShape {
+  int pw, rows, xt, xr;  // xr: lon rows per block
+  int gx, gyz;           // tracer groups (grid y)
+  size_t shx, shy, shz;
+  bool fx, fy, fz;       // shared-memory kernel used for x / y / z
+};
+static size_t pencil_bytes(int n, int pw, int nm) {
+  return (size_t)(4 * (n + 6) + nm * (n + 1)) * pw * sizeof(double);
+}
+static int even_rows(int n, int rows) {  // threads along the line for the fewest passes
+  const int passes = (n + 5 + rows - 1) / rows;
+  return (n + 5 + passes - 1) / passes;
+}
+static FluxShape flux_shape(const DevTransport<double>& T) {
+  FluxShape f;
+  f.pw = (T.pencil == 8 || T.pencil == 16) ? T.pencil : 32;
+  const size_t cap = (size_t)kPencilSmemCap;
+  while (f.pw > 8 && (pencil_bytes(T.nlat, f.pw, 2) > cap || pencil_bytes(T.nlev, f.pw, 1) > cap)) f.pw /= 2;
+  f.rows = (T.rows == 4 || T.rows == 16 || T.rows == 32) ? T.rows : 8;
+  if (f.pw * f.rows > 512) f.rows = 512 / f.pw;
+  f.xt = (T.xthreads >= 64 && T.xthreads <= 256 && T.xthreads % 32 == 0) ? T.xthreads : 128;
+  const int ntr = T.ntr > 0 ? T.ntr : 1;
+  f.gx = T.xgroups < 1 ? 1 : (T.xgroups > ntr ? ntr : T.xgroups);
+  f.gyz = T.yzgroups < 1 ? 1 : (T.yzgroups > ntr ? ntr : T.yzgroups);
+  // lon rows per block: the fewest (up to 8, within 48 KB) whose entries fill the block's last
+  // pass to within 4 %, as long as the grid still has four blocks per SM (152 SMs)
+  const int nrows = T.nlat * T.nlev, len = T.nlon + 6;
+  f.xr = 1;
+  double best = 1e30;
+  for (int r = 1; r <= 8; ++r) {
+    if (r > 1 && ((size_t)5 * len * r * sizeof(double) > 48 * 1024 || (long long)((nrows + r - 1) / r) * f.gx < 4 * 152)) break;
+    const double waste = (double)((r * len + f.xt - 1) / f.xt * f.xt) / (r * len);
+    if (waste < best - 0.04) {
+      best = waste;
+      f.xr = r;
+    }
+  }
+  f.shx = (size_t)5 * len * f.xr * sizeof(double);
+  f.shy = pencil_bytes(T.nlat, f.pw, 2);
+  f.shz = pencil_bytes(T.nlev, f.pw, 1);
+  f.fx = f.shx <= cap;
+  f.fy = f.shy <= cap && !T.yzline;
+  f.fz = f.shz <= cap && !T.yzline;
+  return f;
+}
+template <int DIR>
+static void launch_adv_yz(cudaStream_t st, const DevTransport<double>& T, const StageSel& sel,
+                          const FluxShape& f) {
+  const size_t ncol = (size_t)T.nlon * T.nlat;
+  if (!(DIR == 1 ? f.fy : f.fz)) {
+    const size_t lines = DIR == 1 ? (size_t)T.nlon * T.nlev : ncol;
+    k_adv_line<DIR><<<dim3((unsigned)((lines + kLineThreads - 1) / kLineThreads), (unsigned)T.ntr), kLineThreads, 0, st>>>(T, sel);
+    return;
+  }
+  const unsigned tiles = DIR == 1 ? (unsigned)((T.nlon + f.pw - 1) / f.pw) * (unsigned)T.nlev
+                                  : (unsigned)((ncol + f.pw - 1) / f.pw);
+  const dim3 grid(tiles, (unsigned)f.gyz), block(f.pw, even_rows(DIR == 1 ? T.nlat : T.nlev, f.rows));
+  const size_t sh = DIR == 1 ? f.shy : f.shz;
+  if (f.pw == 8) k_adv_pencil<DIR, 8><<<grid, block, sh, st>>>(T, sel);
+  else if (f.pw == 16) k_adv_pencil<DIR, 16><<<grid, block, sh, st>>>(T, sel);
+  else k_adv_pencil<DIR, 32><<<grid, block, sh, st>>>(T, sel);
+}
+static void launch_flux_one(cudaStream_t st, const DevTransport<double>& T, const StageSel& sel,
+                            const FluxShape& f, int dir) {
+  if (dir == 1) launch_adv_yz<1>(st, T, sel, f);
+  else if (dir == 2) launch_adv_yz<2>(st, T, sel, f);
+  else if (f.fx)
+    k_adv_x_rows<<<dim3((unsigned)((T.nlat * T.nlev + f.xr - 1) / f.xr), (unsigned)f.gx), f.xt, f.shx, st>>>(T, sel, f.xr);
+  else
+    k_adv_x_cell<<<dim3((unsigned)(((size_t)T.nlon * T.nlat * T.nlev + 255) / 256), (unsigned)T.ntr), 256, 0, st>>>(T, sel);
+}
+void launch_scale_fluxes(cudaStream_t st, const DevTransport<double>& T, double* mx6, double* myn6,
+                         double* mys6) {
+  const size_t n = (size_t)T.nlev * std::max((size_t)T.nlat * (T.nlon + 1), (size_t)(T.nlat + 1) * T.nlon);
+  k_scale_fluxes<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(T, mx6, myn6, mys6);
+}
+#endif
 
 // Mixed-precision pencils: the staged hi / lo rows (four with the second set of the bulk-copy
 // staging), the pair rows of the differences and slopes, and the face fluxes as pairs.
