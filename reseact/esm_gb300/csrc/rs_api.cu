@@ -401,9 +401,11 @@ struct rs_handle {
     int pc_threads = 128, pc_blocks_per_sm = 4;      // per-cell chemistry kernel
     int pc_group = 0;  // lanes per cell of the table-walking per-cell kernel (0: one thread)
     int pc_regcap = 0;  // 1: the table-walking per-cell kernel capped at 32 registers
-    int pencil = 32, rows = 8, xthreads = 128;        // transport pencil kernels
-    int xgroups = 1, yzgroups = 1;                    // their tracer groups
-    int yzline = 0;                                   // thread per lat / vertical line
+    int pc_wide = 1;    // the straight-line per-cell kernel of a large mechanism, where built
+    // FP64 transport kernels; 0 (yzline: -1): by the grid's size (flux_shape in rs_transport.cu)
+    int pencil = 0, rows = 0, xthreads = 0;
+    int xgroups = 0, yzgroups = 0;                    // tracer groups
+    int yzline = -1;                                  // thread per lat / vertical line
     int mpencil = 16, mrows = 16, mxthreads = 128;    // mixed-precision pencil kernels
     int msper_x = 1 << 20, msper_yz = 1;             // tracers per block (clamped to ntr)
     int mbulk_x = 1, mbulk_yz = 1;                    // bulk-copy staging per direction

@@ -1861,15 +1861,34 @@ static int even_rows(int n, int rows) {  // threads along the line for the fewes
 }
 static FluxShape flux_shape(const DevTransport<double>& T) {
   FluxShape f;
-  f.pw = (T.pencil == 8 || T.pencil == 16) ? T.pencil : 32;
   const size_t cap = (size_t)kPencilSmemCap;
-  while (f.pw > 8 && (pencil_bytes(T.nlat, f.pw, 2) > cap || pencil_bytes(T.nlev, f.pw, 1) > cap)) f.pw /= 2;
-  f.rows = (T.rows == 4 || T.rows == 16 || T.rows == 32) ? T.rows : 8;
-  if (f.pw * f.rows > 512) f.rows = 512 / f.pw;
-  f.xt = (T.xthreads >= 64 && T.xthreads <= 256 && T.xthreads % 32 == 0) ? T.xthreads : 128;
   const int ntr = T.ntr > 0 ? T.ntr : 1;
-  f.gx = T.xgroups < 1 ? 1 : (T.xgroups > ntr ? ntr : T.xgroups);
-  f.gyz = T.yzgroups < 1 ? 1 : (T.yzgroups > ntr ? ntr : T.yzgroups);
+  // Shapes not set by hand or by the autotuner follow the grid (measured with 12 tracers on
+  // 36x18x10, 67x45x37, 72x46x47, 144x91x47 and 30 on 180x91x72):
+  // - lat / vertical: a thread per line once there are 2,000 warps of them in both directions
+  //   (315 against 335 us on 144x91x47 with 2,538 lat warps, but 100 against 94 us on 72x46x47 with
+  //   1,242: under three warps per sub-partition the last wave is too coarse), else pencils 8 wide
+  //   with up to 32 threads along the line (every grid's fastest pencils);
+  // - pencils: tracer groups for 16 blocks per SM of the smaller direction, as a divisor of the
+  //   tracer count (36x18x10: 49 us in one group, 16 in 12; 72x46x47: 109 in one, 94 in 6);
+  // - lon rows: a row and its halo in whole warps, 128-256 threads (144x91x47: 160 threads 142 us,
+  //   128 156 us, 256 149 us), one tracer per block up to 12 groups (133 us against 142 in one).
+  const size_t ncol = (size_t)T.nlon * T.nlat;
+  const size_t warps = std::min((size_t)T.nlon * T.nlev, ncol) * ntr / 32;
+  const bool line = T.yzline < 0 ? (T.pencil == 0 && T.rows == 0 && warps >= 2000) : T.yzline != 0;
+  f.pw = T.pencil == 16 || T.pencil == 32 ? T.pencil : 8;
+  while (f.pw > 8 && (pencil_bytes(T.nlat, f.pw, 2) > cap || pencil_bytes(T.nlev, f.pw, 1) > cap)) f.pw /= 2;
+  f.rows = (T.rows == 4 || T.rows == 8 || T.rows == 16) ? T.rows : 32;
+  if (f.pw * f.rows > 512) f.rows = 512 / f.pw;
+  const int fit = std::max(128, std::min(256, (T.nlon + 6 + 31) / 32 * 32));
+  f.xt = (T.xthreads >= 64 && T.xthreads <= 256 && T.xthreads % 32 == 0) ? T.xthreads : fit;
+  f.gx = T.xgroups < 1 ? std::min(ntr, 12) : std::min(T.xgroups, ntr);
+  f.gyz = std::min(T.yzgroups, ntr);
+  if (f.gyz < 1) {
+    const size_t tiles = std::min((size_t)((T.nlon + f.pw - 1) / f.pw) * T.nlev, (ncol + f.pw - 1) / f.pw);
+    f.gyz = 1;
+    while (f.gyz < ntr && (ntr % f.gyz != 0 || tiles * f.gyz < (size_t)16 * 152)) ++f.gyz;
+  }
   // lon rows per block: the fewest (up to 8, within 48 KB) whose entries fill the block's last
   // pass to within 4 %, as long as the grid still has four blocks per SM (152 SMs)
   const int nrows = T.nlat * T.nlev, len = T.nlon + 6;
@@ -1887,8 +1906,8 @@ static FluxShape flux_shape(const DevTransport<double>& T) {
   f.shy = pencil_bytes(T.nlat, f.pw, 2);
   f.shz = pencil_bytes(T.nlev, f.pw, 1);
   f.fx = f.shx <= cap;
-  f.fy = f.shy <= cap && !T.yzline;
-  f.fz = f.shz <= cap && !T.yzline;
+  f.fy = f.shy <= cap && !line;
+  f.fz = f.shz <= cap && !line;
   return f;
 }
 template <int DIR>
