@@ -855,7 +855,7 @@ void chem_attempt(rs_handle* h, Ctl* c) {
                              h->cfg.atol_C, h->cfg.clamp_nonneg, h->fsal[0].p, h->fsal[1].p);
   }
   Scope s(h, "finalize");
-  rs::launch_finalize(h->st, c, h->partial.p, (int)((h->nc + 255) / 256));
+  rs::launch_finalize(h->st, c, h->partial.p, rs::ros23_parts(h->lc));
   if (h->rec_on) rs::launch_tape_store(h->st, c, h->U[0].p, h->U[1].p, h->nc * h->nsp);
   h->launches += 2;
 }
@@ -895,7 +895,7 @@ void build_loop_graph(rs_handle* h, int slot) {
   CK(cudaStreamBeginCaptureToGraph(h->cap, body, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeRelaxed));
   Ctl* c = h->ctl.p + slot;
-  int nparts = (int)((h->nc + 255) / 256);
+  const int nparts = slot == 0 ? (int)((h->nc + 255) / 256) : rs::ros23_parts(h->lc);
   if (slot == 0) {
     rs::TransportBufs B{h->U[0].p, h->U[1].p, h->S1.p, h->S2.p, h->S3.p, h->partial.p};
     rs::launch_ssprk43_attempt(h->cap, h->dt, c, B, h->cfg.rtol_T, h->cfg.atol_T,
@@ -1041,7 +1041,7 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
     size_t n = h->nc * h->nsp;
     h->U[0].alloc(n); h->U[1].alloc(n);
     h->U[0].zero(h->st); h->U[1].zero(h->st);
-    h->partial.alloc((h->nc + 255) / 256 + 1);
+    h->partial.alloc(std::max<size_t>((h->nc + 255) / 256, (size_t)rs::ros23_parts(h->lc)) + 1);
     h->krates.alloc(std::max<size_t>(1, (size_t)T.nr * h->nc));
     h->krates.zero(h->st);
     h->ctl.alloc(3);
@@ -1607,7 +1607,8 @@ rs_status rs_single_step(rs_handle* h, int32_t op, double t, double dt, const do
       rs::launch_ros23_attempt(h->lc, c, a, b, h->krates.p, h->have_emis ? h->emis.p : nullptr,
                                h->partial.p, h->cfg.rtol_C, h->cfg.atol_C, 0);
     }
-    rs::launch_finalize(h->st, c, h->partial.p, (int)((h->nc + 255) / 256));
+    rs::launch_finalize(h->st, c, h->partial.p,
+                        op == RS_OP_TRANSPORT ? (int)((h->nc + 255) / 256) : rs::ros23_parts(h->lc));
     rs::launch_to_cellmajor(h->st, b, h->io.p, h->nlon, h->nlat, h->nlev, h->nsp);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(u_out, h->io.p, n * sizeof(double), cudaMemcpyDeviceToHost, h->st));
@@ -2831,7 +2832,7 @@ extern "C" rs_status rs_ros23_attempt_noalloc(rs_handle* h, double dt, const dou
     rs::launch_ros23_attempt(h->lc, ctl, const_cast<double*>(d_u_in), d_u_out, h->krates.p,
                              h->have_emis ? h->emis.p : nullptr, part, h->cfg.rtol_C,
                              h->cfg.atol_C, 0);
-    rs::launch_finalize(h->st, ctl, part, (int)((h->nc + rs::kRedThreads - 1) / rs::kRedThreads));
+    rs::launch_finalize(h->st, ctl, part, rs::ros23_parts(h->lc));
     CK(cudaGetLastError());
     if (eest) {
       CK(cudaMemcpyAsync(&h->hctl[2], ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, h->st));

@@ -654,6 +654,10 @@ void launch_ros23_attempt(const LaunchCtx& L, const Ctl* ctl, double* U0, double
   if (L.size_class == 0) Small::attempt(L, ctl, U0, U1, kr, em, part, rtol, atol, clamp);
   else Large::attempt(L, ctl, U0, U1, kr, em, part, rtol, atol, clamp);
 }
+int ros23_parts(const LaunchCtx& L) {
+  const int block = L.jit ? jit_attempt_block(L.nc) : kRedThreads;
+  return (L.nc + block - 1) / block;
+}
 void launch_ros23_step(const LaunchCtx& L, const Ctl* ctl, double* U0, double* U1,
                        const double* kr, const double* em, double* part, double rtol,
                        double atol, int clamp) {

@@ -428,9 +428,18 @@ __device__ __forceinline__ double quant_dt(double d) {
   return __longlong_as_double(__double_as_longlong(d) & ~((1ll << 48) - 1));
 }
 
-// pairwise tree over 256 lanes, v[t] += v[t+s] for s = 128 ... 1; total in thread 0
-__device__ __forceinline__ double tree256(double v, double* sm) {
+// block total of v in thread 0: strict build (256 threads), the oracle's pairwise tree v[t] +=
+// v[t+s] for s = 128 ... 1; production build, a shuffle tree per warp and the warps' sums in
+// order (whole warps, at most 8)
+__device__ __forceinline__ double block_total(double v, double* sm) {
   const int t = threadIdx.x;
+#if !RS_STRICT
+  for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
+  if ((t & 31) == 0) sm[t >> 5] = v;
+  __syncthreads();
+  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v += sm[w];
+  return v;
+#else
   sm[t] = v;
   __syncthreads();
   for (int s = 128; s >= 32; s >>= 1) {
@@ -467,7 +476,7 @@ std::string generate(const MechTables& T, double ros_d, double ros_c32, bool str
     << offsetof(Ctl, iters) << "\n#define OFF_NACC " << offsetof(Ctl, nacc)
     << "\n#define OFF_KZ " << offsetof(Ctl, kz) << "\n#define OFF_KZCAP "
     << offsetof(Ctl, kzcap) << "\n";
-  o << kPrelude;
+  o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude;
   // Every multiply-add is written out: RS_FMA fuses in the production build and keeps the
   // multiply and the add separate in the strict build; both builds compile with --fmad=false,
   // so no compiler contraction decides anything and all variants compute the same bits.
@@ -639,7 +648,7 @@ __device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ c
       Un[(u64)s * N + c] = clamp ? fmax(xv, 0.0) : xv;
     }
   }
-  const double tot = tree256(e, red);
+  const double tot = block_total(e, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = tot;
 }
 
@@ -1060,6 +1069,21 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
   return J;
 }
 
+// An FP64 warp instruction takes 64 cycles of its SM sub-partition, so a block's warps cost most
+// where they stack on few SMs or leave a coarse last wave: 64 threads while 128-cell blocks would
+// leave SMs idle (152 SMs; 36x18x10, 6,480 cells: 73 us per attempt at 256 threads, 40 at 64),
+// 128 above (314,900 cells: 609 -> 574 us; 155,664: 300 -> 295; 615,888: 1,075 -> 1,070), 256 from
+// 4 M cells on, where the last wave is nothing and the partial sums would outnumber the
+// allocation-free attempt's scratch.  The strict build keeps the oracle's 256-cell partial sums.
+int jit_attempt_block(int nc) {
+#if RS_STRICT
+  (void)nc;
+  return kBlock;
+#else
+  return nc <= 152 * 128 ? 64 : (nc <= (1 << 22) ? 128 : kBlock);
+#endif
+}
+
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                         double* U0, double* U1, const double* kr, const double* em,
                         double* part, double rtol, double atol, int clamp, double* F0,
@@ -1069,8 +1093,8 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
   if (!F0 || !F1) F0 = F1 = nullptr;
   void* args[] = {&c, &U0, &U1, &kr, &em, &part, &nc, &nsp, &rtol, &atol, &clamp, &F0, &F1};
-  int nb = (nc + kBlock - 1) / kBlock;
-  cudaLaunchKernel((const void*)k, dim3(nb), dim3(kBlock), args, J.attempt_smem[v], st);
+  const int block = jit_attempt_block(nc);
+  cudaLaunchKernel((const void*)k, dim3((nc + block - 1) / block), dim3(block), args, J.attempt_smem[v], st);
 }
 
 void jit_launch_step(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,

@@ -60,6 +60,9 @@ std::string jit_chem_source(const MechTables& T, bool strict);
 bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<char>* cubin,
                  std::string* log);
 
+// Threads per block of the attempt kernels over nc cells (one partial sum per block).
+int jit_attempt_block(int nc);
+
 // Same contracts as launch_ros23_attempt / launch_chem_per_cell in rs_kernels.h.
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                         double* U0, double* U1, const double* kr, const double* em,

@@ -118,6 +118,8 @@ void launch_rates(const LaunchCtx& L, const double* T, const double* P, double* 
 void launch_ros23_attempt(const LaunchCtx& L, const Ctl* ctl, double* U0, double* U1,
                           const double* kr, const double* em, double* part, double rtol,
                           double atol, int clamp, double* F0 = nullptr, double* F1 = nullptr);
+// Partial sums of the error norm that an attempt over this many cells writes (its block count).
+int ros23_parts(const LaunchCtx& L);
 // One step at the controller's dtc that is accepted whatever its error (the replay of a
 // recorded step): the specialised kernels skip the error estimate; the table kernels run the
 // full attempt (part: its block partials, unused).  Same new state as launch_ros23_attempt.
