@@ -800,6 +800,10 @@ Ctl make_ctl(rs_handle* h, double t0, double t1, double dt0, const rs_controller
   k.qsmin = c.qsteady_min; k.qsmax = c.qsteady_max; k.qoldinit = c.qoldinit;
   k.ntot = ntot; k.omega = h->omega;
   k.ros_d = h->dm.ros_d;
+  k.rntot = 1.0 / ntot;
+  k.rgamma = 1.0 / c.gamma;
+  k.qmaxv = c.qmax;
+  k.qminv = c.qmin;
   k.seq = nullptr;
   k.nseq = nullptr;
   k.seqcap = 0;
@@ -1391,6 +1395,7 @@ rs_status rs_macro_step(rs_handle* h, double t0, double t1, double* dtT, double*
     if (h->cfg.do_chemistry && okT) {
       if (h->cfg.chem_mode == RS_CHEM_GLOBAL_DT) {
         Ctl init = make_ctl(h, t0, t1, *dtC, h->cfg.ctrl_C, ntot);
+        init.omega = 0.0;  // the flux time factors belong to the transport half
         init.cur = h->cur;
         if (h->rec_on) {
           init.seq = h->seqbuf.p + (size_t)2 * seqcap;

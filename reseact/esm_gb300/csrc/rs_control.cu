@@ -15,6 +15,7 @@
 
 namespace rs {
 
+#if RS_STRICT
 __device__ void prepare_next(Ctl* c) {
   c->dtc = fmin(c->dt, c->tend - c->t);
   c->dto2 = c->dtc / 2;
@@ -77,6 +78,101 @@ __device__ void finalize_body(Ctl* __restrict__ c, const double* __restrict__ pa
   c->iters += 1.0;
   prepare_next(c);
 }
+#else
+// Production close-out.  The chain from the partial sums to the next step size is serial FP64
+// work -- 64 cycles an instruction on this GPU, so a pow is ~2 us -- and the attempts wait for it.
+// It is spread over the block's warps, which run on different sub-partitions: six warps add the
+// partial sums while the other two form qold^+-b2; then x = sse / ntot = EEst^2 goes into
+// x^(+-b1/2) in two warps (no square root on the chain, and no division: every quotient of the
+// controller is a product with one of the inverse powers) while a third forms EEst.  The time
+// factors of the next transport attempt are three cosines in three warps.  17-22 -> 14-15 us per
+// attempt between events (launch included).
+__device__ void next_step(Ctl* c) {
+  c->dtc = fmin(c->dt, c->tend - c->t);
+  c->dto2 = 0.5 * c->dtc;
+  c->dto6 = c->dtc * (1.0 / 6.0);
+  c->dtgamma = c->dtc * c->ros_d;
+  c->done = !((c->t < c->tend - 1.0e-9) && (c->iters < c->maxiters));
+}
+// time factors at the stages: t, t + dt/2, t + dt, t + dt/2 (one warp each; all of the block's
+// threads call this)
+__device__ void stage_factors(Ctl* c) {
+  const int w = threadIdx.x >> 5;
+  if (w > 2 || (threadIdx.x & 31) != 0) return;
+  const double v = c->omega != 0.0 ? cos(c->omega * (c->t + 0.5 * (double)w * c->dtc)) : 1.0;
+  c->g[w] = v;
+  if (w == 1) c->g[3] = v;
+}
+constexpr int kSumWarps = 6;
+__device__ void finalize_body(Ctl* __restrict__ c, const double* __restrict__ partial,
+                              int nparts, double* sm) {
+  if (c->done) return;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w < kSumWarps) {
+    double acc = 0.0;
+    for (int q = threadIdx.x; q < nparts; q += kSumWarps * 32) acc = acc + partial[q];
+    for (int s = 16; s > 0; s >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, s);
+    if (lane == 0) sm[w] = acc;
+  } else {
+    const double p = pow(c->qold, w == 6 ? c->beta2 : -c->beta2);
+    if (lane == 0) sm[w] = p;
+  }
+  __syncthreads();
+  double sse = sm[0];
+  for (int q = 1; q < kSumWarps; ++q) sse += sm[q];
+  double x = sse * c->rntot;
+  if (isnan(x)) x = 1.0e20;  // reject (EEst 1e10)
+  if (w < 2) {
+    const double p = pow(fmax(x, 1.0e-70), w == 0 ? 0.5 * c->beta1 : -0.5 * c->beta1);
+    if (lane == 0) sm[8 + w] = p;
+  } else if (w == 2) {
+    const double e = sqrt(x);
+    if (lane == 0) sm[10] = e;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double q11 = sm[8], q11i = sm[9], qden = sm[6], qdeni = sm[7], EEst = sm[10];
+    const double dtc = c->dtc;
+    c->eest = EEst;
+    const bool accept = EEst <= 1.0;
+    c->accept = accept;
+    if (accept) {
+      // q = q11 / qden / gamma within [invqmax, invqmin], dt / q (1 in the steady band)
+      const double rg = c->rgamma;
+      const double q = fmax(c->invqmax, fmin(c->invqmin, q11 * qdeni * rg));
+      const double qi = fmin(c->qmaxv, fmax(c->qminv, q11i * qden * c->gamma));
+      if (c->seq) {
+        int k = *c->nseq;
+        if (k < c->seqcap) {
+          c->seq[2 * k] = c->t;
+          c->seq[2 * k + 1] = dtc;
+        }
+        *c->nseq = k + 1;
+      }
+      c->cur ^= 1;
+      c->t = c->t + dtc;
+      c->dt = (c->qsmin <= q) && (q <= c->qsmax) ? dtc : dtc * qi;
+      c->qold = fmax(EEst, c->qoldinit);
+      c->nacc += 1.0;
+    } else {
+      c->dt = dtc * fmax(c->qminv, q11i * c->gamma);
+      c->nrej += 1.0;
+    }
+    c->iters += 1.0;
+    next_step(c);
+  }
+  if (c->omega != 0.0) {  // written once, at the controller's start
+    __syncthreads();
+    stage_factors(c);
+  }
+}
+__device__ void prepare_next(Ctl* c) {  // one thread: the first attempt of a solve
+  next_step(c);
+  for (int q = 0; q < 3; ++q)
+    c->g[q] = c->omega != 0.0 ? cos(c->omega * (c->t + 0.5 * (double)q * c->dtc)) : 1.0;
+  c->g[3] = c->g[1];
+}
+#endif
 
 __global__ void __launch_bounds__(kRedThreads) k_finalize(Ctl* __restrict__ c,
                                                           const double* __restrict__ partial,

@@ -95,6 +95,7 @@ struct Ctl {
   double g[4];     // SSPRK43 stage factors of the next attempt: t, t+dt/2, t+dt, t+dt/2
   double dto2, dto6, dtgamma;  // dtc/2, dtc/6, dtc*d of the next attempt (shared by all cells)
   double ros_d;    // ROS23 d, for dtgamma
+  double rntot, rgamma, qmaxv, qminv;  // 1/ntot, 1/gamma, 1/invqmax, 1/invqmin (production build's close-out)
   double* seq;     // if set: accepted (t, dt) pairs are appended here (adjoint recording)
   int* nseq;
   int seqcap;
