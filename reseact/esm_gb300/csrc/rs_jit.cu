@@ -455,6 +455,7 @@ __device__ __forceinline__ double block_total(double v, double* sm) {
   }
   __syncthreads();
   return a;
+#endif
 }
 )";
 
