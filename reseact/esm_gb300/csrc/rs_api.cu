@@ -424,6 +424,9 @@ struct rs_handle {
   bool fixer_on = false;
   DevBuf<double> mcorr;
   std::shared_ptr<rs::JitChem> jit;
+  // straight-line forms of the table-walking kernel this handle's mode runs, for mechanisms too
+  // large for jit (null: not built)
+  std::shared_ptr<rs::WideChem> wide;
   DevBuf<double> fsal[2];  // f(U[b]) planes [ns][nc] for the specialised global-dt attempts
   std::string jit_why;
   int chem_kernel = RS_CHEM_KERNEL_AUTO;
@@ -1038,6 +1041,12 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
     h->lc = rs::LaunchCtx{h->st, h->dm, (int)h->nc, h->nsp, cls};
     h->jit = rs::jit_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32, RS_STRICT != 0, &h->jit_why);
     h->lc.jit = h->jit.get();
+    if (!h->jit && cfg->do_chemistry) {
+      std::string why;
+      h->wide = rs::wide_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32,
+                                    cfg->chem_mode == RS_CHEM_PER_CELL, &why);
+      h->lc.wide = h->wide.get();
+    }
     if (h->jit && cfg->do_chemistry && cfg->chem_mode == RS_CHEM_GLOBAL_DT) {
       h->fsal[0].alloc((size_t)T.ns * h->nc);
       h->fsal[1].alloc((size_t)T.ns * h->nc);
@@ -1432,7 +1441,8 @@ rs_status rs_macro_step(rs_handle* h, double t0, double t1, double* dtT, double*
         int thr = h->tune.pc_threads;
         int nblocks = std::max(1, std::min(nsm * h->tune.pc_blocks_per_sm,
                                            (int)((h->nc + thr - 1) / thr)));
-        const int G = h->lc.jit ? 0 : h->tune.pc_group;
+        const bool wide = !h->lc.jit && h->lc.wide && h->wide->per_cell && h->tune.pc_wide;
+        const int G = h->lc.jit || wide ? 0 : h->tune.pc_group;
         if (G > 0) {  // a persistent grid of resident blocks, one cell per G lanes
           thr = rs::chem_group_threads(h->lc, G);
           const int bps = rs::chem_group_blocks_per_sm(h->lc, G, thr);
@@ -1441,7 +1451,11 @@ rs_status rs_macro_step(rs_handle* h, double t0, double t1, double* dtT, double*
         }
         {
           Scope s(h, "chem_per_cell");
-          if (G > 0)
+          if (wide)
+            rs::wide_launch_per_cell(*h->wide, h->st, nsm, (int)h->nc, h->nsp, h->U[h->cur].p, h->krates.p,
+                                     h->have_emis ? h->emis.p : nullptr, h->dtcell.p, h->stepcell.p,
+                                     h->queue.p, h->flag.p, a);
+          else if (G > 0)
             rs::launch_chem_per_cell_group(h->lc, G, nblocks, thr, h->U[h->cur].p, h->krates.p,
                                            h->have_emis ? h->emis.p : nullptr, h->dtcell.p,
                                            h->stepcell.p, h->queue.p, h->flag.p, a);
@@ -2040,6 +2054,7 @@ extern "C" rs_status rs_set_chem_kernel(rs_handle* h, int32_t kind) {
       throw RsError(RS_ERR_UNSUPPORTED, "specialised chemistry kernels unavailable: " + h->jit_why);
     h->chem_kernel = kind;
     h->lc.jit = (kind == RS_CHEM_KERNEL_TABLE) ? nullptr : h->jit.get();
+    h->lc.wide = (kind == RS_CHEM_KERNEL_TABLE) ? nullptr : h->wide.get();
     invalidate_graphs(h);
   });
 }
@@ -2062,7 +2077,8 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
                       h->jit->regs[0], h->jit->regs[1], h->jit->regs[2], h->jit->regs[3],
                       h->jit->attempt_smem[1], h->jit->attempt_smem[3], h->jit->compile_ms);
       else
-        std::snprintf(line, sizeof line, "{\"kind\": \"table\", \"why\": \"%.600s\"}", why.c_str());
+        std::snprintf(line, sizeof line, "{\"kind\": \"table\", \"wide\": %s, \"why\": \"%.600s\"}",
+                      h->lc.wide ? "true" : "false", why.c_str());
       std::strncpy(info, line, info_len - 1);
       info[info_len - 1] = 0;
     }
@@ -2097,9 +2113,12 @@ extern "C" rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t 
     else if (k == "mixed_yz_bulk") ok = in({0, 1}) && (t.mbulk_yz = value, true);
     else if (k == "mixed_x_stream") ok = in({0, 1}) && (t.mstream_x = value, true);
     else if (k == "mixed_yz_stream") ok = in({0, 1}) && (t.mstream_yz = value, true);
-    else if (k == "per_cell_threads") ok = in({64, 128, 256}) && (t.pc_threads = value, true);
-    else if (k == "per_cell_blocks_per_sm") ok = in({1, 2, 4, 8, 16}) && (t.pc_blocks_per_sm = value, true);
-    else if (k == "per_cell_regcap") ok = in({0, 1}) && (t.pc_regcap = value, true);
+    // a shape of the table-walking per-cell kernels selects them; per_cell_wide 1 selects the
+    // straight-line kernel of a large mechanism again, where it is built
+    else if (k == "per_cell_threads") ok = in({64, 128, 256}) && (t.pc_threads = value, t.pc_wide = 0, true);
+    else if (k == "per_cell_blocks_per_sm") ok = in({1, 2, 4, 8, 16}) && (t.pc_blocks_per_sm = value, t.pc_wide = 0, true);
+    else if (k == "per_cell_regcap") ok = in({0, 1}) && (t.pc_regcap = value, t.pc_wide = 0, true);
+    else if (k == "per_cell_wide") ok = in({0, 1}) && (value == 0 || (h->wide && h->wide->per_cell)) && (t.pc_wide = value, true);
     else if (k == "chem_attempt_variant") {  // the specialised attempt kernel's variant
       ok = value >= 0 && value < rs::kJitVariants && h->jit && h->jit->attempt[value][0];
       if (ok) h->jit->variant = value;
@@ -2108,7 +2127,7 @@ extern "C" rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t 
       // G lanes per cell: the production build's (minimum-fill, descending back substitution)
       // table-walking kernels only, and only where a block of them fits in shared memory
       ok = in({0, 4, 8, 16}) && (value == 0 || (!RS_STRICT && rs::chem_group_threads(h->lc, value) > 0));
-      if (ok) t.pc_group = value;
+      if (ok) t.pc_group = value, t.pc_wide = 0;
     }
     else throw RsError(RS_ERR_INVALID, "unknown launch-shape key: " + k);
     if (!ok) throw RsError(RS_ERR_INVALID, "value out of range for " + k);
@@ -2504,10 +2523,27 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
             h->tune.pc_regcap = 0;
           }
         }
+      if (!h->lc.jit && h->wide && h->wide->per_cell) {
+        const float ms = time_min(h->st, 2, [&] {
+          cudaMemcpyAsync(h->io2.p, h->U[h->cur].p, n * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
+          cudaMemsetAsync(h->io.p, 0, h->nc * sizeof(double), h->st);
+          cudaMemsetAsync(h->queue.p, 0, sizeof(unsigned long long), h->st);
+          rs::wide_launch_per_cell(*h->wide, h->st, nsm, (int)h->nc, h->nsp, h->io2.p, h->krates.p,
+                                   h->have_emis ? h->emis.p : nullptr, h->io.p, nullptr, h->queue.p,
+                                   h->flag.p, a);
+        });
+        // three attempts per cell fit the table-walking kernels, whose 2,048 threads per SM then
+        // all finish together; over a whole window with uneven step counts their warps run as
+        // long as their slowest cell, so the straight-line kernel is kept unless it is far behind
+        h->tune.pc_wide = ms < 2.0f * best;
+        std::snprintf(line, sizeof line, "], \"per_cell_wide\": [{\"ms\": %.4f}", ms);
+        rep += line;
+      }
       std::snprintf(line, sizeof line,
                     "], \"per_cell_choice\": {\"threads\": %d, \"blocks_per_sm\": %d, \"group\": %d, "
-                    "\"regcap\": %d}",
-                    h->tune.pc_threads, h->tune.pc_blocks_per_sm, h->tune.pc_group, h->tune.pc_regcap);
+                    "\"regcap\": %d, \"wide\": %d}",
+                    h->tune.pc_threads, h->tune.pc_blocks_per_sm, h->tune.pc_group, h->tune.pc_regcap,
+                    !h->lc.jit && h->wide && h->wide->per_cell && h->tune.pc_wide);
       rep += line;
     }
     if (h->cfg.do_chemistry && h->cfg.chem_mode == RS_CHEM_GLOBAL_DT && h->lc.jit) {

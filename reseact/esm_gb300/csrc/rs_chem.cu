@@ -651,6 +651,10 @@ void launch_ros23_attempt(const LaunchCtx& L, const Ctl* ctl, double* U0, double
                        clamp, F0, F1);
     return;
   }
+  if (L.wide && L.wide->attempt) {
+    wide_launch_attempt(*L.wide, L.stream, L.nc, L.nsp, ctl, U0, U1, kr, em, part, rtol, atol, clamp);
+    return;
+  }
   if (L.size_class == 0) Small::attempt(L, ctl, U0, U1, kr, em, part, rtol, atol, clamp);
   else Large::attempt(L, ctl, U0, U1, kr, em, part, rtol, atol, clamp);
 }

@@ -18,6 +18,7 @@
 #include <dlfcn.h>
 #include <nvrtc.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstddef>
@@ -585,7 +586,7 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
 #undef WV
 }
 
-// global-dt attempt: every cell steps with the controller's dtc; 256-cell block partials.
+// global-dt attempt: every cell steps with the controller's dtc; one partial sum per block.
 // F0/F1 (may be null) pair with U0/U1: F[cur] holds f(U[cur]) per cell (NaN in plane 0 where
 // unknown); from the second attempt of a solve on, a cell reuses it instead of evaluating
 // f(x) again (the first attempt of a solve starts from a state written elsewhere).
@@ -914,6 +915,353 @@ extern "C" __global__ void rs_jit_rcp(const double* __restrict__ x, double* __re
   return o.str();
 }
 
+// ------------------------------------------------------------------ wide mechanisms
+// Mechanisms too large for the kernels above (their work arrays do not fit a thread's registers)
+// get straight-line forms of the two table-walking kernels that run whole solves,
+// k_ros23_attempt and k_chem_per_cell, with the same operations in the same order: the same bits.
+// What they gain is the table walk itself (an index load in front of every operand) and where the
+// work arrays live.  FP64 issues one warp instruction per 64 cycles and SM sub-partition, so two
+// warps per sub-partition (one 256-thread block per SM) are enough, and at that occupancy
+//   - the least-used LU slots of W, 112 of them, sit in shared memory ([slot][thread]) and the
+//     others in registers or their spills: volatile accesses and compiler barriers keep the
+//     compiler from promoting shared slots to registers and spilling those;
+//   - f, the partials and the Jacobian are formed reaction by reaction (each sum still adds its
+//     terms in ascending order), so no rate or partial outlives its reaction;
+//   - rate constants are loaded in groups one group ahead.
+// 30 species, 60 reactions, 290 slots (3,400 FP64 instructions an attempt, 5.4 ns per cell at the
+// FP64 pipe's rate): 12.4 -> 6.8 ns per cell-attempt against k_ros23_attempt (128 threads per SM
+// with 226 shared slots: 7.4 ns; W in registers and spills alone: 8.4 ns).
+constexpr int kWideSlots = (int)((227 * 1024 - 2 * kBlock * sizeof(double)) / (kBlock * sizeof(double)));
+
+bool wide_eligible(const MechTables& T) {
+  if (T.ns < 1 || T.ns > 64 || T.nlu > 640 || T.nr > 256) return false;
+  for (int e = 0; e < T.njac; ++e)  // the Jacobian's terms arrive with ascending partials
+    for (int t = T.jac_ptr[e] + 1; t < T.jac_ptr[e + 1]; ++t)
+      if (T.jac_part[t] <= T.jac_part[t - 1]) return false;
+  return true;
+}
+int wide_reg_slots(const MechTables& T) { return T.nlu > kWideSlots ? T.nlu - kWideSlots : 0; }
+size_t wide_smem_bytes(const MechTables& T) {
+  return (size_t)(T.nlu - wide_reg_slots(T)) * kBlock * sizeof(double);
+}
+
+struct WideGen {
+  const MechTables& T;
+  bool per_cell;
+  std::ostringstream o;
+  std::vector<int> place;  // position of each slot, hottest first: < KR in a register
+  int KR = 0;
+  static constexpr int kGroup = 10;  // rate constants loaded together
+
+  void rank_slots() {
+    std::vector<long> use(T.nlu, 0);
+    for (int k = 0; k < T.ns; ++k) use[T.lu_diag[k]] += 5;
+    for (size_t m = 0; m < T.elim_lik.size(); ++m) {
+      use[T.elim_lik[m]] += 2;
+      for (int u = T.upd_ptr[m]; u < T.upd_ptr[m + 1]; ++u) {
+        use[T.upd_dst[u]] += 2;
+        use[T.upd_src[u]] += 1;
+      }
+    }
+    for (int sl : T.low_slot) use[sl] += 3;
+    for (int sl : T.up_slot) use[sl] += 3;
+    std::vector<int> by(T.nlu);
+    for (int i = 0; i < T.nlu; ++i) by[i] = i;
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return use[a] > use[b]; });
+    place.assign(T.nlu, 0);
+    for (int i = 0; i < T.nlu; ++i) place[by[i]] = i;
+    KR = wide_reg_slots(T);
+  }
+  std::string w(int slot) const {
+    const int p = place[slot];
+    return p < KR ? "W" + std::to_string(p) : "S[" + std::to_string((p - KR) * kBlock) + "]";
+  }
+  static std::string nm(const char* v, int s) { return v + std::to_string(s); }
+  void fence() { o << "  RS_FENCE\n"; }
+  void load_rates(int g) {
+    for (int r = g; r < std::min(T.nr, g + kGroup); ++r) o << "  LDK(" << r << ")\n";
+  }
+  // one term of a running sum: dst = c * v or dst + c * v, as fma(c, v, dst) of the tables
+  // (c = +-1: the same value as an add)
+  static std::string term(const std::string& dst, bool first, double c, const char* v) {
+    if (first) return dst + " = " + (c == 1.0 ? std::string(v) : c == -1.0 ? "-" + std::string(v) : lit(c) + " * " + v) + ";";
+    if (c == 1.0) return dst + " = " + dst + " + " + v + ";";
+    if (c == -1.0) return dst + " = " + dst + " - " + v + ";";
+    return dst + " = fma(" + lit(c) + ", " + v + ", " + dst + ");";
+  }
+  void rhs(const char* x, const char* f) {
+    std::vector<std::vector<std::pair<int, double>>> per(T.nr);
+    for (int sp = 0; sp < T.ns; ++sp)
+      for (int t = T.rhs_ptr[sp]; t < T.rhs_ptr[sp + 1]; ++t) per[T.rhs_r[t]].push_back({sp, T.rhs_c[t]});
+    std::vector<char> seen(T.ns, 0);
+    o << "  {\n";
+    load_rates(0);
+    for (int g = 0; g < T.nr; g += kGroup) {
+      load_rates(g + kGroup);
+      for (int r = g; r < std::min(T.nr, g + kGroup); ++r) {
+        o << "  { const double v = K" << r;
+        for (int q = T.rptr[r]; q < T.rptr[r + 1]; ++q)
+          for (int t = 0; t < T.rnu[q]; ++t) o << " * " << nm(x, T.rsp[q]);
+        o << ";\n";
+        for (auto& sc : per[r]) {
+          o << "    " << term(nm(f, sc.first), !seen[sc.first], sc.second, "v") << "\n";
+          seen[sc.first] = 1;
+        }
+        o << "  }\n";
+      }
+    }
+    for (int sp = 0; sp < T.ns; ++sp)
+      if (!seen[sp]) o << "  " << nm(f, sp) << " = 0.0;\n";
+    o << "  }\n  if (em) {\n";
+    for (int sp = 0; sp < T.ns; ++sp) o << "  " << nm(f, sp) << " = " << nm(f, sp) << " + EM(" << sp << ");\n";
+    o << "  }\n";
+  }
+  void build_w() {
+    std::vector<std::vector<std::pair<int, double>>> per(T.npart);  // partial -> (entry, coefficient)
+    for (int e = 0; e < T.njac; ++e)
+      for (int t = T.jac_ptr[e]; t < T.jac_ptr[e + 1]; ++t) per[T.jac_part[t]].push_back({e, T.jac_coef[t]});
+    std::vector<char> seen(T.njac, 0), is_jac(T.nlu, 0), is_diag(T.nlu, 0);
+    for (int e = 0; e < T.njac; ++e) is_jac[T.jac_slot[e]] = 1;
+    for (int k = 0; k < T.ns; ++k) is_diag[T.lu_diag[k]] = 1;
+    o << "  {\n";
+    load_rates(0);
+    int p = 0;
+    for (int g = 0; g < T.nr; g += kGroup) {
+      load_rates(g + kGroup);
+      for (int r = g; r < std::min(T.nr, g + kGroup); ++r) {
+        for (; p < T.npart && T.part_r[p] == r; ++p) {
+          o << "  { const double P = K" << r;
+          for (int q = T.rptr[r]; q < T.rptr[r + 1]; ++q) {
+            const int sp = T.rsp[q], nu = T.rnu[q];
+            if (sp == T.part_q[p]) {
+              if (nu < 2) continue;
+              o << " * (" << lit((double)nu);
+              for (int t = 1; t < nu; ++t) o << " * " << nm("x", sp);
+              o << ")";
+            } else {
+              for (int t = 0; t < nu; ++t) o << " * " << nm("x", sp);
+            }
+          }
+          o << ";\n";
+          for (auto& ec : per[p]) {
+            o << "    " << term(w(T.jac_slot[ec.first]), !seen[ec.first], ec.second, "P") << "\n";
+            seen[ec.first] = 1;
+          }
+          o << "  }\n";
+        }
+        fence();
+      }
+    }
+    for (int e = 0; e < T.nlu; ++e) {
+      const char* d = is_diag[e] ? "1.0" : "0.0";
+      if (is_jac[e]) o << "  " << w(e) << " = fma(-dtg, " << w(e) << ", " << d << ");\n";
+      else o << "  " << w(e) << " = " << d << ";\n";
+      if (e % 8 == 7) fence();
+    }
+    o << "  }\n";
+  }
+  // the pivot's reciprocal takes the place of U_kk, which nothing reads again
+  void lu_factor() {
+    int m = 0;
+    for (int k = 0; k < T.ns; ++k) {
+      fence();
+      const std::string d = w(T.lu_diag[k]);
+      o << "  { const double pk = rcp_nr(" << d << ");\n  " << d << " = pk;\n";
+      for (int ii = T.elim_ptr[k]; ii < T.elim_ptr[k + 1]; ++ii, ++m) {
+        const std::string l = w(T.elim_lik[ii]);
+        o << "  { const double mu = " << l << " * pk;\n";
+        for (int u = T.upd_ptr[m]; u < T.upd_ptr[m + 1]; ++u)
+          o << "    " << w(T.upd_dst[u]) << " = fma(-mu, " << w(T.upd_src[u]) << ", " << w(T.upd_dst[u]) << ");\n";
+        o << "    " << l << " = mu; }\n";
+      }
+      o << "  }\n";
+    }
+  }
+  void solve(const char* b) {
+    fence();
+    for (int k = 0; k < T.ns; ++k) {
+      if (k % 4 == 3) fence();
+      for (int e = T.low_ptr[k]; e < T.low_ptr[k + 1]; ++e)
+        o << "  " << nm(b, T.low_row[e]) << " = fma(-" << w(T.low_slot[e]) << ", " << nm(b, T.ord[k]) << ", "
+          << nm(b, T.low_row[e]) << ");\n";
+    }
+    for (int i = T.ns - 1; i >= 0; --i) {
+      if (i % 4 == 3) fence();
+      const std::string bi = nm(b, T.ord[i]);
+      for (int e = T.up_ptr[i]; e < T.up_ptr[i + 1]; ++e)
+        o << "  " << bi << " = fma(-" << w(T.up_slot[e]) << ", " << nm(b, T.up_col[e]) << ", " << bi << ");\n";
+      o << "  " << bi << " = " << bi << " * " << w(T.lu_diag[i]) << ";\n";
+    }
+  }
+  void each(const std::string& text) {  // text with # for the species
+    for (int sp = 0; sp < T.ns; ++sp) {
+      std::string t = text;
+      for (size_t i; (i = t.find('#')) != std::string::npos;) t.replace(i, 1, std::to_string(sp));
+      o << "  " << t << "\n";
+    }
+  }
+  void decl(const char* v, const char* init = "") {
+    o << "  double ";
+    for (int sp = 0; sp < T.ns; ++sp) o << (sp ? ", " : "") << nm(v, sp) << init;
+    o << ";\n";
+  }
+  // one attempt from x: n (unclamped) and acc, with f0 = f(x) evaluated unless `have`
+  void attempt() {
+    for (int i = 0; i < KR; ++i) o << (i ? ", W" : "  double W") << i << (i + 1 == KR ? ";\n" : "");
+    decl("k1_"); decl("f1_"); decl("k2_"); decl("n"); decl("b");
+    o << "  if (!have) {\n";
+    rhs("x", "f0_");
+    o << "  }\n";
+    build_w();
+    lu_factor();
+    each("k1_# = f0_#;");
+    solve("k1_");
+    each("n# = fma(dto2, k1_#, x#);");
+    rhs("n", "f1_");
+    each("k2_# = f1_# - k1_#;");
+    solve("k2_");
+    each("k2_# = k2_# + k1_#; n# = fma(dt, k2_#, x#);");
+    rhs("n", "b");
+    if (per_cell) each("f2_# = b#;");
+    each("b# = fma(-2.0, k1_# - f0_#, fma(-ROS_C32, k2_# - f1_#, b#));");
+    solve("b");
+    o << "  double acc = 0.0;\n";
+    each("{ const double ut = dto6 * (fma(-2.0, k2_#, k1_#) + b#); const double at = ut * "
+         "rcp_nr1(fma(amax_bits(x#, n#), rtol, atol)); acc = fma(at, at, acc); }");
+  }
+};
+
+std::string generate_wide(const MechTables& T, double ros_d, double ros_c32, bool per_cell) {
+  WideGen g{T, per_cell, {}, {}, 0};
+  g.rank_slots();
+  auto& o = g.o;
+  o << "// generated: " << T.ns << " species, " << T.nr << " reactions, " << T.nlu << " LU slots, " << g.KR
+    << " of them in registers\n#define NS " << T.ns << "\n#define NRA " << (T.nr > 0 ? T.nr : 1)
+    << "\n#define ROS_D " << lit(ros_d) << "\n#define ROS_C32 " << lit(ros_c32) << "\n#define OFF_DONE "
+    << offsetof(Ctl, done) << "\n#define OFF_CUR " << offsetof(Ctl, cur) << "\n#define OFF_DTC "
+    << offsetof(Ctl, dtc) << "\n#define OFF_DTO2 " << offsetof(Ctl, dto2) << "\n#define OFF_DTO6 "
+    << offsetof(Ctl, dto6) << "\n#define OFF_DTG " << offsetof(Ctl, dtgamma) << "\n#define RS_STRICT 1\n"
+    << kPrelude << "#define RS_FENCE asm volatile(\"\" ::: \"memory\");\n#define EM(s) __ldg(em + (u64)(s) * N + c)\n";
+  if (!per_cell) {
+    o << R"(#define LDK(r) double K##r; asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(K##r) : "l"(kr + (u64)(r) * N + c));
+extern "C" __global__ void __launch_bounds__(256, 1) rs_wide_attempt(
+    const unsigned char* __restrict__ ctl, double* __restrict__ U0, double* __restrict__ U1,
+    const double* __restrict__ kr, const double* __restrict__ em, double* __restrict__ partial,
+    int nc, int nsp, double rtol, double atol, int clamp) {
+  extern __shared__ double wsm[];
+  __shared__ double red[256];
+  if (*(const int*)(ctl + OFF_DONE)) return;
+  volatile double* S = wsm + threadIdx.x;
+  const double dt = *(const double*)(ctl + OFF_DTC), dto2 = *(const double*)(ctl + OFF_DTO2);
+  const double dto6 = *(const double*)(ctl + OFF_DTO6), dtg = *(const double*)(ctl + OFF_DTG);
+  const int cur = *(const int*)(ctl + OFF_CUR);
+  const double* __restrict__ U = cur ? U1 : U0;
+  double* __restrict__ Un = cur ? U0 : U1;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const u64 N = (u64)nc;
+  double e = 0.0;
+  if (c < nc) {
+  const bool have = false;
+)";
+    g.decl("f0_");
+    g.each("const double x# = U[(u64)# * N + c];");
+    g.attempt();
+    g.each("Un[(u64)# * N + c] = clamp ? fmax(n#, 0.0) : n#;");
+    o << R"(  for (int s = NS; s < nsp; ++s) {
+    const double xv = U[(u64)s * N + c];
+    Un[(u64)s * N + c] = clamp ? fmax(xv, 0.0) : xv;
+  }
+  e = acc;
+  }
+  const double tot = block_total(e, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+}
+)";
+    return o.str();
+  }
+  o << R"(#define LDK(r) const double K##r = kc[r];
+extern "C" __global__ void __launch_bounds__(256, 1) rs_wide_per_cell(int nc, int nsp,
+    double* __restrict__ U, const double* __restrict__ kr, const double* __restrict__ em,
+    double* __restrict__ dt_cell, double* __restrict__ steps_cell,
+    unsigned long long* __restrict__ queue, int* __restrict__ status, PCA a) {
+  extern __shared__ double wsm[];
+  volatile double* S = wsm + threadIdx.x;
+  volatile double kc[NRA];
+  const u64 N = (u64)nc;
+  const double rtol = a.rtol, atol = a.atol;
+  double my_steps = 0.0, my_attempts = 0.0;
+  double t = 0, dtn = 0, qold = 0, iters = 0, nacc = 0;
+  bool have = false;
+  int c = -1;
+  const double tlim = a.t1 - 1.0e-9;
+)";
+  g.decl("x", " = 0.0");
+  g.decl("f0_", " = 0.0");
+  g.decl("f2_", " = 0.0");
+  o << R"(  for (;;) {
+  if (c < 0) {
+    const unsigned long long nxt = atomicAdd(queue, 1ull);
+    if (nxt >= (unsigned long long)nc) break;
+    c = (int)nxt;
+)";
+  g.each("x# = U[(u64)# * N + c];");
+  o << R"(#pragma unroll 4
+    for (int r = 0; r < NRA; ++r) kc[r] = kr[(u64)r * N + c];
+    have = false;
+    t = a.t0;
+    dtn = quant_dt(dt_cell[c] > 0.0 ? dt_cell[c] : a.dt0);
+    qold = a.qoldinit;
+    iters = 0;
+    nacc = 0;
+  }
+  if ((t < tlim) && (iters < a.maxiters)) {
+  const double dt = fmin(dtn, a.t1 - t), dto2 = dt / 2, dto6 = dt / 6, dtg = dt * ROS_D;
+)";
+  g.attempt();
+  o << R"(  have = true;  // f0 == f(x); replaced below if x moves
+  double EEst = sqrt(acc / (double)nsp);
+  if (isnan(EEst)) EEst = 1.0e10;
+  const double q11 = pow(fmax(EEst, 1.0e-35), a.beta1);
+  double q = q11 / pow(qold, a.beta2);
+  q = fmax(a.invqmax, fmin(a.invqmin, q / a.gamma));
+  if (EEst <= 1.0) {
+    bool same = true;  // the clamp left the candidate as it was: f(x) is f2
+)";
+  g.each("{ const double xs = a.clamp ? fmax(n#, 0.0) : n#; same = same && (__double_as_longlong(xs) == "
+         "__double_as_longlong(n#)); x# = xs; }");
+  o << "    if (same) {\n";
+  g.each("f0_# = f2_#;");
+  o << R"(    }
+    have = same;
+    t = t + dt;
+    const bool insteady = (a.qsmin <= q) && (q <= a.qsmax);
+    dtn = quant_dt(dt / (insteady ? 1.0 : q));
+    qold = fmax(EEst, a.qoldinit);
+    nacc += 1.0;
+  } else {
+    dtn = quant_dt(dt / fmin(a.invqmin, q11 / a.gamma));
+  }
+  iters += 1.0;
+  } else {
+    if (t < tlim) atomicOr(status, 1);
+)";
+  g.each("U[(u64)# * N + c] = x#;");
+  o << R"(    dt_cell[c] = dtn;
+    if (steps_cell) steps_cell[c] = nacc;
+    my_steps += nacc;
+    my_attempts += iters;
+    c = -1;
+  }
+  }
+  if (a.totals) {
+    atomicAdd(a.totals, my_steps);
+    atomicAdd(a.totals + 1, my_attempts);
+  }
+}
+)";
+  return o.str();
+}
+
 // ------------------------------------------------------------------ compile cache
 struct Compiled {
   cudaLibrary_t lib = nullptr;
@@ -1127,6 +1475,67 @@ void jit_launch_per_cell(const JitChem& J, cudaStream_t st, int nc, int nsp, int
   PerCellArgs av = a;
   void* args[] = {&nc, &nsp, &U, &kr, &em, &dtc, &steps, &queue, &status, &av};
   cudaLaunchKernel((const void*)k, dim3(nblocks), dim3(threads), args, 0, st);
+}
+
+std::shared_ptr<WideChem> wide_chem_build(const MechTables& T, double ros_d, double ros_c32,
+                                          bool per_cell, std::string* why) {
+#if RS_STRICT
+  *why = "the strict build walks the tables";
+  return nullptr;
+#else
+  if (jit_chem_eligible(T) || !wide_eligible(T)) {
+    *why = "mechanism outside the wide kernels' range";
+    return nullptr;
+  }
+  const std::string src = generate_wide(T, ros_d, ros_c32, per_cell);
+  Compiled cmp;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_cache.find(src + "|wide");
+    if (it != g_cache.end()) {
+      cmp = it->second;
+    } else {
+      if (!compile_and_load(src, false, &cmp, why)) return nullptr;
+      g_cache[src + "|wide"] = cmp;
+    }
+  }
+  auto Wc = std::make_shared<WideChem>();
+  cudaKernel_t* k = per_cell ? &Wc->per_cell : &Wc->attempt;
+  cudaError_t e = cudaLibraryGetKernel(k, cmp.lib, per_cell ? "rs_wide_per_cell" : "rs_wide_attempt");
+  Wc->smem = wide_smem_bytes(T);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)*k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wc->smem);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *why = std::string("wide kernels: ") + cudaGetErrorString(e);
+    return nullptr;
+  }
+  why->clear();
+  return Wc;
+#endif
+}
+std::string wide_chem_source(const MechTables& T, bool per_cell) {
+  return wide_eligible(T) ? generate_wide(T, 1.0 / (2.0 + std::sqrt(2.0)), 6.0 + std::sqrt(2.0), per_cell)
+                          : std::string();
+}
+void wide_launch_attempt(const WideChem& Wc, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
+                         double* U0, double* U1, const double* kr, const double* em, double* part,
+                         double rtol, double atol, int clamp) {
+  const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
+  void* args[] = {&c, &U0, &U1, &kr, &em, &part, &nc, &nsp, &rtol, &atol, &clamp};
+  cudaLaunchKernel((const void*)Wc.attempt, dim3((nc + kBlock - 1) / kBlock), dim3(kBlock), args, Wc.smem, st);
+}
+// One block per SM (its shared memory); fewer threads each while the cells do not fill 256 per
+// SM, so that small batches still use every SM.
+void wide_launch_per_cell(const WideChem& Wc, cudaStream_t st, int nsm, int nc, int nsp, double* U,
+                          const double* kr, const double* em, double* dtc, double* steps,
+                          unsigned long long* queue, int* status, const PerCellArgs& a) {
+  const int per = (nc + nsm - 1) / nsm;
+  const int thr = per >= kBlock ? kBlock : (per + 31) / 32 * 32;
+  const int nb = std::min(nsm, (nc + thr - 1) / thr);
+  PerCellArgs av = a;
+  void* args[] = {&nc, &nsp, &U, &kr, &em, &dtc, &steps, &queue, &status, &av};
+  cudaLaunchKernel((const void*)Wc.per_cell, dim3(nb), dim3(thr), args, Wc.smem, st);
 }
 
 }  // namespace rs

@@ -82,4 +82,21 @@ void jit_launch_per_cell(const JitChem& J, cudaStream_t st, int nc, int nsp, int
                          double* dtc, double* steps, unsigned long long* queue, int* status,
                          const PerCellArgs& a);
 
+// Straight-line forms of the table-walking attempt or per-cell kernel for mechanisms too large for
+// JitChem (production build): the same bits, chosen behind the TABLE kernel kind.
+struct WideChem {
+  cudaKernel_t attempt = nullptr, per_cell = nullptr;
+  size_t smem = 0;
+};
+// the one kernel asked for, or null and *why
+std::shared_ptr<WideChem> wide_chem_build(const MechTables& T, double ros_d, double ros_c32,
+                                          bool per_cell, std::string* why);
+std::string wide_chem_source(const MechTables& T, bool per_cell);  // empty: not eligible
+void wide_launch_attempt(const WideChem& W, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
+                         double* U0, double* U1, const double* kr, const double* em, double* part,
+                         double rtol, double atol, int clamp);
+void wide_launch_per_cell(const WideChem& W, cudaStream_t st, int nsm, int nc, int nsp, double* U,
+                          const double* kr, const double* em, double* dtc, double* steps,
+                          unsigned long long* queue, int* status, const PerCellArgs& a);
+
 }  // namespace rs

@@ -15,6 +15,7 @@ constexpr int kLargeMS = 64, kLargeMR = 128, kLargeMLU = 1600, kLargeMP = 256;
 constexpr int kMaxProgStack = 32;
 
 struct JitChem;
+struct WideChem;
 struct MixedTmaps;  // tensor maps of the mixed-precision split planes (rs_transport.cu)
 
 struct LaunchCtx {
@@ -24,6 +25,7 @@ struct LaunchCtx {
   int nsp;         // species per cell in the state (chemistry species + air mass)
   int size_class;  // 0 small, 1 large
   const JitChem* jit = nullptr;  // mechanism-specialised kernels, or null: table-walking ones
+  const WideChem* wide = nullptr;  // their straight-line forms for large mechanisms, or null
 };
 
 struct PerCellArgs {
