@@ -29,6 +29,7 @@
 #include <mutex>
 #include <sstream>
 #include <string>
+#include <thread>
 #include <type_traits>
 #include <vector>
 
@@ -96,6 +97,7 @@ std::string lit(double v) {  // exact hex-float literal
 
 // W storage: shared-memory variant only while NLU doubles per thread x 256 threads fit
 constexpr int kBlock = 256;
+constexpr int kJitUnits = 8;  // RS_IN units of the generated source
 constexpr size_t kSmemCap = 227 * 1024 - kBlock * sizeof(double);
 
 size_t smem_bytes(const MechTables& T) { return (size_t)T.nlu * kBlock * sizeof(double); }
@@ -265,6 +267,17 @@ struct Gen {
     for (int e = 0; e < T.nlu; ++e) o << "  WV(" << e << ") = " << w[e] << ";\n";
     o << "  }\n";
   }
+  // (eh, el) <- W^-1 (eh, el) in float pairs from the FP64 factors, split entry by entry
+  void solve_pairs() {
+    for (int k = 0; k < T.ns; ++k)
+      for (int e = T.low_ptr[k]; e < T.low_ptr[k + 1]; ++e)
+        o << "  pair_msub(" << T.low_row[e] << ", " << T.low_slot[e] << ", " << T.ord[k] << ")\n";
+    for (int i = T.ns - 1; i >= 0; --i) {
+      for (int e = T.up_ptr[i]; e < T.up_ptr[i + 1]; ++e)
+        o << "  pair_msub(" << T.ord[i] << ", " << T.up_slot[e] << ", " << T.up_col[e] << ")\n";
+      o << "  pair_scale(" << T.ord[i] << ", " << i << ")\n";
+    }
+  }
   void lu_factor() {
     int m = 0;
     for (int k = 0; k < T.ns; ++k) {
@@ -421,6 +434,54 @@ __device__ __forceinline__ double amax_bits(double a, double b) {
   return __hiloint2double((int)(bl ? hb : ha), (int)(bl ? lb : la));
 }
 
+// ---- float pairs (value = h + l, about 47 bits) for the error estimate
+struct fp2 {
+  float h, l;
+};
+// A double as a pair, on the integer pipe (an FP64 conversion costs an FP64 instruction): h the
+// leading 24 bits, l the 29 below them rounded to 24.  Below 2^-74 l loses bits, below 2^-126 the
+// value counts as 0; `big` collects the magnitudes so that the caller can refuse values from
+// 2^127 on, infinities and NaN.
+__device__ __forceinline__ fp2 split_pair(double v, unsigned& big) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mag = hi & 0x7fffffffu;
+  big = big > mag ? big : mag;
+  const unsigned f = (__funnelshift_l(lo, hi, 3) ^ 0x40000000u) & 0x7fffffffu;  // exponent - 896
+  const int sc = max((int)(f & 0x7f800000u) - (52 << 23), 0);
+  const float l = __int2float_rn((int)(lo & 0x1fffffffu)) * __int_as_float(sc);
+  const unsigned sg = hi & 0x80000000u;
+  const bool z = mag < (898u << 20);
+  return {z ? 0.0f : __uint_as_float(f | sg), z ? 0.0f : __uint_as_float(__float_as_uint(l) ^ sg)};
+}
+constexpr unsigned kPairBig = 1150u << 20;
+__device__ __forceinline__ fp2 pair_renorm(float s, float e) {
+  const float h = s + e;
+  return {h, e - (h - s)};
+}
+__device__ __forceinline__ fp2 pair_mul(fp2 a, fp2 b) {
+  const float p = a.h * b.h;
+  return pair_renorm(p, fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p))));
+}
+__device__ __forceinline__ fp2 pair_add(fp2 a, fp2 b) {
+  const float s = a.h + b.h, bb = s - a.h;
+  return pair_renorm(s, ((a.h - (s - bb)) + (b.h - bb)) + (a.l + b.l));
+}
+__device__ __forceinline__ fp2 pair_fnma(fp2 a, fp2 b, fp2 c) {  // c - a b
+  const float p = a.h * b.h;
+  const float pe = fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p)));
+  const float s = c.h - p, bb = s - c.h;
+  return pair_renorm(s, ((c.h - (s - bb)) + (-p - bb)) + (c.l - pe));
+}
+// a / b: the quotient of the leading parts and one correction from the exact remainder
+__device__ __forceinline__ fp2 pair_div(fp2 a, fp2 b) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b.h));
+  const float q = a.h * r;
+  const float rem = fmaf(-q, b.l, fmaf(-q, b.h, a.h) + a.l);
+  return pair_renorm(q, rem * r);
+}
+__device__ __forceinline__ double pair_to_d(fp2 a) { return (double)a.h + (double)a.l; }
+
 // Per-cell step sizes are rounded down to 4 fraction bits (16 sizes per octave): a perturbation
 // of the inputs then changes a cell's step sequence only where a proposal sits within the
 // perturbation of a lattice point, so per-cell trajectories stay within roundoff of each other
@@ -474,21 +535,20 @@ std::string generate(const MechTables& T, double ros_d, double ros_c32, bool str
   o << "#define OFF_DONE " << offsetof(Ctl, done) << "\n#define OFF_CUR " << offsetof(Ctl, cur)
     << "\n#define OFF_DTC " << offsetof(Ctl, dtc) << "\n#define OFF_DTO2 "
     << offsetof(Ctl, dto2) << "\n#define OFF_DTO6 " << offsetof(Ctl, dto6)
-    << "\n#define OFF_DTG " << offsetof(Ctl, dtgamma) << "\n#define OFF_ITERS "
+    << "\n#define OFF_DTG " << offsetof(Ctl, dtgamma)
+    << "\n#define OFF_ITERS "
     << offsetof(Ctl, iters) << "\n#define OFF_NACC " << offsetof(Ctl, nacc)
     << "\n#define OFF_KZ " << offsetof(Ctl, kz) << "\n#define OFF_KZCAP "
     << offsetof(Ctl, kzcap) << "\n";
+  // the kernels in units that compile side by side (RS_UNIT 0: all of them)
+  o << "#ifndef RS_UNIT\n#define RS_UNIT 0\n#endif\n#define RS_IN(k) (RS_UNIT == 0 || RS_UNIT == (k))\n";
   o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude;
   // Every multiply-add is written out: RS_FMA fuses in the production build and keeps the
   // multiply and the add separate in the strict build; both builds compile with --fmad=false,
   // so no compiler contraction decides anything and all variants compute the same bits.
-  // RS_NQUOT / RS_AMAX serve the error norm only (its value steers the controller and nothing
-  // else): a one-step reciprocal and an integer magnitude max in the production build.
-  o << (strict ? "#define RS_QUOT(a, b) ((a) / (b))\n#define RS_FMA(a, b, c) ((a) * (b) + (c))\n"
-                 "#define RS_NQUOT(a, b) ((a) / (b))\n#define RS_AMAX(a, b) fmax(fabs(a), fabs(b))\n"
+  o << (strict ? "#define RS_FMA(a, b, c) ((a) * (b) + (c))\n"
                  "#define RS_VDECL double v[NRA];  // the rates of the oracle-order RHS\n"
-               : "#define RS_QUOT(a, b) ((a) * rcp_nr(b))\n#define RS_FMA(a, b, c) fma((a), (b), (c))\n"
-                 "#define RS_NQUOT(a, b) ((a) * rcp_nr1(b))\n#define RS_AMAX(a, b) amax_bits((a), (b))\n"
+               : "#define RS_FMA(a, b, c) fma((a), (b), (c))\n"
                  "#define RS_VDECL  // the fused RHS keeps no rate array\n");
   // One ROS23 attempt of one cell: xn (unclamped) and the cell's sum of squared scaled errors.
   // f0 = f(x) is computed here unless the caller already holds it (have_f0): after an
@@ -509,12 +569,17 @@ __device__ __forceinline__ double* stage_slot(const unsigned char* __restrict__ 
 // W storage: LU slots e < KR in the register array W, the others in shared memory at
 // WSM[(e - KR) * 256] (this thread's column of a [slot][thread] array); every slot index is a
 // compile-time constant, so each access resolves to one of the two when compiled.
-template <bool HE, int KR, bool KEEP, bool SOL = false>
+// un, fin (may be null): where the clamped new state and, unless have_f0, f(x) go in global
+// memory -- written as soon as they are final, so that neither stays live through the error solve.
+// PAIRS: the error estimate in float pairs; returns a negative value where the pairs' range does
+// not hold it (the caller forms the estimate again without PAIRS).
+template <bool HE, int KR, bool KEEP, bool SOL = false, bool PAIRS = false>
 __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
     const double* __restrict__ em, u64 N, int c, const double* x, double* xn, double* W,
     double* WSM, double* f0, bool have_f0, double* __restrict__ fout, int clamp, double* f2,
     double dt, double dto2, double dto6, double dtg, double rtol, double atol,
-    double* __restrict__ kzo) {
+    double* __restrict__ kzo, double* __restrict__ un = nullptr,
+    double* __restrict__ fin = nullptr) {
 #define K(r) __ldg(kr + (u64)(r) * N + c)
 #define EM(s) __ldg(em + (u64)(s) * N + c)
 #define WV(e) (*((e) < KR ? &W[(e)] : &WSM[((e) - KR) * 256]))
@@ -563,24 +628,94 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
 #pragma unroll
     for (int s = 0; s < NS; ++s) f2[s] = b[s];
   }
-#pragma unroll
-  for (int s = 0; s < NS; ++s)  // y - 2d as fma(-2, d, y): exact doubling, one rounding either way
-    b[s] = RS_FMA(-2.0, k1[s] - f0[s], RS_FMA(-ROS_C32, (k2[s] - f1[s]), b[s]));
 )";
-  g.lu_solve("b");
-  // error norm sum_s (dto6 * e_s / den_s)^2; the production build takes dto6^2 out of the sum
-  const char* ut = g.strict ? "dto6 * (RS_FMA(-2.0, k2[s], k1[s]) + b[s])" : "RS_FMA(-2.0, k2[s], k1[s]) + b[s]";
-  o << R"(  double acc = 0.0;
+  o << R"(  if (fin && !have_f0) {  // f(x), for a retry of this state after a rejection
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    const double ut = )" << ut << R"(;
-    const double am = RS_AMAX(x[s], xn[s]);
-    const double den = RS_FMA(am, rtol, atol);
-    const double at = RS_NQUOT(ut, den);
-    acc = RS_FMA(at, at, acc);
+    for (int s = 0; s < NS; ++s) fin[(u64)s * N + c] = f0[s];
   }
 )";
-  o << (g.strict ? "  return acc;\n" : "  return acc * (dto6 * dto6);\n");
+  const char* store_un = R"(  if (un) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) un[(u64)s * N + c] = clamp ? fmax(xn[s], 0.0) : xn[s];
+  }
+)";
+  if (!g.strict) {
+    // The error estimate dt/6 (k1 - 2 k2 + k3).  With W k1 = f0 and W k2 = f1 - k1 + f0 the third
+    // stage's equation becomes W (k1 - 2 k2 + k3) = (f2 - 2 f1 + f0) - c32 (k2 - f1): one solve for
+    // the whole estimate, whose right-hand side takes the cancellation in FP64.  Nothing after it
+    // cancels, and the norm only steers the step size, so on large grids solve and norm run in
+    // float pairs on the FP32 pipe (relative error ~1e-13; the FP64 norm's one-step reciprocal
+    // has 1e-12): 131 FP64 instructions of 64 cycles each become ~2,900 instructions on pipes that
+    // stand idle beside them.  Where one warp per sub-partition runs alone (attempt_fp64_norm) the
+    // FP64 form's shorter chain wins.
+    o << R"(#pragma unroll
+  for (int s = 0; s < NS; ++s)
+    b[s] = fma(-ROS_C32, k2[s] - f1[s], fma(-2.0, f1[s], b[s]) + f0[s]);
+  if constexpr (PAIRS) {
+  unsigned big = 0;
+  float eh[NS], el[NS], dh[NS], dl[NS];
+  const fp2 rt = split_pair(rtol, big), at0 = split_pair(atol, big);
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const fp2 v = split_pair(b[s], big);
+    const fp2 den = pair_add(pair_mul(split_pair(amax_bits(x[s], xn[s]), big), rt), at0);
+    eh[s] = v.h;
+    el[s] = v.l;
+    dh[s] = den.h;
+    dl[s] = den.l;
+  }
+)" << store_un << R"(#define pair_msub(i, slot, k)                                                              \
+  {                                                                                        \
+    const fp2 v_ = pair_fnma(split_pair(WV(slot), big), fp2{eh[k], el[k]}, fp2{eh[i], el[i]}); \
+    eh[i] = v_.h;                                                                          \
+    el[i] = v_.l;                                                                          \
+  }
+#define pair_scale(i, q)                                                                   \
+  {                                                                                        \
+    const fp2 v_ = pair_mul(fp2{eh[i], el[i]}, split_pair(pv[q], big));                    \
+    eh[i] = v_.h;                                                                          \
+    el[i] = v_.l;                                                                          \
+  }
+)";
+    g.solve_pairs();
+    o << R"(#undef pair_msub
+#undef pair_scale
+  fp2 sum = {0.0f, 0.0f};
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const fp2 q = pair_div(fp2{eh[s], el[s]}, fp2{dh[s], dl[s]});
+    sum = pair_add(sum, pair_mul(q, q));
+  }
+  return big < kPairBig && at0.h >= 0x1p-100f ? pair_to_d(sum) * (dto6 * dto6) : -1.0;
+  } else {
+)" << store_un;
+    g.lu_solve("b");
+    o << R"(  double acc = 0.0;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double at = b[s] * rcp_nr1(fma(amax_bits(x[s], xn[s]), rtol, atol));
+    acc = fma(at, at, acc);
+  }
+  return acc * (dto6 * dto6);
+  }
+)";
+  } else {
+    o << store_un << R"(#pragma unroll
+  for (int s = 0; s < NS; ++s)
+    b[s] = RS_FMA(-2.0, k1[s] - f0[s], RS_FMA(-ROS_C32, (k2[s] - f1[s]), b[s]));
+)";
+    g.lu_solve("b");
+    o << R"(  double acc = 0.0;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double ut = dto6 * (RS_FMA(-2.0, k2[s], k1[s]) + b[s]);
+    const double den = RS_FMA(fmax(fabs(x[s]), fabs(xn[s])), rtol, atol);
+    const double at = ut / den;
+    acc = RS_FMA(at, at, acc);
+  }
+  return acc;
+)";
+  }
   o << R"(#undef K
 #undef EM
 #undef WV
@@ -591,7 +726,19 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
 // unknown); from the second attempt of a solve on, a cell reuses it instead of evaluating
 // f(x) again (the first attempt of a solve starts from a state written elsewhere).
 // MODE 0: W in registers; 1: W in shared memory; 2: split (NLU_R slots in registers)
-template <bool HE, int MODE>
+#if !RS_STRICT
+// the error estimate of one cell once more in FP64 (values outside the float pairs' range)
+template <bool HE>
+__device__ __noinline__ double attempt_error_fp64(const double* __restrict__ U,
+    const double* __restrict__ kr, const double* __restrict__ em, u64 N, int c, double dt,
+    double dto2, double dto6, double dtg, double rtol, double atol) {
+  double x[NS], xn[NS], f0[NS], W[NLU];
+  for (int s = 0; s < NS; ++s) x[s] = U[(u64)s * N + c];
+  return ros23_cell<HE, NLU, false>(kr, em, N, c, x, xn, W, nullptr, f0, false, nullptr, 0,
+                                    nullptr, dt, dto2, dto6, dtg, rtol, atol, nullptr);
+}
+#endif
+template <bool HE, int MODE, bool PAIRS>
 __device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ ctl,
     double* __restrict__ U0, double* __restrict__ U1, const double* __restrict__ kr,
     const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,
@@ -624,27 +771,25 @@ __device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ c
     }
     if constexpr (MODE == 1) {
       extern __shared__ double wsm[];
-      e = ros23_cell<HE, 0, false>(kr, em, N, c, x, xn, nullptr, wsm + threadIdx.x, f0, have,
+      e = ros23_cell<HE, 0, false, false, PAIRS>(kr, em, N, c, x, xn, nullptr, wsm + threadIdx.x, f0, have,
                                    F0 ? Fout : nullptr, clamp, nullptr, dt, dto2, dto6, dtg,
-                                   rtol, atol, kzo);
+                                   rtol, atol, kzo, Un, F0 ? Fin : nullptr);
     } else if constexpr (MODE == 2) {
       extern __shared__ double wsm[];
       double W[NLU_R > 0 ? NLU_R : 1];
-      e = ros23_cell<HE, NLU_R, false>(kr, em, N, c, x, xn, W, wsm + threadIdx.x, f0, have,
+      e = ros23_cell<HE, NLU_R, false, false, PAIRS>(kr, em, N, c, x, xn, W, wsm + threadIdx.x, f0, have,
                                        F0 ? Fout : nullptr, clamp, nullptr, dt, dto2, dto6,
-                                       dtg, rtol, atol, kzo);
+                                       dtg, rtol, atol, kzo, Un, F0 ? Fin : nullptr);
     } else {
       double W[NLU];
-      e = ros23_cell<HE, NLU, false>(kr, em, N, c, x, xn, W, nullptr, f0, have,
+      e = ros23_cell<HE, NLU, false, false, PAIRS>(kr, em, N, c, x, xn, W, nullptr, f0, have,
                                      F0 ? Fout : nullptr, clamp, nullptr, dt, dto2, dto6, dtg,
-                                     rtol, atol, kzo);
+                                     rtol, atol, kzo, Un, F0 ? Fin : nullptr);
     }
-    if (F0 && !have) {  // keep f(x) for a retry of this state after a rejection
-#pragma unroll
-      for (int s = 0; s < NS; ++s) Fin[(u64)s * N + c] = f0[s];
-    }
-#pragma unroll
-    for (int s = 0; s < NS; ++s) Un[(u64)s * N + c] = clamp ? fmax(xn[s], 0.0) : xn[s];
+#if !RS_STRICT
+    if constexpr (PAIRS)
+      if (e < 0.0) e = attempt_error_fp64<HE>(U, kr, em, N, c, dt, dto2, dto6, dtg, rtol, atol);
+#endif
     for (int s = NS; s < nsp; ++s) {
       const double xv = U[(u64)s * N + c];
       Un[(u64)s * N + c] = clamp ? fmax(xv, 0.0) : xv;
@@ -732,20 +877,29 @@ __device__ __forceinline__ void per_cell_body(int nc, int nsp, double* __restric
   }
 }
 
-#define RS_ATTEMPT(NAME, HE, MODE, MINB)                                                    \
+#define RS_ATTEMPT(NAME, HE, MODE, MINB, PAIRS)                                                  \
   extern "C" __global__ void __launch_bounds__(256, MINB) NAME(                             \
       const unsigned char* __restrict__ ctl, double* __restrict__ U0,                       \
       double* __restrict__ U1, const double* __restrict__ kr,                               \
       const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,         \
       double rtol, double atol, int clamp, double* __restrict__ F0,                         \
       double* __restrict__ F1) {                                                            \
-    attempt_body<HE, MODE>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
+    attempt_body<HE, MODE, PAIRS>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
                            F1);                                                             \
   }
-RS_ATTEMPT(rs_jit_attempt_r0, false, 0, 1)
-RS_ATTEMPT(rs_jit_attempt_r1, true, 0, 1)
-RS_ATTEMPT(rs_jit_attempt_q0, false, 0, 2)
-RS_ATTEMPT(rs_jit_attempt_q1, true, 0, 2)
+#define RS_PAIRS (!RS_STRICT)
+#if RS_IN(1)
+RS_ATTEMPT(rs_jit_attempt_l0, false, 0, 1, false)
+RS_ATTEMPT(rs_jit_attempt_l1, true, 0, 1, false)
+#endif
+#if RS_IN(2)
+RS_ATTEMPT(rs_jit_attempt_r0, false, 0, 1, RS_PAIRS)
+RS_ATTEMPT(rs_jit_attempt_r1, true, 0, 1, RS_PAIRS)
+#endif
+#if RS_IN(3)
+RS_ATTEMPT(rs_jit_attempt_q0, false, 0, 2, RS_PAIRS)
+RS_ATTEMPT(rs_jit_attempt_q1, true, 0, 2, RS_PAIRS)
+#endif
 
 // one accepted step at the controller's dtc without the error estimate: the attempt's own
 // arithmetic up to the new state (the same bits), for the fixed-sequence replay of a recorded
@@ -783,13 +937,15 @@ __device__ __forceinline__ void step_body(const unsigned char* __restrict__ ctl,
       const double* __restrict__ em, int nc, int nsp, int clamp) {                          \
     step_body<HE>(ctl, U0, U1, kr, em, nc, nsp, clamp);                                     \
   }
+#if RS_IN(6)
 RS_STEP(rs_jit_step_0, false)
 RS_STEP(rs_jit_step_1, true)
+#endif
 )";
   if (with_smem)
-    o << "RS_ATTEMPT(rs_jit_attempt_s0, false, 1, 1)\nRS_ATTEMPT(rs_jit_attempt_s1, true, 1, 1)\n";
+    o << "#if RS_IN(4)\nRS_ATTEMPT(rs_jit_attempt_s0, false, 1, 1, RS_PAIRS)\nRS_ATTEMPT(rs_jit_attempt_s1, true, 1, 1, RS_PAIRS)\n#endif\n";
   if (nsplit > 0)
-    o << "RS_ATTEMPT(rs_jit_attempt_h0, false, 2, 2)\nRS_ATTEMPT(rs_jit_attempt_h1, true, 2, 2)\n";
+    o << "#if RS_IN(5)\nRS_ATTEMPT(rs_jit_attempt_h0, false, 2, 2, RS_PAIRS)\nRS_ATTEMPT(rs_jit_attempt_h1, true, 2, 2, RS_PAIRS)\n#endif\n";
   o << R"(
 #define RS_PER_CELL(NAME, HE)                                                                \
   extern "C" __global__ void __launch_bounds__(256) NAME(int nc, int nsp,                   \
@@ -798,8 +954,10 @@ RS_STEP(rs_jit_step_1, true)
       unsigned long long* __restrict__ queue, int* __restrict__ status, PCA a) {             \
     per_cell_body<HE>(nc, nsp, U, kr, em, dt_cell, steps_cell, queue, status, a);            \
   }
+#if RS_IN(7)
 RS_PER_CELL(rs_jit_per_cell_0, false)
 RS_PER_CELL(rs_jit_per_cell_1, true)
+#endif
 
 // VJP of one ROS23 step at a recorded dt (the table kernel k_ros23_vjp, specialised): forward
 // recompute of the live stages, then lam_out = (d unew / d u)^T lam and ebar += d J / d emission.
@@ -900,17 +1058,21 @@ __device__ __forceinline__ void vjp_body(int nc, int nsp, const double* __restri
       double* __restrict__ ebar, double dt, int clamp, const double* __restrict__ kzi) {     \
     vjp_body<HE, KZ>(nc, nsp, U, Uout, lam, lam_out, kr, em, ebar, dt, clamp, kzi);          \
   }
+#if RS_IN(8)
 RS_VJP(rs_jit_vjp_0, false, false)
 RS_VJP(rs_jit_vjp_1, true, false)
 RS_VJP(rs_jit_vjpk_0, false, true)
 RS_VJP(rs_jit_vjpk_1, true, true)
+#endif
 
+#if RS_IN(6)
 // the production reciprocal applied elementwise (accuracy check against IEEE division)
 extern "C" __global__ void rs_jit_rcp(const double* __restrict__ x, double* __restrict__ r,
                                       int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) r[i] = rcp_nr(x[i]);
 }
+#endif
 )";
   return o.str();
 }
@@ -1264,7 +1426,7 @@ extern "C" __global__ void __launch_bounds__(256, 1) rs_wide_per_cell(int nc, in
 
 // ------------------------------------------------------------------ compile cache
 struct Compiled {
-  cudaLibrary_t lib = nullptr;
+  std::vector<cudaLibrary_t> libs;
   double ms = 0;
 };
 std::mutex g_mu;
@@ -1275,7 +1437,7 @@ std::map<std::string, Compiled> g_cache;  // source + options -> loaded library 
 // NVRTC compile of generated source to an sm_103a cubin (no device needed).  With verbose
 // the log carries ptxas's resource usage (registers, spill stores/loads, shared memory).
 bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<char>* cubin,
-                 std::string* log) {
+                 std::string* log, int unit) {
   const Nvrtc& N = nvrtc();
   if (!N.ok()) {
     *log = N.why;
@@ -1287,8 +1449,10 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
     *log = std::string("nvrtcCreateProgram: ") + N.err(r);
     return false;
   }
-  (void)strict;  // the source itself differs between the builds (RS_FMA, RS_QUOT)
+  (void)strict;  // the source itself differs between the builds (RS_FMA)
   std::vector<const char*> opts = {"-arch=sm_103a", "-std=c++17", "--fmad=false"};
+  const std::string def = "-DRS_UNIT=" + std::to_string(unit);
+  opts.push_back(def.c_str());
   if (verbose) opts.push_back("--ptxas-options=-v");
   r = N.compile(prog, (int)opts.size(), opts.data());
   size_t n = 0;
@@ -1314,23 +1478,44 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
 
 namespace {
 
-bool compile_and_load(const std::string& src, bool strict, Compiled* out, std::string* why) {
+// Compiles the source's units (1 .. units) in parallel threads -- NVRTC compiles a whole program
+// in one -- and loads them; units = 0: the source is one unit.
+bool compile_and_load(const std::string& src, bool strict, int units, Compiled* out, std::string* why) {
   auto t0 = std::chrono::steady_clock::now();
-  std::vector<char> cubin;
-  std::string log;
-  if (!jit_compile(src, strict, false, &cubin, &log)) {
-    *why = log.substr(0, 4000);
-    return false;
-  }
-  cudaError_t e = cudaLibraryLoadData(&out->lib, cubin.data(), nullptr, nullptr, 0, nullptr,
-                                      nullptr, 0);
-  if (e != cudaSuccess) {
-    *why = std::string("cudaLibraryLoadData: ") + cudaGetErrorString(e);
-    return false;
+  const int n = std::max(1, units);
+  std::vector<std::vector<char>> cubin(n);
+  std::vector<std::string> log(n);
+  std::vector<char> ok(n, 0);
+  std::vector<std::thread> work;
+  for (int u = 1; u < n; ++u)
+    work.emplace_back([&, u] { ok[u] = jit_compile(src, strict, false, &cubin[u], &log[u], u + 1); });
+  ok[0] = jit_compile(src, strict, false, &cubin[0], &log[0], units ? 1 : 0);
+  for (auto& t : work) t.join();
+  for (int u = 0; u < n; ++u) {
+    if (!ok[u]) {
+      *why = log[u].substr(0, 4000);
+      return false;
+    }
+    cudaLibrary_t lib = nullptr;
+    cudaError_t e = cudaLibraryLoadData(&lib, cubin[u].data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
+    if (e != cudaSuccess) {
+      *why = std::string("cudaLibraryLoadData: ") + cudaGetErrorString(e);
+      for (auto l : out->libs) cudaLibraryUnload(l);
+      out->libs.clear();
+      return false;
+    }
+    out->libs.push_back(lib);
   }
   out->ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0)
                 .count();
   return true;
+}
+cudaError_t find_kernel(const Compiled& c, cudaKernel_t* k, const char* name) {
+  cudaError_t e = cudaErrorSymbolNotFound;
+  for (auto lib : c.libs)
+    if ((e = cudaLibraryGetKernel(k, lib, name)) == cudaSuccess) return e;
+  cudaGetLastError();  // the units that do not hold it
+  return e;
 }
 
 }  // namespace
@@ -1363,7 +1548,7 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
     if (it != g_cache.end()) {
       cmp = it->second;
     } else {
-      if (!compile_and_load(src, strict, &cmp, why)) return nullptr;
+      if (!compile_and_load(src, strict, kJitUnits, &cmp, why)) return nullptr;
       g_cache[key] = cmp;
       ms = cmp.ms;
     }
@@ -1371,12 +1556,13 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
   auto J = std::make_shared<JitChem>();
   J->compile_ms = ms;
   auto get = [&](cudaKernel_t* k, const char* name) {
-    cudaError_t e = cudaLibraryGetKernel(k, cmp.lib, name);
+    cudaError_t e = find_kernel(cmp, k, name);
     if (e != cudaSuccess && why->empty())
       *why = std::string("cudaLibraryGetKernel(") + name + "): " + cudaGetErrorString(e);
     return e == cudaSuccess;
   };
-  bool ok = get(&J->attempt[0][0], "rs_jit_attempt_r0") && get(&J->attempt[0][1], "rs_jit_attempt_r1") &&
+  bool ok = get(&J->small[0], "rs_jit_attempt_l0") && get(&J->small[1], "rs_jit_attempt_l1") &&
+            get(&J->attempt[0][0], "rs_jit_attempt_r0") && get(&J->attempt[0][1], "rs_jit_attempt_r1") &&
             get(&J->attempt[2][0], "rs_jit_attempt_q0") && get(&J->attempt[2][1], "rs_jit_attempt_q1") &&
             get(&J->per_cell[0], "rs_jit_per_cell_0") && get(&J->per_cell[1], "rs_jit_per_cell_1") &&
             get(&J->rcp, "rs_jit_rcp") && get(&J->vjp[0], "rs_jit_vjp_0") &&
@@ -1433,17 +1619,30 @@ int jit_attempt_block(int nc) {
 #endif
 }
 
+// The attempt variant a handle starts with: 128 registers and 16 warps per SM ("regs2") hide the
+// spills' latency once the grid fills them (1,042 us per call against 1,145 with 255 registers on
+// 615,888 cells, 348 against 364 on 155,664); below, their last wave is too coarse (285 against 259
+// us on 111,555).
+int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.attempt[2][0] ? 2 : 0; }
+
+// Up to one warp per SM sub-partition (152 SMs, four each) the attempt's time is its FP64 chain: W in
+// registers and the FP64 norm, whatever variant is set (6,480 cells: 40 us per attempt, 45 with the
+// float-pair norm).  Beyond, the pairs win (615,888 cells: 1,070 us with the FP64 norm, 981 with
+// pairs, both with 128 registers).
+static bool attempt_fp64_norm(int nc) { return nc <= 152 * 128; }
+
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                         double* U0, double* U1, const double* kr, const double* em,
                         double* part, double rtol, double atol, int clamp, double* F0,
                         double* F1) {
   const int v = J.attempt[J.variant][0] ? J.variant : 0;
-  cudaKernel_t k = J.attempt[v][em ? 1 : 0];
+  const bool small = attempt_fp64_norm(nc);
+  cudaKernel_t k = small ? J.small[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
   if (!F0 || !F1) F0 = F1 = nullptr;
   void* args[] = {&c, &U0, &U1, &kr, &em, &part, &nc, &nsp, &rtol, &atol, &clamp, &F0, &F1};
   const int block = jit_attempt_block(nc);
-  cudaLaunchKernel((const void*)k, dim3((nc + block - 1) / block), dim3(block), args, J.attempt_smem[v], st);
+  cudaLaunchKernel((const void*)k, dim3((nc + block - 1) / block), dim3(block), args, small ? 0 : J.attempt_smem[v], st);
 }
 
 void jit_launch_step(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
@@ -1495,13 +1694,13 @@ std::shared_ptr<WideChem> wide_chem_build(const MechTables& T, double ros_d, dou
     if (it != g_cache.end()) {
       cmp = it->second;
     } else {
-      if (!compile_and_load(src, false, &cmp, why)) return nullptr;
+      if (!compile_and_load(src, false, 0, &cmp, why)) return nullptr;
       g_cache[src + "|wide"] = cmp;
     }
   }
   auto Wc = std::make_shared<WideChem>();
   cudaKernel_t* k = per_cell ? &Wc->per_cell : &Wc->attempt;
-  cudaError_t e = cudaLibraryGetKernel(k, cmp.lib, per_cell ? "rs_wide_per_cell" : "rs_wide_attempt");
+  cudaError_t e = find_kernel(cmp, k, per_cell ? "rs_wide_per_cell" : "rs_wide_attempt");
   Wc->smem = wide_smem_bytes(T);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)*k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wc->smem);

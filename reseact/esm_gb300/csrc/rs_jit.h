@@ -32,6 +32,7 @@ extern const char* const kJitVariantNames[kJitVariants];
 
 struct JitChem {
   cudaKernel_t attempt[kJitVariants][2] = {};  // [variant][has emission]; null: not built
+  cudaKernel_t small[2] = {};                  // grids of up to a warp per SM sub-partition
   cudaKernel_t per_cell[2] = {};               // [has emission]
   cudaKernel_t rcp = nullptr;                  // elementwise production reciprocal
   cudaKernel_t vjp[2] = {};                    // ROS23 step VJP [has emission]
@@ -58,10 +59,12 @@ std::string jit_chem_source(const MechTables& T, bool strict);
 // NVRTC compile of generated source to an sm_103a cubin; needs no device.  With verbose the
 // log carries ptxas's resource usage.  Returns false with the error text in *log.
 bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<char>* cubin,
-                 std::string* log);
+                 std::string* log, int unit = 0);  // unit: one of the source's units, 0 for all
 
 // Threads per block of the attempt kernels over nc cells (one partial sum per block).
 int jit_attempt_block(int nc);
+// The attempt variant for nc cells before the autotuner or the caller picks one.
+int jit_default_variant(const JitChem& J, int nc);
 
 // Same contracts as launch_ros23_attempt / launch_chem_per_cell in rs_kernels.h.
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
