@@ -374,24 +374,6 @@ __global__ void __launch_bounds__(128) k_adv_line(DevTransport<double> T, StageS
   }
 }
 
-// The air-mass fluxes with the cells' metric and the uniform edges' 1/6 folded in: mx6 (both
-// cells of a lon face share the row's factor), myn6 / mys6 (as the cell south / north of a lat face
-// sees it; zero through closed walls; the south-most open face has no cell south of it, its myn6
-// serves the upwind direction only).  Once per forcing change.
-__global__ void k_scale_fluxes(DevTransport<double> T, double* __restrict__ mx6,
-                               double* __restrict__ myn6, double* __restrict__ mys6) {
-  const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t nx = (size_t)T.nlev * T.nlat * (T.nlon + 1), ny = (size_t)T.nlev * (T.nlat + 1) * T.nlon;
-  if (x < nx) mx6[x] = T.mx[x] * (T.gx[(x / (T.nlon + 1)) % T.nlat] * kOneSixth);
-  if (x < ny) {
-    const int f = (int)((x / T.nlon) % (T.nlat + 1));
-    const bool wall = T.lat_bc != 1 && (f == 0 || f == T.nlat);
-    const double m = T.my[x];
-    myn6[x] = wall ? 0.0 : m * ((f > 0 ? T.gyhi[f - 1] : T.gylo[0]) * kOneSixth);
-    mys6[x] = wall || f == T.nlat ? 0.0 : m * (T.gylo[f] * kOneSixth);
-  }
-}
-
 // ------------------------------------------------------------------ stage kernels
 // stage in 1..4 of one attempt from the accumulator acc (m dq/dt = -g acc):
 //   1: S1 = U + dt/2 f(U)           2: S2 = S1 + dt/2 f(S1)

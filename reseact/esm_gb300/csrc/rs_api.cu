@@ -330,8 +330,8 @@ struct rs_handle {
   DevBuf<double> mx, my, mz, qw, qe, qs, qn, gx, gylo, gyhi, vsA, vsB, veAB, veC, veD, dtcell,
       stepcell, totals;
   DevBuf<float> qhi, qlo;  // mixed-precision transport: split planes
-  DevBuf<float> gx2, gylo2, gyhi2, vsA2, vsB2, veAB2, veC2, veD2;  // (hi, lo) pairs
-  DevBuf<float> mx2, my2, mz2;  // the face fluxes as (hi, lo) pairs (mixed precision)
+  DevBuf<float> vsA2, vsB2, veAB2, veC2, veD2;  // hi and lo planes
+  DevBuf<float> mx12, myn12, mys12, mz2;  // the face fluxes as hi and lo planes (mixed precision)
   rs::MixedTmaps* tmaps = nullptr;  // bulk-copy staging of the mixed pencils (null: unavailable)
   void* noalloc_base = nullptr;     // this device's scratch of rs_ros23_attempt_noalloc
   std::string tmaps_why;
@@ -534,34 +534,37 @@ void build_device_mech(rs_handle* h) {
   h->slot_col.upload(T.slot_col.data(), T.slot_col.size(), h->st);
 }
 
-// (hi, lo) float pairs of a double array for the compensated FP32 transport:
+// scale times a double array as hi and lo planes for the compensated FP32 transport:
 // hi = fl32(v), lo = fl32(v - hi); hi + lo = v to about 2^-48 relative
-void upload_pairs(const std::vector<double>& v, DevBuf<float>& d, cudaStream_t st) {
-  std::vector<float> w(2 * v.size());
-  for (size_t i = 0; i < v.size(); ++i) {
-    const float hi = (float)v[i];
-    w[2 * i] = hi;
-    w[2 * i + 1] = (float)(v[i] - (double)hi);
+void upload_pairs(const std::vector<double>& v, double scale, DevBuf<float>& d, cudaStream_t st) {
+  const size_t n = v.size();
+  std::vector<float> w(2 * n);
+  for (size_t i = 0; i < n; ++i) {
+    const double x = v[i] * scale;
+    const float hi = (float)x;
+    w[i] = hi;
+    w[n + i] = (float)(x - (double)hi);
   }
   d.upload(w.data(), w.size(), st);
   CK(cudaStreamSynchronize(st));  // w is a temporary
 }
 
-// The air-mass face fluxes as (hi, lo) pairs for the compensated FP32 kernels (after every
+// The air-mass face fluxes as hi and lo planes for the compensated FP32 kernels (after every
 // flux change, including the pressure fixer's diagnosed Mz).
 void make_flux_pairs(rs_handle* h) {
-  h->mx2.alloc(2 * h->mx.n);
-  h->my2.alloc(2 * h->my.n);
-  h->mz2.alloc(2 * h->mz.n);
-  rs::launch_make_pairs(h->st, h->mx.p, reinterpret_cast<float2*>(h->mx2.p), h->mx.n);
-  rs::launch_make_pairs(h->st, h->my.p, reinterpret_cast<float2*>(h->my2.p), h->my.n);
-  rs::launch_make_pairs(h->st, h->mz.p, reinterpret_cast<float2*>(h->mz2.p), h->mz.n);
+  auto planes = [&](const DevBuf<double>& src, double scale, DevBuf<float>& dst) {
+    dst.alloc(2 * src.n);
+    rs::launch_make_pairs(h->st, src.p, scale, dst.p, src.n);
+  };
+  planes(h->mx6, 0.5, h->mx12);
+  planes(h->myn6, 0.5, h->myn12);
+  planes(h->mys6, 0.5, h->mys12);
+  planes(h->mz, 1.0, h->mz2);
   CK(cudaGetLastError());
 }
 
-// The production FP64 kernels' scaled fluxes (after every flux change).
+// The kernels' scaled fluxes (after every flux change).
 void scale_fluxes(rs_handle* h) {
-#if !RS_STRICT
   h->mx6.alloc(h->mx.n);
   h->myn6.alloc(h->my.n);
   h->mys6.alloc(h->my.n);
@@ -572,9 +575,6 @@ void scale_fluxes(rs_handle* h) {
   T.mx = h->mx.p; T.my = h->my.p;
   rs::launch_scale_fluxes(h->st, T, h->mx6.p, h->myn6.p, h->mys6.p);
   CK(cudaGetLastError());
-#else
-  (void)h;
-#endif
 }
 
 // Lat-lon geometry on the unit sphere (same formulas and order as the CPU restatement).
@@ -602,11 +602,6 @@ void build_geometry(rs_handle* h) {
   h->gx_host = gx;
   h->gylo_host = gl;
   h->gyhi_host = gh;
-  if (h->cfg.precision == RS_PREC_MIXED) {
-    upload_pairs(gx, h->gx2, h->st);
-    upload_pairs(gl, h->gylo2, h->st);
-    upload_pairs(gh, h->gyhi2, h->st);
-  }
 }
 
 // CW84 nonuniform coefficients from dp (eqs. 1.6-1.7), mirror ghosts at the no-flux walls.
@@ -646,11 +641,12 @@ void build_vertical(rs_handle* h) {
   h->veC.upload(eC.data(), eC.size(), h->st);
   h->veD.upload(eD.data(), eD.size(), h->st);
   if (h->cfg.precision == RS_PREC_MIXED) {
-    upload_pairs(sA, h->vsA2, h->st);
-    upload_pairs(sB, h->vsB2, h->st);
-    upload_pairs(eAB, h->veAB2, h->st);
-    upload_pairs(eC, h->veC2, h->st);
-    upload_pairs(eD, h->veD2, h->st);
+    // the mixed kernels carry twice the slopes
+    upload_pairs(sA, 2.0, h->vsA2, h->st);
+    upload_pairs(sB, 2.0, h->vsB2, h->st);
+    upload_pairs(eAB, 1.0, h->veAB2, h->st);
+    upload_pairs(eC, 0.5, h->veC2, h->st);
+    upload_pairs(eD, 0.5, h->veD2, h->st);
   }
   CK(cudaStreamSynchronize(h->st));  // the host vectors above are temporaries
 }
@@ -670,12 +666,12 @@ void refresh_dt(rs_handle* h) {
   T.mx6 = h->mx6.p; T.myn6 = h->myn6.p; T.mys6 = h->mys6.p;
   T.mixed = h->cfg.precision == RS_PREC_MIXED;
   T.qhi = h->qhi.p; T.qlo = h->qlo.p;
-  auto f2 = [](const DevBuf<float>& b) { return reinterpret_cast<const float2*>(b.p); };
-  T.gx2 = f2(h->gx2); T.gylo2 = f2(h->gylo2); T.gyhi2 = f2(h->gyhi2);
-  T.vsA2 = f2(h->vsA2); T.vsB2 = f2(h->vsB2); T.veAB2 = f2(h->veAB2); T.veC2 = f2(h->veC2);
-  T.veD2 = f2(h->veD2);
-  T.acc = T.mixed ? reinterpret_cast<float2*>(h->fx.p) : nullptr;  // ntr*nc pairs
-  T.mx2 = f2(h->mx2); T.my2 = f2(h->my2); T.mz2 = f2(h->mz2);
+  auto pp = [](const DevBuf<float>& b) { return rs::PairPlanes{b.p, b.p ? b.p + b.n / 2 : nullptr}; };
+  T.vsA2 = pp(h->vsA2); T.vsB2 = pp(h->vsB2); T.veAB2 = pp(h->veAB2); T.veC2 = pp(h->veC2);
+  T.veD2 = pp(h->veD2);
+  T.mx12 = pp(h->mx12); T.myn12 = pp(h->myn12); T.mys12 = pp(h->mys12); T.mz2 = pp(h->mz2);
+  T.acc.h = T.mixed ? reinterpret_cast<float*>(h->fx.p) : nullptr;  // ntr*nc pairs
+  T.acc.l = T.mixed ? T.acc.h + (size_t)h->ntr * h->nc : nullptr;
   T.pencil = h->tune.pencil;
   T.rows = h->tune.rows;
   T.xthreads = h->tune.xthreads;
@@ -1095,8 +1091,8 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
       h->dp_host.assign(h->nc, 1.0);
       build_vertical(h);
     }
-    if (cfg->do_transport && cfg->precision == RS_PREC_MIXED) make_flux_pairs(h);  // zero fluxes
     if (cfg->do_transport) scale_fluxes(h);
+    if (cfg->do_transport && cfg->precision == RS_PREC_MIXED) make_flux_pairs(h);  // zero fluxes
     refresh_dt(h);
     if (cfg->do_transport && cfg->precision == RS_PREC_MIXED) {
       const char* why = nullptr;
@@ -1122,8 +1118,8 @@ void rs_destroy(rs_handle* h) {
   if (h->cap) cudaStreamDestroy(h->cap);
   for (auto& b : h->itabs) b.release();
   for (auto& b : h->dtabs) b.release();
-  DevBuf<float>* fbufs[] = {&h->qhi, &h->qlo, &h->gx2, &h->gylo2, &h->gyhi2, &h->vsA2,
-                            &h->vsB2, &h->veAB2, &h->veC2, &h->veD2, &h->mx2, &h->my2, &h->mz2};
+  DevBuf<float>* fbufs[] = {&h->qhi, &h->qlo, &h->vsA2, &h->vsB2, &h->veAB2, &h->veC2, &h->veD2,
+                            &h->mx12, &h->myn12, &h->mys12, &h->mz2};
   for (auto* b : fbufs) b->release();
   DevBuf<double>* bufs[] = {&h->U[0], &h->U[1], &h->S1, &h->S2, &h->S3, &h->fx, &h->fy, &h->fz,
                             &h->mx6, &h->myn6, &h->mys6,
@@ -1245,8 +1241,8 @@ rs_status rs_set_forcing(rs_handle* h, const rs_forcing* f) {
       if (pbl_inputs) build_pbl(h);
       if (f->dps_dt) h->dpsdt_host.assign(f->dps_dt, f->dps_dt + ncol);
       if (f->dps_dt || f->hyb_b || f->mx || f->my || f->mz || f->dp) build_fixer(h);
-      if (h->cfg.precision == RS_PREC_MIXED) make_flux_pairs(h);
       if (f->mx || f->my) scale_fluxes(h);
+      if (h->cfg.precision == RS_PREC_MIXED) make_flux_pairs(h);
     }
     if (f->temperature) {
       h->T.upload(f->temperature, nc, st);

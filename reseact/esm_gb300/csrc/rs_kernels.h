@@ -35,6 +35,11 @@ struct PerCellArgs {
   double* totals;  // [accepted substeps, attempts] summed over cells, or null
 };
 
+struct PairPlanes {  // values as hi + lo, one plane each
+  const float* h;
+  const float* l;
+};
+
 // Transport geometry and forcing on the device (grid SoA, lon fastest).
 template <typename R>
 struct DevTransport {
@@ -66,22 +71,17 @@ struct DevTransport {
   const double* myn6;  // shape of my, as the cell south of the face sees it
   const double* mys6;  // and the cell north of it
   // mixed precision (compensated FP32): the RHS input split into hi, lo planes [ntr][nc]
-  // (hi + lo = q to 2^-47), the metric factors and vertical coefficients as (hi, lo) pairs, and
-  // the per-cell accumulator of m dq/dt as pairs [ntr][nc]
+  // (hi + lo = q to 2^-47), the vertical coefficients (twice the slopes', half the edges' slope
+  // terms) and the air-mass face fluxes as hi and lo planes (mx12 .. mys12: mx6 .. mys6 / 2), and
+  // the accumulator of -m dq/dt / g per cell
   float* qhi;
   float* qlo;
-  const float2* gx2;    // [nlat]
-  const float2* gylo2;  // [nlat]
-  const float2* gyhi2;  // [nlat]
-  const float2* vsA2;   // as vsA / vsB / veAB / veC / veD
-  const float2* vsB2;
-  const float2* veAB2;
-  const float2* veC2;
-  const float2* veD2;
-  float2* acc;
-  const float2* mx2;    // the air-mass face fluxes as pairs (shapes of mx, my, mz)
-  const float2* my2;
-  const float2* mz2;
+  PairPlanes vsA2, vsB2, veAB2, veC2, veD2;  // as vsA / vsB / veAB / veC / veD
+  PairPlanes mx12, myn12, mys12, mz2;
+  struct {
+    float* h;
+    float* l;
+  } acc;               // [ntr][nc]
   int mixed;
   // full PBL mixing (transport half): per-layer fraction f and weight w = dp*f, the column
   // normaliser max(sum_k w, 1 Pa), scratch for the per-tracer column means, 1/tau
@@ -174,11 +174,11 @@ size_t mixed_pencil_cap();
 void mixed_tmaps_destroy(MixedTmaps* m);
 bool mixed_tmaps_dir_ok(const MixedTmaps* m, int dir);  // dir 0 lon rows, 1 lat, 2 vertical
 void launch_flux_dir(cudaStream_t st, const DevTransport<double>& T, const double* Q, int dir);
-// the scaled air-mass fluxes mx6, myn6, mys6 from mx, my (production build)
+// the scaled air-mass fluxes mx6, myn6, mys6 from mx, my
 void launch_scale_fluxes(cudaStream_t st, const DevTransport<double>& T, double* mx6, double* myn6,
                          double* mys6);
-// (hi, lo) float pairs of n doubles (the mixed kernels' face fluxes)
-void launch_make_pairs(cudaStream_t st, const double* src, float2* dst, size_t n);
+// scale times n doubles as hi and lo planes, dst[0..n) and dst[n..2n)
+void launch_make_pairs(cudaStream_t st, const double* src, double scale, float* dst, size_t n);
 void launch_flux_dir_mixed(cudaStream_t st, const DevTransport<double>& T, const double* Q, int dir,
                            bool split);
 

@@ -530,126 +530,237 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
 // Compensated FP32 transport.  Every transport value is carried as a double-float pair
 // (value = h + l, |l| <= ulp(h)/2: two FP32 numbers, about 48 significant bits) and combined
 // with error-free transformations (Knuth's TwoSum for sums, FMA-based TwoProduct for products),
-// so the reconstruction runs on the FP32 pipe at FP64-class accuracy.  The face terms are written
-// in advective form: for cell c and face f with air-mass flux M_f, the CWC tendency
-//   m dq/dt = -div(M q) + q div(M) = sum_f sigma_f G_f M_f (q_c - q_f)
-// (sigma_f = +1 on the east / north / top face, -1 on the west / south / bottom face, G_f the
-// face's metric factor) needs only differences: q_c - q_f is minus the edge deviation when c is
-// upwind, or minus (neighbour difference + edge deviation) when it is not.  With
-//   Phi_f = M_f (q_f - q_L),  Psi_f = M_f (q_R - q_f)      (L / R: the cells below / above f)
-// a cell's tendency is -G (Phi_e + Psi_w) along x, -(G_n Phi_n + G_s Psi_s) along y and
-// -(Phi_t + Psi_b) vertically.  No term is of the size of q itself, so a value far smaller
-// than its neighbours keeps its relative accuracy (an FP32 reconstruction of deviations does
-// not: its error scales with the neighbour difference).  q == const gives exactly zero.
+// so the reconstruction runs on the FP32 pipe at FP64-class accuracy.  The face terms are in
+// advective form on edge deviations, as in rs_adv64.cuh: for cell c and face f with air-mass flux
+// M_f, m dq/dt is -(sum over its faces of G_f M_f times A or B), where A = q_f - q_{f-1} goes to
+// the cell below the face, B = D - A to the one above, and q_f - q of the upwind cell is its limited
+// edge deviation -- its own sign with min(|e|, 2 |the opposite edge's|), 0 unless the two edges
+// have strictly opposite signs.  No term is of the size of q itself, so a value far smaller than
+// its neighbours keeps its relative accuracy.  q == const gives exactly zero.
 //
-// Each direction's pencil adds its part of m dq/dt into a per-cell double-float accumulator
-// (x writes it, y and z add), and the stage kernel turns it into the stage update in FP64.
-// The state, the air mass, the stage combinations and the error norm stay FP64.
-struct df {
-  float h, l;
+// The uniform directions carry 12 x the deviations (with slopes doubled, so that every scaling is
+// exact): 12 E_p = 6 D_p - (S'_{p+1} - S'_p), 12 eL_p = -(6 D_{p-1} + (S'_p - S'_{p-1})); the 1/12
+// and the cells' metric are folded into the air-mass fluxes once per forcing, the vertical slope
+// and edge coefficients carry the 2 and 1/2.  Comparisons of pairs are the sign of a difference
+// (three FP32 operations), so they ride the FP32 pipe too.
+//
+// Each direction adds its part into a per-cell pair accumulator (x writes it, y and z add), and
+// the stage kernel turns it into the stage update.  The state, the air mass and the error
+// control stay FP64.
+//
+// What bounds it: issue slots and the FP32 / integer pipes.  Packed f32x2 operations do two
+// tracers per instruction at the scalar rate of flops, so the streaming kernels carry a pair of
+// tracers per thread: half the FP32 issue slots, and the fluxes, vertical coefficients and
+// addresses once for two.  FV<1> and FV<2> form the same values bit for bit (every operation is
+// rounded to nearest on its own; subtraction of packed values is an exact multiply-add with -1).
+// A stage at 360x181x72 with 30 tracers (144x91x47 with 12), one tracer per thread and flux-form
+// pairs before -> now: lon rows 1.20 -> 0.74 ms (85 -> 52 us; of the 0.33 ms its bytes take), lat
+// lines 1.29 -> 0.78 ms (137 -> 65 us; 0.49 ms), vertical lines 2.16 -> 1.04 ms (128 -> 77 us;
+// 0.55 ms).  Doing stages 1-3's update inside the vertical line kernel (one read and one write of
+// the accumulator less) was slower, 1.35 ms and an air-mass kernel of 0.23 against 1.04 + 0.57.
+template <int N>
+struct FV;
+template <>
+struct FV<1> {
+  float v;
 };
-__device__ __forceinline__ df df_two_sum(float a, float b) {  // a + b = s + e exactly
-  const float s = a + b, bb = s - a;
-  return {s, (a - (s - bb)) + (b - bb)};
+template <>
+struct FV<2> {
+  unsigned long long v;
+};
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-// Sum of pairs: TwoSum of the high parts, the low parts added to its error, then the fast
-// renormalisation (h = s + e, l = e - (h - s)).  The renormalisation is exact unless the high
-// parts cancel below the low parts; its error is then below 2^-46 max(|a|, |b|), a few times
-// the operands' own representation error, so the sum keeps the pairs' accuracy at 11
-// operations instead of the 14 of a second TwoSum.
-__device__ __forceinline__ df df_add(df a, df b) {
-  const df s = df_two_sum(a.h, b.h);
-  const float e = s.l + (a.l + b.l);
-  const float h = s.h + e;
-  return {h, e - (h - s.h)};
+__device__ __forceinline__ float half(FV<1> a, int) { return a.v; }
+__device__ __forceinline__ float half(FV<2> a, int i) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return i ? y : x;
 }
-__device__ __forceinline__ df df_neg(df a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ df df_sub(df a, df b) { return df_add(a, df_neg(b)); }
-__device__ __forceinline__ df df_mul(df a, df b) {
-  const float p = a.h * b.h;
-  const float e = fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p)));
-  const float s = p + e;
-  return {s, e - (s - p)};
+template <int N>
+__device__ __forceinline__ FV<N> splat(float a) {
+  if constexpr (N == 1) return {a};
+  else return {pack2(a, a)};
 }
-__device__ __forceinline__ df df_scale(df a, float pow2) { return {a.h * pow2, a.l * pow2}; }
-__device__ __forceinline__ df df_ld(const float* H, const float* L, long long x) {
-  return {H[x], L[x]};
+__device__ __forceinline__ FV<1> vadd(FV<1> a, FV<1> b) { return {__fadd_rn(a.v, b.v)}; }
+__device__ __forceinline__ FV<1> vsub(FV<1> a, FV<1> b) { return {__fsub_rn(a.v, b.v)}; }
+__device__ __forceinline__ FV<1> vmul(FV<1> a, FV<1> b) { return {__fmul_rn(a.v, b.v)}; }
+__device__ __forceinline__ FV<1> vfma(FV<1> a, FV<1> b, FV<1> c) { return {__fmaf_rn(a.v, b.v, c.v)}; }
+__device__ __forceinline__ FV<2> vadd(FV<2> a, FV<2> b) {
+  FV<2> r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
 }
-__device__ __forceinline__ df df_ld2(const float2* p, size_t x) {
-  const float2 v = p[x];
-  return {v.x, v.y};
+__device__ __forceinline__ FV<2> vmul(FV<2> a, FV<2> b) {
+  FV<2> r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
 }
-// 1/6 as a pair (hi = fl(1/6), lo = fl(1/6 - hi))
-constexpr float kSixthH = (float)(1.0 / 6.0);
-constexpr float kSixthL = (float)(1.0 / 6.0 - (double)(float)(1.0 / 6.0));
+__device__ __forceinline__ FV<2> vfma(FV<2> a, FV<2> b, FV<2> c) {
+  FV<2> r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ FV<2> vsub(FV<2> a, FV<2> b) { return vfma(b, splat<2>(-1.0f), a); }
+// halves of a where m[i], of b otherwise
+template <int N>
+struct Mask {
+  bool m[N];
+};
+template <int N>
+__device__ __forceinline__ FV<N> vsel(const Mask<N>& k, FV<N> a, FV<N> b) {
+  if constexpr (N == 1) return {k.m[0] ? a.v : b.v};
+  else return {pack2(k.m[0] ? half(a, 0) : half(b, 0), k.m[1] ? half(a, 1) : half(b, 1))};
+}
+// x and y have the same sign bit (one logic instruction that sets the predicate)
+template <int N>
+__device__ __forceinline__ Mask<N> same_sign(FV<N> x, FV<N> y) {
+  Mask<N> r;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    r.m[i] = ((__float_as_uint(half(x, i)) ^ __float_as_uint(half(y, i))) & 0x80000000u) == 0u;
+  return r;
+}
 
-// |a| < |b| for pairs of the same sign (sg = +1 or -1 their sign)
-__device__ __forceinline__ bool df_absless(df a, df b, float sg) {
-  return (fabsf(a.h) < fabsf(b.h)) || (a.h == b.h && sg * a.l < sg * b.l);
+template <int N>
+struct DF {
+  FV<N> h, l;
+};
+using df = DF<1>;
+__device__ __forceinline__ df mkdf(float h, float l) { return {{h}, {l}}; }
+// the pair (h, l) in both halves
+template <int N>
+__device__ __forceinline__ DF<N> splat_df(float h, float l) {
+  return {splat<N>(h), splat<N>(l)};
 }
-// CW84 eq. 1.8 monotonised slope from the neighbour differences d0 (left) and d1 (right):
-// 0 unless they have the same strict sign, else the smallest in magnitude of the centred
-// slope da and 2 d0, 2 d1 (all three share that sign)
-__device__ __forceinline__ df mc_pick(df d0, df d1, df da) {
-  const bool same = (d0.h > 0.0f && d1.h > 0.0f) || (d0.h < 0.0f && d1.h < 0.0f);
-  const float sg = d0.h > 0.0f ? 1.0f : -1.0f;
-  df m = da;
-  const df t0 = df_scale(d0, 2.0f), t1 = df_scale(d1, 2.0f);
-  if (df_absless(t0, m, sg)) m = t0;
-  if (df_absless(t1, m, sg)) m = t1;
-  return same ? m : df{0.0f, 0.0f};
+// (h, l) from a leading part s and a small correction e
+template <int N>
+__device__ __forceinline__ DF<N> df_renorm(DF<N> a) {
+  const FV<N> h = vadd(a.h, a.l);
+  return {h, vsub(a.l, vsub(h, a.h))};
 }
-__device__ __forceinline__ df mc_slope(df d0, df d1) {
-  return mc_pick(d0, d1, df_scale(df_add(d0, d1), 0.5f));
+// Sums of pairs: TwoSum of the high parts, the low parts added to its error.  Exact but for the
+// roundings of the low parts, 2^-48 of the operands.  The _raw forms leave the result
+// unnormalised (l may be a few ulp of h, more where the high parts cancel); that is enough for
+// an operand of another sum or product, while a pair whose sign or size is looked at is normalised
+// unless its parts cannot cancel.
+template <int N>
+__device__ __forceinline__ DF<N> add_raw(DF<N> a, DF<N> b) {
+  const FV<N> s = vadd(a.h, b.h), bb = vsub(s, a.h);
+  return {s, vadd(vadd(vsub(a.h, vsub(s, bb)), vsub(b.h, bb)), vadd(a.l, b.l))};
 }
-__device__ __forceinline__ df mc_slope_n(df d0, df d1, df sA, df sB) {  // dp-weighted centre
-  return mc_pick(d0, d1, df_add(df_mul(sA, d1), df_mul(sB, d0)));
+template <int N>
+__device__ __forceinline__ DF<N> sub_raw(DF<N> a, DF<N> b) {
+  const FV<N> s = vsub(a.h, b.h), bb = vsub(s, a.h);
+  return {s, vadd(vsub(vsub(a.h, vsub(s, bb)), vadd(b.h, bb)), vsub(a.l, b.l))};
 }
-// CW84 eq. 1.10 limiter on the upwind cell's edge deviations (aL, aR) from its own value
-// (a = 0): flatten unless aL and aR have strictly opposite signs, else steepen where the
-// parabola overshoots; the tests dA a6 > dA^2 and -dA^2 > dA a6 of the FP64 form become sign
-// tests of aL + 2 aR and 2 aL + aR.  Returns the limited right (M > 0) or left edge.
-__device__ __forceinline__ df lim_pick(df aL, df aR, bool right) {
-  const bool opp = (aR.h > 0.0f && aL.h < 0.0f) || (aR.h < 0.0f && aL.h > 0.0f);
-  const float sR = aR.h > 0.0f ? 1.0f : -1.0f;
-  const df t1 = df_add(aL, df_scale(aR, 2.0f));
-  const df t2 = df_add(df_scale(aL, 2.0f), aR);
-  const bool c1 = sR * t1.h < 0.0f;
-  const bool c2 = !c1 && sR * t2.h > 0.0f;
-  df r = right ? (c2 ? df_scale(aL, -2.0f) : aR) : (c1 ? df_scale(aR, -2.0f) : aL);
-  return opp ? r : df{0.0f, 0.0f};
+// a + b and a - b for |a| > |b| or a = b = 0: the shorter FastTwoSum
+template <int N>
+__device__ __forceinline__ DF<N> add_big(DF<N> a, DF<N> b) {
+  const FV<N> s = vadd(a.h, b.h);
+  return {s, vadd(vadd(vsub(a.h, s), b.h), vadd(a.l, b.l))};
 }
-// Edge term E_p of cell p (the deviation of edge p+1/2 from cell p, unlimited), uniform grid:
-// E_p = D_p / 2 - (S_{p+1} - S_p) / 6; the left edge of cell p is E_{p-1} - D_{p-1}.
-__device__ __forceinline__ df edge_u(df Dp, df Sp, df Sp1) {
-  return df_sub(df_scale(Dp, 0.5f), df_mul(df_sub(Sp1, Sp), df{kSixthH, kSixthL}));
+template <int N>
+__device__ __forceinline__ DF<N> sub_big(DF<N> a, DF<N> b) {
+  const FV<N> s = vsub(a.h, b.h);
+  return {s, vadd(vsub(vsub(a.h, s), b.h), vsub(a.l, b.l))};
 }
-// dp-weighted: E_p = ab D_p + c S_{p+1} + d S_p with the coefficients of edge p+1
-__device__ __forceinline__ df edge_n(df Dp, df Sp, df Sp1, df ab, df c, df d) {
-  return df_add(df_add(df_mul(ab, Dp), df_mul(c, Sp1)), df_mul(d, Sp));
+template <int N>
+__device__ __forceinline__ DF<N> df_add(DF<N> a, DF<N> b) { return df_renorm(add_raw(a, b)); }
+template <int N>
+__device__ __forceinline__ DF<N> df_sub(DF<N> a, DF<N> b) { return df_renorm(sub_raw(a, b)); }
+template <int N>
+__device__ __forceinline__ DF<N> df_scale(DF<N> a, float pow2) {
+  return {vmul(a.h, splat<N>(pow2)), vmul(a.l, splat<N>(pow2))};
 }
-// A cell's two faces along one direction: w (below, flux Mw) and e (above, flux Me).
-// E(o), D(o) give E_{p+o}, D_{p+o}.  Returns {Psi_w, Phi_e}; a face with M == 0 (a wall)
-// contributes exactly 0.
-template <class FE, class FD>
-__device__ __forceinline__ void cell_faces(df Mw, df Me, FE E, FD D, df& psi, df& phi) {
-  psi = df{0.0f, 0.0f};
-  phi = df{0.0f, 0.0f};
-  if (Mw.h > 0.0f) {  // upwind p-1: its right edge
-    const df dev = lim_pick(df_sub(E(-2), D(-2)), E(-1), true);
-    psi = df_mul(Mw, df_sub(D(-1), dev));
-  } else if (Mw.h < 0.0f) {  // upwind p: its left edge
-    const df dev = lim_pick(df_sub(E(-1), D(-1)), E(0), false);
-    psi = df_mul(Mw, df_neg(dev));
-  }
-  if (Me.h > 0.0f) {  // upwind p: its right edge
-    const df dev = lim_pick(df_sub(E(-1), D(-1)), E(0), true);
-    phi = df_mul(Me, dev);
-  } else if (Me.h < 0.0f) {  // upwind p+1: its left edge
-    const df dev = lim_pick(df_sub(E(0), D(0)), E(1), false);
-    phi = df_mul(Me, df_add(D(0), dev));
-  }
+template <int N>
+__device__ __forceinline__ DF<N> mul_raw(DF<N> a, DF<N> b) {
+  const FV<N> p = vmul(a.h, b.h);
+  return {p, vfma(a.h, b.l, vfma(a.l, b.h, vfma(a.h, b.h, vmul(p, splat<N>(-1.0f)))))};
 }
+template <int N>
+__device__ __forceinline__ DF<N> fma_raw(DF<N> a, DF<N> b, DF<N> c) {  // a b + c
+  const DF<N> p = mul_raw(a, b);
+  const FV<N> s = vadd(c.h, p.h), bb = vsub(s, c.h);
+  return {s, vadd(vadd(vsub(c.h, vsub(s, bb)), vsub(p.h, bb)), vadd(c.l, p.l))};
+}
+template <int N>
+__device__ __forceinline__ DF<N> df_fma(DF<N> a, DF<N> b, DF<N> c) { return df_renorm(fma_raw(a, b, c)); }
+template <int N>
+__device__ __forceinline__ DF<N> times6(DF<N> a) {  // unnormalised
+  const FV<N> k = splat<N>(6.0f), p = vmul(a.h, k);
+  return {p, vfma(a.l, k, vfma(a.h, k, vmul(p, splat<N>(-1.0f))))};
+}
+template <int N>
+__device__ __forceinline__ DF<N> df_sel(const Mask<N>& k, DF<N> a, DF<N> b) {
+  return {vsel(k, a.h, b.h), vsel(k, a.l, b.l)};
+}
+template <int N>
+__device__ __forceinline__ FV<N> df_diff(DF<N> a, DF<N> b) {  // a - b, exact in sign
+  return vadd(vsub(a.h, b.h), vsub(a.l, b.l));
+}
+__device__ __forceinline__ df df_ld(const float* H, const float* L, long long x) { return mkdf(H[x], L[x]); }
+__device__ __forceinline__ df df_ldp(const PairPlanes& P, size_t x) { return mkdf(P.h[x], P.l[x]); }
+template <int N>
+__device__ __forceinline__ DF<N> df_ldc(const PairPlanes& P, size_t x) {  // one value for all tracers
+  return splat_df<N>(P.h[x], P.l[x]);
+}
+
+// k where a and b have the same sign, else 0 (a zero counts by its sign bit: the limited values
+// below are 0 either way)
+template <int N>
+__device__ __forceinline__ FV<N> live(DF<N> a, DF<N> b, float k) {
+  const Mask<N> m = same_sign(a.h, b.h);
+  if constexpr (N == 1) return {m.m[0] ? k : 0.0f};
+  else return {pack2(m.m[0] ? k : 0.0f, m.m[1] ? k : 0.0f)};
+}
+// the smaller in magnitude of `self` and k `other`, which have one sign wherever k is not 0
+template <int N>
+__device__ __forceinline__ DF<N> limit(DF<N> self, DF<N> other, FV<N> k) {
+  const DF<N> m{vmul(other.h, k), vmul(other.l, k)};
+  return df_sel(same_sign(df_diff(self, m), self.h), m, self);
+}
+// Twice the CW84 eq. 1.8 monotonised slope from the neighbour differences d0 (left), d1 (right) and
+// twice the centred slope w: 0 unless d0, d1 have the same sign (k4 = live(d0, d1, 4)), else the
+// smallest in magnitude of w, 4 d0, 4 d1.
+template <int N>
+__device__ __forceinline__ DF<N> slope2(DF<N> d0, DF<N> d1, DF<N> w, FV<N> k4) {
+  return limit(w, df_sel(same_sign(df_diff(d0, d1), d0.h), d1, d0), k4);
+}
+// The two face terms A, B of a face from x, the limited q_f - q_{f-1} (upwind below) or q_f' of
+// the cell above, and y, the rest of the neighbour difference
+template <int N>
+__device__ __forceinline__ void face_terms(DF<N> x, DF<N> y, bool right, DF<N>& A, DF<N>& B) {
+  A = right ? x : y;
+  B = right ? y : x;
+}
+// Uniform directions: 6 D, 12 E_p = 6 D_p - (S'_{p+1} - S'_p) and 12 L_{p+1} = 6 D_p + (S'_{p+1} -
+// S'_p), L = -eL.  Both slopes are limited by 4 D_p and have its sign, so |dS'| <= 4 |D_p|: no
+// cancellation, E_p and L_{p+1} have the sign of D_p and need no normalisation.
+template <int N>
+__device__ __forceinline__ void edges_u(DF<N> D, DF<N> S0, DF<N> S1, DF<N>& t, DF<N>& E, DF<N>& Lnext) {
+  t = times6(D);
+  const DF<N> ds = sub_raw(S1, S0);
+  E = sub_big(t, ds);
+  Lnext = add_big(t, ds);
+}
+// x = 12 (limited deviation) lies between 0 and 10 D: the rest of 12 D does not cancel
+template <int N>
+__device__ __forceinline__ DF<N> rest_u(DF<N> t, DF<N> x) { return sub_big(df_scale(t, 2.0f), x); }
+// dp-weighted: E_p = ab D_p + c S_{p+1} + d S_p with the coefficients of edge p+1; L = D - E of
+// the cell before
+template <int N>
+__device__ __forceinline__ DF<N> edge_n(DF<N> D, DF<N> S0, DF<N> S1, DF<N> ab, DF<N> c, DF<N> d) {
+  return df_fma(d, S0, fma_raw(c, S1, mul_raw(ab, D)));
+}
+template <int N>
+__device__ __forceinline__ DF<N> centre_n(DF<N> d0, DF<N> d1, DF<N> sA, DF<N> sB) {  // twice the centred slope
+  return df_fma(sA, d1, mul_raw(sB, d0));
+}
+// the upwind cell is the one below the face: sign of g M (gs: the bits of g's high word)
+__device__ __forceinline__ bool upwind_lo(float M, int gs) { return (__float_as_int(M) ^ gs) >= 0; }
 // split a double into a pair: production build with integer operations (split_bits below,
 // truncating: hi + lo = v to 2^-47), strict build with conversions
 __device__ __forceinline__ df split_df(double v);
@@ -663,11 +774,11 @@ __device__ __forceinline__ double f2d_bits(float x) {
   return __hiloint2double((int)((u & 0x80000000u) | ((fe + 896u) << 20) | ((u & 0x7fffffu) >> 3)),
                           (int)(u << 29));
 }
-__device__ __forceinline__ double df_to_d(float2 v) {
+__device__ __forceinline__ double df_to_d(df v) {
 #if RS_STRICT
-  return (double)v.x + (double)v.y;
+  return (double)v.h.v + (double)v.l.v;
 #else
-  return f2d_bits(v.x) + f2d_bits(v.y);
+  return f2d_bits(v.h.v) + f2d_bits(v.l.v);
 #endif
 }
 
@@ -762,7 +873,7 @@ __global__ void __launch_bounds__(256) k_adv_x_mixed(DevTransport<double> T, Sta
   const double* Q;
   double g;
   if (!resolve_stage(sel, Q, g)) return;
-  const df gd = split_df(g);  // the stage time factor as a pair
+  const int gs = __double2hiint(g);  // only its sign is needed here
   const int s0 = blockIdx.y * sper, s1 = min(T.ntr, s0 + sper);  // this block's tracers
   extern __shared__ __align__(16) unsigned char smx32_raw[];
   float* smx32 = align128(smx32_raw);
@@ -785,7 +896,6 @@ __global__ void __launch_bounds__(256) k_adv_x_mixed(DevTransport<double> T, Sta
   const size_t rbase = ((size_t)k * T.nlat + j) * n;
   const bool periodic = T.lon_bc == 0;
   const int tid = threadIdx.x;
-  const df G = df_ld2(T.gx2, j);
   auto X = [&](int p) { return bck(T, p + kHoX, L); };  // row index of cell p
   int uses0 = 0, uses1 = 0;  // copies issued per buffer
   auto issue = [&](int s, int b) {  // one tracer's interior hi / lo rows (n floats each)
@@ -806,9 +916,9 @@ __global__ void __launch_bounds__(256) k_adv_x_mixed(DevTransport<double> T, Sta
     uses0 = s0 < s1;
   }
   for (int f = tid; f <= n; f += blockDim.x) {
-    const df M = df_mul(gd, df_ld2(T.mx2, ((size_t)k * T.nlat + j) * nf + f));
-    Mh[bck(T, f, mixed_frows(n))] = M.h;
-    Ml[bck(T, f, mixed_frows(n))] = M.l;
+    const df M = df_ldp(T.mx12, ((size_t)k * T.nlat + j) * nf + f);
+    Mh[bck(T, f, mixed_frows(n))] = M.h.v;
+    Ml[bck(T, f, mixed_frows(n))] = M.l.v;
   }
   for (int s = s0; s < s1; ++s) {
     const int it = s - s0, b = kTma ? (it & 1) : 0;
@@ -859,30 +969,41 @@ __global__ void __launch_bounds__(256) k_adv_x_mixed(DevTransport<double> T, Sta
     }
     for (int p = tid - 3; p <= n + 1; p += blockDim.x) {
       const df d = df_sub(df_ld(H, Lo, X(p + 1)), df_ld(H, Lo, X(p)));
-      Dh[X(p)] = d.h;
-      Dl[X(p)] = d.l;
+      Dh[X(p)] = d.h.v;
+      Dl[X(p)] = d.l.v;
     }
     __syncthreads();
     for (int p = tid - 2; p <= n + 1; p += blockDim.x) {
-      const df sl = mc_slope(df_ld(Dh, Dl, X(p - 1)), df_ld(Dh, Dl, X(p)));
-      Sh[X(p)] = sl.h;
-      Sl[X(p)] = sl.l;
+      const df d0 = df_ld(Dh, Dl, X(p - 1)), d1 = df_ld(Dh, Dl, X(p));
+      const df sl = slope2(d0, d1, df_add(d0, d1), live(d0, d1, 4.0f));
+      Sh[X(p)] = sl.h.v;
+      Sl[X(p)] = sl.l.v;
     }
     __syncthreads();
     for (int p = tid - 2; p <= n; p += blockDim.x) {  // edge terms over the staged values
-      const df e = edge_u(df_ld(Dh, Dl, X(p)), df_ld(Sh, Sl, X(p)), df_ld(Sh, Sl, X(p + 1)));
-      H[X(p)] = e.h;
-      Lo[X(p)] = e.l;
+      df t, e, lnext;
+      edges_u(df_ld(Dh, Dl, X(p)), df_ld(Sh, Sl, X(p)), df_ld(Sh, Sl, X(p + 1)), t, e, lnext);
+      H[X(p)] = e.h.v;
+      Lo[X(p)] = e.l.v;
     }
     __syncthreads();
+    auto face = [&](int f, df& A, df& B) {
+      const bool right = upwind_lo(Mh[bck(T, f, nf)], gs);
+      const int up = right ? f - 1 : f;
+      const df Dm = df_ld(Dh, Dl, X(up - 1)), Er = df_ld(H, Lo, X(up));
+      df t, e, l;
+      edges_u(Dm, df_ld(Sh, Sl, X(up - 1)), df_ld(Sh, Sl, X(up)), t, e, l);
+      const df x = limit(right ? Er : l, right ? l : Er, live(Dm, df_ld(Dh, Dl, X(up)), 2.0f));
+      face_terms(x, rest_u(times6(df_ld(Dh, Dl, X(f - 1))), x), right, A, B);
+    };
     for (int p = tid; p < n; p += blockDim.x) {
-      df psi, phi;
-      cell_faces(df{Mh[bck(T, p, nf)], Ml[bck(T, p, nf)]},
-                 df{Mh[bck(T, p + 1, nf)], Ml[bck(T, p + 1, nf)]},
-                 [&](int o) { return df_ld(H, Lo, X(p + o)); },
-                 [&](int o) { return df_ld(Dh, Dl, X(p + o)); }, psi, phi);
-      const df a = df_neg(df_mul(G, df_add(phi, psi)));
-      T.acc[bck(T, pb + p, nall)] = make_float2(a.h, a.l);
+      df A, B, o;
+      face(p, o, B);
+      face(p + 1, A, o);
+      const df a = fma_raw(mkdf(Mh[bck(T, p + 1, nf)], Ml[bck(T, p + 1, nf)]), A,
+                           mul_raw(mkdf(Mh[bck(T, p, nf)], Ml[bck(T, p, nf)]), B));
+      T.acc.h[bck(T, pb + p, nall)] = a.h.v;
+      T.acc.l[bck(T, pb + p, nall)] = a.l.v;
     }
     __syncthreads();
   }
@@ -899,7 +1020,7 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
   const double* Q;
   double g;
   if (!resolve_stage(sel, Q, g)) return;
-  const df gd = split_df(g);  // the stage time factor as a pair
+  const int gs = __double2hiint(g);  // only its sign is needed here
   const int s0 = blockIdx.y * sper, s1 = min(T.ntr, s0 + sper);  // this block's tracers
   extern __shared__ __align__(16) unsigned char smp32_raw[];
   float* smp32 = align128(smp32_raw);
@@ -914,8 +1035,10 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
   float* const Dl = Dh + R;
   float* const Sh = Dl + R;
   float* const Sl = Sh + R;
-  float* const Mh = Sl + R;  // [n+1][kPencil]
-  float* const Ml = Mh + (n + 1) * kPencil;
+  // the fluxes as the cell below the face sees them, [n+1][kPencil] (those of the cell above a lat
+  // face come from the cache: staging them too would shrink the largest grid that fits)
+  float* const Nh = Sl + R;
+  float* const Nl = Nh + (n + 1) * kPencil;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const bool lead = tx == 0 && ty == 0;
   const size_t ncol = (size_t)T.nlon * T.nlat;
@@ -929,7 +1052,7 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
   const size_t col0 = DIR == 2 ? (size_t)blockIdx.x * kPencil : 0;
   const int i = i0 + tx;
   const size_t col = col0 + tx;
-  const bool live = DIR == 1 ? i < T.nlon : col < ncol;
+  const bool inside = DIR == 1 ? i < T.nlon : col < ncol;
   const size_t stride = DIR == 1 ? (size_t)T.nlon : ncol;  // cell p to p+1
   const size_t cbase = DIR == 1 ? (size_t)k * ncol + i : col;  // cell 0 of the pencil
   const bool open = DIR == 1 && T.lat_bc == 1;
@@ -960,17 +1083,18 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
     uses0 = s0 < s1;
   }
 #define RS_P(a, p) a[bck(T, ((p) + kHoP) * kPencil + tx, R)]
-  if (live)
+  if (inside)
     for (int f = ty; f <= n; f += blockDim.y) {
-      df M{0.0f, 0.0f};
-      if (DIR == 1) {
-        if (open || (f > 0 && f < n))  // closed walls: no flux through the poles
-          M = df_mul(gd, df_ld2(T.my2, ((size_t)k * (n + 1) + f) * T.nlon + i));
-      } else if (f > 0 && f < n) {  // no flux through the surface and the model top
-        M = df_mul(gd, df_ld2(T.mz2, (size_t)f * ncol + col));
+      const long long m = bck(T, f * kPencil + tx, mb);
+      if (DIR == 1) {  // zero through closed walls
+        const size_t x = ((size_t)k * (n + 1) + f) * T.nlon + i;
+        Nh[m] = T.myn12.h[x];
+        Nl[m] = T.myn12.l[x];
+      } else {  // no flux through the surface and the model top
+        const bool in = f > 0 && f < n;
+        Nh[m] = in ? T.mz2.h[(size_t)f * ncol + col] : 0.0f;
+        Nl[m] = in ? T.mz2.l[(size_t)f * ncol + col] : 0.0f;
       }
-      Mh[bck(T, f * kPencil + tx, mb)] = M.h;
-      Ml[bck(T, f * kPencil + tx, mb)] = M.l;
     }
   for (int s = s0; s < s1; ++s) {
     const int it = s - s0, b = kTma ? (it & 1) : 0;
@@ -980,7 +1104,7 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
     auto cell = [&](int p, float& h, float& l) {  // a ghost (p outside 0..n-1) or interior cell
       h = 0.0f;
       l = 0.0f;
-      if (!live) return;
+      if (!inside) return;
       if (p < 0 || p >= n) {
         if (open) {
           split_d((p < 0 ? T.qs : T.qn)[bck(T, ((size_t)s * T.nlev + k) * T.nlon + i,
@@ -1020,246 +1144,336 @@ __global__ void __launch_bounds__(512) k_adv_yz_mixed(DevTransport<double> T, St
       __syncthreads();
     }
     for (int p = (int)ty - 3; p <= n + 1; p += blockDim.y) {
-      const df d = df_sub(df{RS_P(H, p + 1), RS_P(Lo, p + 1)}, df{RS_P(H, p), RS_P(Lo, p)});
-      RS_P(Dh, p) = d.h;
-      RS_P(Dl, p) = d.l;
+      const df d = df_sub(mkdf(RS_P(H, p + 1), RS_P(Lo, p + 1)), mkdf(RS_P(H, p), RS_P(Lo, p)));
+      RS_P(Dh, p) = d.h.v;
+      RS_P(Dl, p) = d.l.v;
     }
     __syncthreads();
+#define RS_PP(a, b, p) mkdf(RS_P(a, p), RS_P(b, p))
     for (int p = (int)ty - 2; p <= n + 1; p += blockDim.y) {
-      const df d0{RS_P(Dh, p - 1), RS_P(Dl, p - 1)}, d1{RS_P(Dh, p), RS_P(Dl, p)};
-      df sl{0.0f, 0.0f};
+      const df d0 = RS_PP(Dh, Dl, p - 1), d1 = RS_PP(Dh, Dl, p);
+      df sl = mkdf(0.0f, 0.0f);
       if (DIR == 1) {
-        sl = mc_slope(d0, d1);
-      } else if (p >= -1 && p <= n && live) {  // slopes of cells -1..n (coefficient row p+1)
+        sl = slope2(d0, d1, df_add(d0, d1), live(d0, d1, 4.0f));
+      } else if (p >= -1 && p <= n && inside) {  // slopes of cells -1..n (coefficient row p+1)
         const size_t x = bck(T, (size_t)(p + 1) * ncol + col, (long long)(n + 2) * ncol);
-        sl = mc_slope_n(d0, d1, df_ld2(T.vsA2, x), df_ld2(T.vsB2, x));
+        sl = slope2(d0, d1, centre_n(d0, d1, df_ldp(T.vsA2, x), df_ldp(T.vsB2, x)), live(d0, d1, 4.0f));
       }
-      RS_P(Sh, p) = sl.h;
-      RS_P(Sl, p) = sl.l;
+      RS_P(Sh, p) = sl.h.v;
+      RS_P(Sl, p) = sl.l.v;
     }
     __syncthreads();
     // edge terms over the staged values: cells -2..n (uniform), -1..n-1 (coefficient rows
     // 0..n of the dp-weighted edges)
     for (int p = (int)ty - 2; p <= n; p += blockDim.y) {
-      const df Dp{RS_P(Dh, p), RS_P(Dl, p)};
-      const df Sp{RS_P(Sh, p), RS_P(Sl, p)}, Sp1{RS_P(Sh, p + 1), RS_P(Sl, p + 1)};
-      df e{0.0f, 0.0f};
+      const df Dp = RS_PP(Dh, Dl, p), Sp = RS_PP(Sh, Sl, p), Sp1 = RS_PP(Sh, Sl, p + 1);
+      df e = mkdf(0.0f, 0.0f), l, t;
       if (DIR == 1) {
-        e = edge_u(Dp, Sp, Sp1);
-      } else if (p >= -1 && p <= n - 1 && live) {
+        edges_u(Dp, Sp, Sp1, t, e, l);
+      } else if (p >= -1 && p <= n - 1 && inside) {
         const size_t x = bck(T, (size_t)(p + 1) * ncol + col, (long long)(n + 1) * ncol);
-        e = edge_n(Dp, Sp, Sp1, df_ld2(T.veAB2, x), df_ld2(T.veC2, x), df_ld2(T.veD2, x));
+        e = edge_n(Dp, Sp, Sp1, df_ldp(T.veAB2, x), df_ldp(T.veC2, x), df_ldp(T.veD2, x));
       }
-      RS_P(H, p) = e.h;
-      RS_P(Lo, p) = e.l;
+      RS_P(H, p) = e.h.v;
+      RS_P(Lo, p) = e.l.v;
     }
     __syncthreads();
-    if (live) {
+    auto face = [&](int f, df& A, df& B) {
+      A = B = mkdf(0.0f, 0.0f);
+      if (DIR == 2 && (f == 0 || f == n)) return;
+      const bool right = upwind_lo(Nh[bck(T, f * kPencil + tx, mb)], gs);
+      const int up = right ? f - 1 : f;
+      const df Dm = RS_PP(Dh, Dl, up - 1), D = RS_PP(Dh, Dl, f - 1), Er = RS_PP(H, Lo, up);
+      df t, e, l, x, y;
+      if (DIR == 1) {
+        edges_u(Dm, RS_PP(Sh, Sl, up - 1), RS_PP(Sh, Sl, up), t, e, l);
+        x = limit(right ? Er : l, right ? l : Er, live(Dm, RS_PP(Dh, Dl, up), 2.0f));
+        y = rest_u(times6(D), x);
+      } else {
+        l = df_sub(Dm, RS_PP(H, Lo, up - 1));
+        x = limit(right ? Er : l, right ? l : Er, live(l, Er, 2.0f));
+        y = sub_raw(D, x);
+      }
+      face_terms(x, y, right, A, B);
+    };
+    if (inside) {
       for (int p = ty; p < n; p += blockDim.y) {
-        df psi, phi;
-        cell_faces(df{Mh[bck(T, p * kPencil + tx, mb)], Ml[bck(T, p * kPencil + tx, mb)]},
-                   df{Mh[bck(T, (p + 1) * kPencil + tx, mb)], Ml[bck(T, (p + 1) * kPencil + tx, mb)]},
-                   [&](int o) { return df{RS_P(H, p + o), RS_P(Lo, p + o)}; },
-                   [&](int o) { return df{RS_P(Dh, p + o), RS_P(Dl, p + o)}; }, psi, phi);
-        df a;
-        if (DIR == 1)
-          a = df_neg(df_add(df_mul(df_ld2(T.gyhi2, p), phi), df_mul(df_ld2(T.gylo2, p), psi)));
-        else
-          a = df_neg(df_add(phi, psi));
+        df A, B, o;
+        face(p, o, B);
+        face(p + 1, A, o);
         const size_t x = bck(T, pb + (size_t)p * stride, nall);
-        const float2 o = T.acc[x];
-        const df t = df_add(df{o.x, o.y}, a);
-        T.acc[x] = make_float2(t.h, t.l);
+        const long long ms = bck(T, p * kPencil + tx, mb), mn = bck(T, (p + 1) * kPencil + tx, mb);
+        const df Ms = DIR == 1 ? df_ldp(T.mys12, ((size_t)k * (n + 1) + p) * T.nlon + i) : mkdf(Nh[ms], Nl[ms]);
+        const df t = fma_raw(mkdf(Nh[mn], Nl[mn]), A, fma_raw(Ms, B, mkdf(T.acc.h[x], T.acc.l[x])));
+        T.acc.h[x] = t.h.v;
+        T.acc.l[x] = t.l.v;
       }
     }
     __syncthreads();
   }
+#undef RS_PP
 #undef RS_P
 }
 
 // ---- streaming forms of the mixed pencils (no shared memory, no barriers).  The same pair
 // operations in the same order as k_adv_x_mixed / k_adv_yz_mixed, so the accumulators are bit
-// for bit those of the pencils; rs_autotune picks per direction.
-//
-// Lon rows: one warp per segment of kSegX = 26 cells of a row; lane l holds cell
-// p = base - 3 + l, and the neighbour values the stencil needs move between lanes by shuffles.
-// Lane l computes the limited deviation of face p (its west face); cells at lanes 3..28 have
-// all of D(p-2..p), E(p-2..p+1) and their east face's Phi from lane l+1.
-constexpr int kSegX = 26;
-__device__ __forceinline__ df shfl_up_df(df v, int d) {
-  return {__shfl_up_sync(0xffffffffu, v.h, d), __shfl_up_sync(0xffffffffu, v.l, d)};
-}
-__device__ __forceinline__ df shfl_down_df(df v, int d) {
-  return {__shfl_down_sync(0xffffffffu, v.h, d), __shfl_down_sync(0xffffffffu, v.l, d)};
-}
-// Face f's two pair terms from the upwind cell's edges: Psi_f (for cell f) and Phi_f (for cell
-// f-1).  E(o), D(o) give E_{f+o}, D_{f+o}.  The expressions of cell_faces, so the same bits.
-template <class FE, class FD>
-__device__ __forceinline__ void face_terms(df M, FE E, FD D, df& psi, df& phi) {
-  psi = df{0.0f, 0.0f};
-  phi = df{0.0f, 0.0f};
-  if (M.h > 0.0f) {  // upwind f-1: its right edge
-    const df dev = lim_pick(df_sub(E(-2), D(-2)), E(-1), true);
-    psi = df_mul(M, df_sub(D(-1), dev));
-    phi = df_mul(M, dev);
-  } else if (M.h < 0.0f) {  // upwind f: its left edge
-    const df dev = lim_pick(df_sub(E(-1), D(-1)), E(0), false);
-    psi = df_mul(M, df_neg(dev));
-    phi = df_mul(M, df_add(D(-1), dev));
+// for bit those of the pencils; rs_autotune picks per direction.  N tracers side by side in the
+// halves of packed operations (an odd last tracer runs beside a copy of itself that is not
+// stored).
+template <int N>
+struct Tracers {  // this block's tracers s .. s + N - 1, of which the second may not count
+  size_t off[N];
+  bool two;
+  __device__ __forceinline__ Tracers(int s, int s1, size_t nc) : two(N == 2 && s + 1 < s1) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) off[i] = (size_t)min(s + i, s1 - 1) * nc;
   }
+  // the plane offsets are the same for the whole block, the cell's is 32 bits: addresses then cost
+  // no 64-bit arithmetic per thread
+  __device__ __forceinline__ DF<N> load(const float* H, const float* L, unsigned x) const {
+    if constexpr (N == 1) return {{(H + off[0])[x]}, {(L + off[0])[x]}};
+    else return {{pack2((H + off[0])[x], (H + off[1])[x])}, {pack2((L + off[0])[x], (L + off[1])[x])}};
+  }
+  __device__ __forceinline__ void store(float* H, float* L, unsigned x, const DF<N>& v) const {
+    (H + off[0])[x] = half(v.h, 0);
+    (L + off[0])[x] = half(v.l, 0);
+    if constexpr (N == 2)
+      if (two) {
+        (H + off[1])[x] = half(v.h, 1);
+        (L + off[1])[x] = half(v.l, 1);
+      }
+  }
+};
+// an open wall's ghost: the prescribed boundary values of the thread's tracers
+template <int N>
+__device__ __forceinline__ DF<N> ghost_df(const DevTransport<double>& T, const double* b, int s, int s1,
+                                          size_t plane, size_t x, long long n) {
+  float h[2], l[2];
+#pragma unroll
+  for (int i = 0; i < N; ++i) split_d(b[bck(T, (size_t)min(s + i, s1 - 1) * plane + x, n)], h[i], l[i]);
+  if constexpr (N == 1) return {{h[0]}, {l[0]}};
+  else return {{pack2(h[0], h[1])}, {pack2(l[0], l[1])}};
 }
 
+// Lon rows: one warp per segment of kSegX = 26 cells of a row; lane l holds cell
+// p = base - 3 + l, and the neighbour values the stencil needs move between lanes by shuffles.
+// Each lane limits both edges of its own cell, so that its west face takes the neighbour's right
+// deviation or its own left one; cells at lanes 3..28 have their east face's A from lane l+1.
+constexpr int kSegX = 26;
+template <int N>
+__device__ __forceinline__ FV<N> shfl_up_v(FV<N> v, int d) {
+  if constexpr (N == 1) return {__shfl_up_sync(0xffffffffu, v.v, d)};
+  else return {pack2(__shfl_up_sync(0xffffffffu, half(v, 0), d), __shfl_up_sync(0xffffffffu, half(v, 1), d))};
+}
+template <int N>
+__device__ __forceinline__ FV<N> shfl_down_v(FV<N> v, int d) {
+  if constexpr (N == 1) return {__shfl_down_sync(0xffffffffu, v.v, d)};
+  else return {pack2(__shfl_down_sync(0xffffffffu, half(v, 0), d), __shfl_down_sync(0xffffffffu, half(v, 1), d))};
+}
+template <int N>
+__device__ __forceinline__ DF<N> shfl_up_df(DF<N> v, int d) { return {shfl_up_v(v.h, d), shfl_up_v(v.l, d)}; }
+template <int N>
+__device__ __forceinline__ DF<N> shfl_down_df(DF<N> v, int d) { return {shfl_down_v(v.h, d), shfl_down_v(v.l, d)}; }
+
+template <int N>
 __global__ void __launch_bounds__(128) k_adv_x_stream(DevTransport<double> T, StageSel sel,
                                                       int sper) {
   const double* Q;
   double g;
   if (!resolve_stage(sel, Q, g)) return;
-  const df gd = split_df(g);  // the stage time factor as a pair
+  const int gs = __double2hiint(g);  // only its sign is needed here
   const int n = T.nlon, nf = n + 1;
   const int nseg = (n + kSegX - 1) / kSegX;
   const int lane = threadIdx.x & 31;
-  const long long wg = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int ngrp = (T.ntr + sper - 1) / sper;  // the tracer groups are the fastest grid dimension
+  const long long wg = (long long)(blockIdx.x / ngrp) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wg >= (long long)nseg * T.nlat * T.nlev) return;  // whole warps leave together
   const int row = (int)(wg / nseg), seg = (int)(wg % nseg);
-  const int j = row % T.nlat, k = row / T.nlat;
   const int p = seg * kSegX - 3 + lane;  // this lane's cell (and west face)
   const size_t nc = (size_t)T.nlon * T.nlat * T.nlev;
-  const long long nall = (long long)T.ntr * nc;
-  const size_t rbase = ((size_t)k * T.nlat + j) * n;
+  const size_t rbase = (size_t)row * n;
   const bool periodic = T.lon_bc == 0;
-  const df G = df_ld2(T.gx2, j);
-  const df M = (p >= 0 && p <= n) ? df_mul(gd, df_ld2(T.mx2, ((size_t)k * T.nlat + j) * nf + p))
-                                   : df{0.0f, 0.0f};
+  const df M1 = (p >= 0 && p <= n) ? df_ldp(T.mx12, (size_t)row * nf + p) : mkdf(0.0f, 0.0f);
+  const bool right = upwind_lo(M1.h.v, gs);
+  const DF<N> Mw = splat_df<N>(M1.h.v, M1.l.v);
+  const df E1 = shfl_down_df(M1, 1);
+  const DF<N> Me = splat_df<N>(E1.h.v, E1.l.v);
   const bool out = lane >= 3 && lane <= 28 && p >= 0 && p < n;
-  const int s0 = blockIdx.y * sper, s1 = min(T.ntr, s0 + sper);
-  for (int s = s0; s < s1; ++s) {
-    const size_t pb = (size_t)s * nc + rbase;
-    df q;
-    if (p >= 0 && p < n) {
-      q = df{T.qhi[bck(T, pb + p, nall)], T.qlo[bck(T, pb + p, nall)]};
-    } else if (periodic) {
-      const int w = ((p % n) + n) % n;
-      q = df{T.qhi[bck(T, pb + w, nall)], T.qlo[bck(T, pb + w, nall)]};
-    } else {
-      split_d((p < 0 ? T.qw : T.qe)[bck(T, ((size_t)s * T.nlev + k) * T.nlat + j,
-                                        (long long)T.ntr * T.nlev * T.nlat)], q.h, q.l);
-    }
-    const df D = df_sub(shfl_down_df(q, 1), q);                 // D(p), lanes 0..30
-    const df S = mc_slope(shfl_up_df(D, 1), D);                 // S(p), lanes 1..30
-    const df E = edge_u(D, S, shfl_down_df(S, 1));              // E(p), lanes 1..29
-    const df Dm1 = shfl_up_df(D, 1), Dm2 = shfl_up_df(D, 2);
-    const df Em1 = shfl_up_df(E, 1), Em2 = shfl_up_df(E, 2);
-    df psi, phi;
-    face_terms(M, [&](int o) { return o == 0 ? E : (o == -1 ? Em1 : Em2); },
-               [&](int o) { return o == -1 ? Dm1 : Dm2; }, psi, phi);
-    const df phie = shfl_down_df(phi, 1);  // the east face's Phi, computed by lane + 1
-    if (out) {
-      const df a = df_neg(df_mul(G, df_add(phie, psi)));
-      T.acc[bck(T, pb + p, nall)] = make_float2(a.h, a.l);
-    }
+  const int pw = periodic ? ((p % n) + n) % n : p;
+  const int s0 = (int)(blockIdx.x % ngrp) * sper, s1 = min(T.ntr, s0 + sper);
+  for (int s = s0; s < s1; s += N) {
+    const Tracers<N> tr(s, s1, nc);
+    DF<N> q;
+    if (pw >= 0 && pw < n) q = tr.load(T.qhi, T.qlo, (unsigned)(rbase + bck(T, pw, n)));
+    else q = ghost_df<N>(T, p < 0 ? T.qw : T.qe, s, s1, (size_t)T.nlev * T.nlat, row, (long long)T.ntr * T.nlev * T.nlat);
+    const DF<N> D = df_sub(shfl_down_df(q, 1), q);              // D(p), lanes 0..30
+    const DF<N> Dm = shfl_up_df(D, 1);                          // D(p-1)
+    const FV<N> k4 = live(Dm, D, 4.0f);
+    const DF<N> S = slope2(Dm, D, df_add(Dm, D), k4);           // lanes 1..30
+    DF<N> t, E, Ln;
+    edges_u(D, S, shfl_down_df(S, 1), t, E, Ln);                // E(p), L(p+1), lanes 1..29
+    const DF<N> L = shfl_up_df(Ln, 1), tm = shfl_up_df(t, 1);   // lanes 2..30
+    const FV<N> k2 = vmul(k4, splat<N>(0.5f));
+    const DF<N> xRm = shfl_up_df(limit(E, L, k2), 1);           // of cell p-1, lanes 3..30
+    const DF<N> x = right ? xRm : limit(L, E, k2);
+    DF<N> A, B;
+    face_terms(x, rest_u(tm, x), right, A, B);
+    const DF<N> Ae = shfl_down_df(A, 1);  // the east face's A, formed by lane + 1
+    if (out) tr.store(T.acc.h, T.acc.l, (unsigned)(rbase + p), fma_raw(Me, Ae, mul_raw(Mw, B)));
   }
 }
 
-// Lat (DIR 1) and vertical (DIR 2) lines: one thread per line (consecutive lon points at one
-// level, or consecutive columns), walking the line once per tracer with a register window:
-// when q(p) arrives, D(p-1), S(p-1), E(p-2) are formed and face p-2 is complete; its Phi
-// closes cell p-3 and its Psi opens cell p-2.
-template <int DIR>
-__global__ void __launch_bounds__(128) k_adv_yz_stream(DevTransport<double> T, StageSel sel,
-                                                       int sper) {
+// Lat (DIR 1) and vertical (DIR 2) lines: one thread per line (consecutive lon points over all
+// levels, or consecutive columns), walking the line once per N tracers with a register window:
+// when q(p) arrives, D(p-1), S(p-1), E(p-2), L(p-1) are formed and face p-2 is complete; its A
+// closes cell p-3 and its B opens cell p-2.  The tracer groups are the fastest grid dimension:
+// the fluxes and coefficients of a set of lines are read from DRAM once and come from L2 for the
+// other groups.
+constexpr int kLine32 = 64;  // threads per block of the line kernels
+// Blocks per SM (168 registers) and iterations that a line's loads run ahead.  Both directions
+// together, 360x181x72 / 144x91x47: 6 x 4 1.84 ms / 145 us, 6 x 3 1.81 / 143, 6 x 2 1.86 / 141,
+// 8 x 2 (128 registers, spilling) 1.75 / 145, no bound and 4 ahead (192-220 registers, a second wave
+// of a few blocks) 2.13 / 176.
+constexpr int kLineBlocks = 6;
+constexpr int kAhead = 3;
+template <int DIR, int N>
+__global__ void __launch_bounds__(kLine32, kLineBlocks) k_adv_yz_stream(DevTransport<double> T, StageSel sel,
+                                                           int sper) {
   const double* Q;
   double g;
   if (!resolve_stage(sel, Q, g)) return;
-  const df gd = split_df(g);  // the stage time factor as a pair
+  const int gs = __double2hiint(g);  // only its sign is needed here
   const int n = DIR == 1 ? T.nlat : T.nlev;
-  const size_t ncol = (size_t)T.nlon * T.nlat;
-  const size_t nc = ncol * T.nlev;
-  const long long nall = (long long)T.ntr * nc;
-  const int ntile = (T.nlon + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int k = DIR == 1 ? (int)(blockIdx.x / ntile) : 0;
-  const int i = DIR == 1 ? (int)(blockIdx.x % ntile) * (int)blockDim.x + (int)threadIdx.x : 0;
-  const size_t col = DIR == 2 ? (size_t)blockIdx.x * blockDim.x + threadIdx.x : 0;
-  if (DIR == 1 ? i >= T.nlon : col >= ncol) return;
-  const size_t stride = DIR == 1 ? (size_t)T.nlon : ncol;
-  const size_t cbase = DIR == 1 ? (size_t)k * ncol + i : col;
+  const unsigned ncol = (unsigned)(T.nlon * T.nlat);
+  const size_t nc = (size_t)ncol * T.nlev;
+  const unsigned ngrp = (unsigned)((T.ntr + sper - 1) / sper);
+  const unsigned id = blockIdx.x / ngrp * blockDim.x + threadIdx.x;
+  if (id >= (DIR == 1 ? (unsigned)(T.nlon * T.nlev) : ncol)) return;
+  const unsigned k = DIR == 1 ? id / T.nlon : 0, i = DIR == 1 ? id % T.nlon : 0;
+  const unsigned stride = DIR == 1 ? (unsigned)T.nlon : ncol;
+  const unsigned cbase = DIR == 1 ? k * ncol + i : id;
+  const unsigned fb = DIR == 1 ? k * (unsigned)(n + 1) * T.nlon + i : id;  // face 0 of the line
   const bool open = DIR == 1 && T.lat_bc == 1;
-  auto flux = [&](int f) -> df {  // face f's air-mass flux, zero through closed walls
-    if (DIR == 1) {
-      if (open || (f > 0 && f < n)) return df_mul(gd, df_ld2(T.my2, ((size_t)k * (n + 1) + f) * T.nlon + i));
-    } else if (f > 0 && f < n) {
-      return df_mul(gd, df_ld2(T.mz2, (size_t)f * ncol + col));
-    }
-    return df{0.0f, 0.0f};
-  };
-  const int s0 = blockIdx.y * sper, s1 = min(T.ntr, s0 + sper);
-  for (int s = s0; s < s1; ++s) {
-    const size_t pb = (size_t)s * nc + cbase;
-    auto load = [&](int p) -> df {
-      if (p < 0 || p >= n) {
-        if (open) {
-          df v;
-          split_d((p < 0 ? T.qs : T.qn)[bck(T, ((size_t)s * T.nlev + k) * T.nlon + i,
-                                            (long long)T.ntr * T.nlev * T.nlon)], v.h, v.l);
-          return v;
-        }
+  const int s0 = (int)(blockIdx.x % ngrp) * sper, s1 = min(T.ntr, s0 + sper);
+  for (int s = s0; s < s1; s += N) {
+    const Tracers<N> tr(s, s1, nc);
+    auto cell = [&](int p) { return cbase + (unsigned)bck(T, p, n) * stride; };
+    auto value = [&](int p, bool edge) -> DF<N> {
+      if (edge && (p < 0 || p >= n)) {
+        if (open)
+          return ghost_df<N>(T, p < 0 ? T.qs : T.qn, s, s1, (size_t)T.nlev * T.nlon, (size_t)k * T.nlon + i,
+                             (long long)T.ntr * T.nlev * T.nlon);
         p = p < 0 ? -1 - p : 2 * n - 1 - p;  // mirror ghosts at the walls
       }
-      const size_t x = bck(T, pb + (size_t)p * stride, nall);
-      return df{T.qhi[x], T.qlo[x]};
+      return tr.load(T.qhi, T.qlo, cell(p));
     };
-    const df z{0.0f, 0.0f};
-    // window: qp = q(p-1); D4..D1 = D(p-4..p-1); S2, S1 = S(p-2), S(p-1); E4..E2 = E(p-4..p-2)
-    df qp = load(-3), D4 = z, D3 = z, D2 = z, D1 = z, S2 = z, S1 = z, E4 = z, E3 = z, E2 = z;
-    df psi_prev = z;  // Psi of the previous face (the open cell's west face)
-    // one iteration ahead: q(p), the flux of face p-2 and the accumulator of cell p-3
-    df q_nx = load(-2), m_nx = z;
-    float2 a_nx = make_float2(0.0f, 0.0f);
-    for (int p = -2; p <= n + 2; ++p) {
-      const df qn = q_nx, Mf = m_nx;
-      const float2 o = a_nx;
-      if (p < n + 2) q_nx = load(p + 1);
-      if (p - 1 >= 0 && p - 1 <= n) m_nx = flux(p - 1);
-      if (p - 2 >= 0 && p - 2 < n) a_nx = T.acc[bck(T, pb + (size_t)(p - 2) * stride, nall)];
-      D4 = D3; D3 = D2; D2 = D1;
-      D1 = df_sub(qn, qp);  // D(p-1)
-      qp = qn;
-      S2 = S1;
-      const int ps = p - 1;  // the slope formed now
+    const DF<N> z = splat_df<N>(0.0f, 0.0f);
+    const FV<N> z1 = splat<N>(0.0f);
+    // what iteration p reads: q(p), face p-2's fluxes, the accumulator of the cell above that face,
+    // the coefficients of slope p-1 and edge p-2.  kAhead iterations are in flight.
+    struct In {
+      DF<N> q, a;
+      df mn, ms, sA, sB, ab, c, d;
+    };
+    auto fetch = [&](int p, bool edge, In& in) {
+      const int f = p - 2;
+      if (!edge || p <= n + 2) in.q = value(p, edge);
+      if (!edge || (f >= 0 && f <= n)) {
+        const unsigned x = fb + (unsigned)f * stride;
+        if (DIR == 1) {
+          in.mn = df_ldp(T.myn12, x);
+          in.ms = df_ldp(T.mys12, x);
+        } else {
+          in.mn = !edge || (f > 0 && f < n) ? df_ldp(T.mz2, x) : mkdf(0.0f, 0.0f);
+        }
+        if (!edge || f < n) in.a = tr.load(T.acc.h, T.acc.l, cell(f));
+      }
+      if (DIR == 2) {
+        if (!edge || (p >= 0 && p <= n + 1)) {  // slopes of cells -1..n (coefficient row of cell + 1)
+          const unsigned x = (unsigned)bck(T, p, n + 2) * ncol + id;
+          in.sA = df_ldp(T.vsA2, x);
+          in.sB = df_ldp(T.vsB2, x);
+        }
+        if (!edge || (f >= -1 && f <= n - 1)) {  // right edges of cells -1..n-1 (row f+1)
+          const unsigned x = (unsigned)bck(T, f + 1, n + 1) * ncol + id;
+          in.ab = df_ldp(T.veAB2, x);
+          in.c = df_ldp(T.veC2, x);
+          in.d = df_ldp(T.veD2, x);
+        }
+      }
+    };
+    auto both = [](df v) { return splat_df<N>(v.h.v, v.l.v); };
+    // window: qp = q(p-1); D3, D2 = D(p-3), D(p-2), t3, t2 = 6 D; S1 = S(p-1); E3, E2 = E(p-3),
+    // E(p-2); L3, L2, L1 and k3, k2, k1 (live) of cells p-3, p-2, p-1; ac the open cell's
+    // accumulator
+    DF<N> qp = value(-2, true), D3 = z, D2 = df_sub(qp, value(-3, true)), t3 = z, t2 = z, S1 = z;
+    DF<N> E3 = z, E2 = z, L3 = z, L2 = z, L1 = z, ac = z;
+    FV<N> k3 = z1, k2 = z1, k1 = z1;
+    auto step = [&](int p, bool edge, const In& in) {  // edge: near a wall, every range is checked
+      const int f = p - 2;
+      const DF<N> D1 = df_sub(in.q, qp);  // D(p-1)
+      qp = in.q;
+      const DF<N> S2 = S1;
+      E3 = E2;
+      L3 = L2;
+      k3 = k2;
       if (DIR == 1) {
-        S1 = mc_slope(D2, D1);
-      } else if (ps >= -1 && ps <= n) {  // slopes of cells -1..n (coefficient row ps+1)
-        const size_t x = bck(T, (size_t)(ps + 1) * ncol + col, (long long)(n + 2) * ncol);
-        S1 = mc_slope_n(D2, D1, df_ld2(T.vsA2, x), df_ld2(T.vsB2, x));
+        const FV<N> k4 = live(D2, D1, 4.0f);
+        S1 = slope2(D2, D1, df_add(D2, D1), k4);  // S(p-1)
+        t3 = t2;
+        L2 = L1;
+        k2 = k1;
+        k1 = vmul(k4, splat<N>(0.5f));
+        edges_u(D2, S2, S1, t2, E2, L1);
       } else {
-        S1 = z;
+        if (!edge || (p >= 0 && p <= n + 1))
+          S1 = slope2(D2, D1, centre_n(D2, D1, both(in.sA), both(in.sB)), live(D2, D1, 4.0f));
+        if (!edge || (f >= -1 && f <= n - 1)) {
+          E2 = edge_n(D2, S2, S1, both(in.ab), both(in.c), both(in.d));
+          L2 = df_sub(D3, E3);
+        }
       }
-      E4 = E3; E3 = E2;
-      const int pe = p - 2;  // the edge term formed now: E(pe) from D(pe), S(pe), S(pe+1)
-      if (DIR == 1) {
-        E2 = edge_u(D2, S2, S1);
-      } else if (pe >= -1 && pe <= n - 1) {
-        const size_t x = bck(T, (size_t)(pe + 1) * ncol + col, (long long)(n + 1) * ncol);
-        E2 = edge_n(D2, S2, S1, df_ld2(T.veAB2, x), df_ld2(T.veC2, x), df_ld2(T.veD2, x));
+      if (!edge || f >= 0) {  // the face now complete
+        DF<N> A = z, B = z;
+        if (DIR == 1 || !edge || (f > 0 && f < n)) {
+          const bool right = upwind_lo(in.mn.h.v, gs);
+          const DF<N> self = right ? E3 : L2, other = right ? L3 : E2;
+          DF<N> x, y;
+          if (DIR == 1) {
+            x = limit(self, other, right ? k3 : k2);
+            y = rest_u(t3, x);
+          } else {
+            x = limit(self, other, live(other, self, 2.0f));
+            y = sub_raw(D3, x);
+          }
+          face_terms(x, y, right, A, B);
+        }
+        if (!edge || f >= 1)  // cell f-1 is complete
+          tr.store(T.acc.h, T.acc.l, cell(f - 1), fma_raw(both(in.mn), A, ac));
+        ac = fma_raw(both(DIR == 1 ? in.ms : in.mn), B, in.a);
+      }
+      D3 = D2;
+      D2 = D1;
+    };
+    In buf[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) fetch(-1 + j, true, buf[j]);
+    for (int p = -1; p <= n + 2; p += kAhead) {
+      if (p >= 3 && p + 2 * kAhead <= n) {  // this group and the one it fetches are inside
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+          const In in = buf[j];
+          fetch(p + kAhead + j, false, buf[j]);
+          step(p + j, false, in);
+        }
       } else {
-        E2 = z;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+          const In in = buf[j];
+          fetch(p + kAhead + j, true, buf[j]);
+          if (p + j <= n + 2) step(p + j, true, in);
+        }
       }
-      const int f = p - 2;  // the face now complete (needs E(f-2..f), D(f-2..f-1))
-      if (f < 0 || f > n) continue;
-      df psi, phi;
-      face_terms(Mf, [&](int o) { return o == 0 ? E2 : (o == -1 ? E3 : E4); },
-                 [&](int o) { return o == -1 ? D3 : D4; }, psi, phi);
-      if (f >= 1) {  // cell f-1 is complete: its east face f, west face f-1
-        const int c = f - 1;
-        df a;
-        if (DIR == 1)
-          a = df_neg(df_add(df_mul(df_ld2(T.gyhi2, c), phi), df_mul(df_ld2(T.gylo2, c), psi_prev)));
-        else
-          a = df_neg(df_add(phi, psi_prev));
-        const size_t x = bck(T, pb + (size_t)c * stride, nall);
-        const df t = df_add(df{o.x, o.y}, a);
-        T.acc[x] = make_float2(t.h, t.l);
-      }
-      psi_prev = psi;
     }
   }
 }
@@ -1273,7 +1487,8 @@ __device__ __forceinline__ void split_bits(double v, float& hi, float& lo) {
   const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
   const int e = (int)((h >> 20) & 0x7ff);
   if (e < 949 || e > 1150) {
-    hi = (float)v;
+    // volatile: the compiler otherwise runs this branch's FP64 instructions on every value
+    asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(hi) : "d"(v));
     lo = (float)(v - (double)hi);
     return;
   }
@@ -1301,26 +1516,46 @@ __device__ __forceinline__ void split_store(const DevTransport<double>& T, size_
   T.qlo[x] = lo;
 }
 __device__ __forceinline__ df split_df(double v) {
-  df r;
+  float h, l;
 #if RS_STRICT
-  r.h = (float)v;
-  r.l = (float)(v - (double)r.h);
+  h = (float)v;
+  l = (float)(v - (double)h);
 #else
-  split_bits(v, r.h, r.l);
+  split_bits(v, h, l);
 #endif
-  return r;
+  return mkdf(h, l);
 }
 
-// (hi, lo) pairs of a double array (the air-mass face fluxes of the mixed kernels)
-__global__ void k_make_pairs(const double* __restrict__ src, float2* __restrict__ dst, size_t n) {
+// hi and lo planes of scale times a double array (the air-mass face fluxes of the mixed kernels)
+__global__ void k_make_pairs(const double* __restrict__ src, double scale, float* __restrict__ hi,
+                             float* __restrict__ lo, size_t n) {
   const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (x < n) {
-    const df v = split_df(src[x]);
-    dst[x] = make_float2(v.h, v.l);
+    const df v = split_df(src[x] * scale);
+    hi[x] = v.h.v;
+    lo[x] = v.l.v;
   }
 }
-void launch_make_pairs(cudaStream_t st, const double* src, float2* dst, size_t n) {
-  if (n) k_make_pairs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, dst, n);
+void launch_make_pairs(cudaStream_t st, const double* src, double scale, float* dst, size_t n) {
+  if (n) k_make_pairs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(src, scale, dst, dst + n, n);
+}
+
+// The air-mass fluxes with the cells' metric and the uniform edges' 1/6 folded in: mx6 (both
+// cells of a lon face share the row's factor), myn6 / mys6 (as the cell south / north of a lat face
+// sees it; zero through closed walls; the south-most open face has no cell south of it, its myn6
+// serves the upwind direction only).  Once per forcing change.
+__global__ void k_scale_fluxes(DevTransport<double> T, double* __restrict__ mx6,
+                               double* __restrict__ myn6, double* __restrict__ mys6) {
+  const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nx = (size_t)T.nlev * T.nlat * (T.nlon + 1), ny = (size_t)T.nlev * (T.nlat + 1) * T.nlon;
+  if (x < nx) mx6[x] = T.mx[x] * (T.gx[(x / (T.nlon + 1)) % T.nlat] * kOneSixth);
+  if (x < ny) {
+    const int f = (int)((x / T.nlon) % (T.nlat + 1));
+    const bool wall = T.lat_bc != 1 && (f == 0 || f == T.nlat);
+    const double m = T.my[x];
+    myn6[x] = wall ? 0.0 : m * ((f > 0 ? T.gyhi[f - 1] : T.gylo[0]) * kOneSixth);
+    mys6[x] = wall || f == T.nlat ? 0.0 : m * (T.gylo[f] * kOneSixth);
+  }
 }
 
 // split the attempt's input state U[cur] (stage 1's RHS argument) into hi/lo planes
@@ -1418,7 +1653,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pbl_mean(DevTransport<double> T
   if (T.mixed) {  // the stage input is the pencils' (hi, lo) planes
     for (int k = 0; k < T.nlev; ++k) {
       const size_t x = s * nc + (size_t)k * ncol + col;
-      acc = acc + T.pbl_w[(size_t)k * ncol + col] * df_to_d(make_float2(T.qhi[x], T.qlo[x]));
+      acc = acc + T.pbl_w[(size_t)k * ncol + col] * df_to_d(mkdf(T.qhi[x], T.qlo[x]));
     }
   } else {
     for (int k = 0; k < T.nlev; ++k) acc = acc + T.pbl_w[(size_t)k * ncol + col] * q[(size_t)k * ncol];
@@ -1445,7 +1680,7 @@ static void launch_pbl_mean(cudaStream_t st, const DevTransport<double>& T, cons
 // stage in 1..4.  Qin: the field whose fluxes were computed (RHS argument).
 //   1: S1 = U + dt/2 f(U)           2: S2 = S1 + dt/2 f(S1)
 //   3: S1 = u3 = S2 + dt/2 f(S2), S3 = u4 = 2/3 U + 1/3 u3
-//   4: unew = S3 + dt/2 f(S3); err = 1/2 (1/3 U + 2/3 u3 - unew); candidate = clamp(unew)
+//   4: unew = S3 + dt/2 f(S3); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
                                                        const Ctl* __restrict__ ctl,
@@ -1554,18 +1789,37 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
 #include "rs_adv64.cuh"
 
 // Compensated-FP32 stage kernel (mixed precision).  The tracers of stages 1-3 stay pairs:
-// the stage input is the pencils' own (hi, lo) planes, the update q + dt/2 * (m dq/dt) / m is
-// formed in pairs and written back into those planes (in place: the update is pointwise), u3
-// is kept as pairs in the tracer part of S1; only stage 4 returns to FP64 -- the candidate
-// state, the embedded error and the hairer norm, as the benchmark spec keeps them.  The air-mass
-// row is the FP64 scheme's, stage by stage (m in the air-mass planes of U, S1, S2, S3).
+// the stage input is the (hi, lo) planes, the update q + dt/2 * (m dq/dt) / m is formed in pairs
+// and written back into those planes (in place: the update is pointwise), u3 is kept as hi and lo
+// planes in the tracer part of S1; stage 4 returns to FP64 with the candidate state.  Its embedded
+// error and the hairer norm are formed in pairs as well (relative error ~1e-13 after the one
+// cancellation, which the pairs of the states carry anyway; the FP64 form's one-step reciprocal has
+// 1e-12): eight FP64 instructions per cell and tracer, 64 cycles each, had made this stage five
+// times as long as the others (144x91x47: 211 us against 41; 360x181x72 with 30 tracers 3.47 ms).
+// The air-mass row is the FP64 scheme's, stage by stage (m in the air-mass planes of U, S1, S2, S3).
 //   1: P = U + dt/2 f(U)          2: P = P + dt/2 f(P)
-//   3: u3 = P + dt/2 f(P) -> S1 (pairs), P = u4 = 2/3 U + 1/3 u3
-//   4: unew = P + dt/2 f(P); err = 1/2 (1/3 U + 2/3 u3 - unew); candidate = clamp(unew)
-constexpr float kTwoThirdsH = (float)(2.0 / 3.0);
-constexpr float kTwoThirdsL = (float)(2.0 / 3.0 - (double)(float)(2.0 / 3.0));
+//   3: u3 = P + dt/2 f(P) -> S1 (pairs), P = u4 = U + (u3 - U) / 3
+//   4: unew = P + dt/2 f(P); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 constexpr float kThirdH = (float)(1.0 / 3.0);
 constexpr float kThirdL = (float)(1.0 / 3.0 - (double)(float)(1.0 / 3.0));
+__device__ __forceinline__ df df_abs(df a) {  // of a normalised pair
+  const unsigned sg = __float_as_uint(a.h.v) & 0x80000000u;
+  return mkdf(fabsf(a.h.v), __uint_as_float(__float_as_uint(a.l.v) ^ sg));
+}
+// a / b: the quotient of the leading parts and one correction from the exact remainder
+__device__ __forceinline__ df df_div(df a, df b) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b.h.v));
+  const float q = __fmul_rn(a.h.v, r);
+  const float rem = __fmaf_rn(-q, b.l.v, __fadd_rn(__fmaf_rn(-q, b.h.v, a.h.v), a.l.v));
+  return df_renorm(df{{q}, {__fmul_rn(rem, r)}});
+}
+// one tracer's squared error ratio in FP64, for what is outside the pairs' range (and NaN).  A
+// call: inlined, its FP64 instructions ran (and were thrown away) on the ordinary path too.
+__device__ __noinline__ double error_fp64(float dh, float dl, double am, double rtol, double atol) {
+  const double at = df_to_d(mkdf(dh, dl)) * rcp_nr1(fma(am, rtol, atol));  // den >= atol > 0
+  return at * at;
+}
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double> T,
                                                              const Ctl* __restrict__ ctl,
@@ -1581,10 +1835,14 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
   // air mass of the stage input
   const double* Qm = STAGE == 1 ? U : (STAGE == 2 ? B.S1 : (STAGE == 3 ? B.S2 : B.S3));
   const size_t nc = (size_t)T.nlon * T.nlat * T.nlev;
-  float2* u3p = reinterpret_cast<float2*>(B.S1);  // u3 of the tracers as pairs, [ntr][nc]
-  const df c23{kTwoThirdsH, kTwoThirdsL}, c13{kThirdH, kThirdL};
+  float* u3h = reinterpret_cast<float*>(B.S1);  // u3 of the tracers, hi and lo planes [ntr][nc]
+  float* u3l = u3h + (size_t)T.ntr * nc;
+  const df c13 = mkdf(kThirdH, kThirdL);
+  const df rt = split_df(rtol), at0 = split_df(atol);
+  const bool pairs = atol >= 0x1p-100 && atol <= 0x1p100 && rtol >= 0x1p-60;  // else the norm in FP64
   const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0.0;
+  df ep = mkdf(0.0f, 0.0f);
   if (c < nc) {
     const int i = (int)(c % T.nlon);
     const int j = (int)((c / T.nlon) % T.nlat);
@@ -1597,11 +1855,11 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
     const size_t xm = (size_t)(T.nsp - 1) * nc + c;
     const double m = Qm[xm];
 #if RS_STRICT
-    const double rm = 1.0 / m;
+    const double rmg = g / m;
 #else
-    const double rm = rcp_nr(m);  // m > 0
+    const double rmg = g * rcp_nr(m);  // m > 0
 #endif
-    const df sc = split_df(dt_2 * rm);  // the tracer increment is (m dq/dt) * dt/2 / m
+    const df sc = split_df(-dt_2 * rmg);  // the tracer increment is acc * sc
     const size_t col = (size_t)j * T.nlon + i;
     // the air-mass row, in FP64 as the FP64 scheme forms it
     const double mn = fma(dmdt, dt_2, m);
@@ -1621,63 +1879,66 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
     }
     // one tracer from its loaded inputs (q, the accumulator, and for stages 3-4 the attempt's
     // input u0 and stage 4's u3); the norm terms are added in tracer order
-    auto tracer = [&](int s, size_t x, df q, float2 a, double u0, float2 u3) {
+    auto tracer = [&](int s, size_t x, df q, df a, double u0, df u3) {
       df nx;
       if (T.pbl) {  // with full PBL mixing the tendency is formed in FP64 (rare combination)
-        const double qd = df_to_d(make_float2(q.h, q.l));
-        const double du = fma(df_to_d(a), rm, pbl_term(T, c, col, s, qd));
+        const double qd = df_to_d(q);
+        const double du = fma(-df_to_d(a), rmg, pbl_term(T, c, col, s, qd));
         nx = split_df(fma(du, dt_2, qd));
       } else {
-        nx = df_add(q, df_mul(df{a.x, a.y}, sc));
+        nx = df_fma(a, sc, q);
       }
       if (STAGE == 1 || STAGE == 2) {
-        T.qhi[x] = nx.h;
-        T.qlo[x] = nx.l;
+        T.qhi[x] = nx.h.v;
+        T.qlo[x] = nx.l.v;
       } else if (STAGE == 3) {
-        u3p[x] = make_float2(nx.h, nx.l);
-        const df u4 = df_add(df_mul(c23, split_df(u0)), df_mul(c13, nx));
-        T.qhi[x] = u4.h;
-        T.qlo[x] = u4.l;
+        u3h[x] = nx.h.v;
+        u3l[x] = nx.l.v;
+        const df u0p = split_df(u0);
+        const df u4 = df_fma(c13, df_sub(nx, u0p), u0p);  // u0 + (u3 - u0) / 3
+        T.qhi[x] = u4.h.v;
+        T.qlo[x] = u4.l.v;
       } else {
-        const double un = df_to_d(make_float2(nx.h, nx.l));
-        // (1/3 u0 + 2/3 u3) - un in pairs, then FP64 for the norm; its factor 1/2 goes onto
-        // the cell's sum as an exact 1/4
-        const df ut = df_add(df_mul(c13, split_df(u0)), df_mul(c23, df{u3.x, u3.y}));
-        const df d = df_sub(ut, nx);
-        const double err = df_to_d(make_float2(d.h, d.l));
-        const double den = fma(amax_bits(u0, un), rtol, atol);
-        const double at = err * rcp_nr1(den);  // den >= atol > 0
-        e = fma(at, at, e);
+        const double un = df_to_d(nx);
+        // (1/3 u0 + 2/3 u3) - un from the two increments, so that no rounding is of the size of u;
+        // its factor 1/2 goes onto the cell's sum as an exact 1/4
+        const df u0p = split_df(u0);
+        const df d = df_fma(c13, df_sub(u0p, u3), df_sub(u3, nx));
+        // the larger of |U| and |unew|: signs off, then the sign of the difference
+        const df a0 = df_abs(u0p), a1 = df_abs(nx);
+        const df t = df_div(d, df_fma(df_diff(a0, a1).v < 0.0f ? a1 : a0, rt, at0));
+        if (pairs && fabsf(t.h.v) < 0x1p60f) ep = df_fma(t, t, ep);
+        else e += error_fp64(d.h.v, d.l.v, amax_bits(u0, un), rtol, atol);
         Un[x] = (clamp && __double2hiint(un) < 0) ? 0.0 : un;
       }
     };
     // tracers in groups of four: every load of a group is issued before its arithmetic, so a
     // thread keeps four tracers' loads in flight (the same arithmetic, in the same order)
     constexpr int kGrp = 4;
+    const df zero = mkdf(0.0f, 0.0f);
     int s = 0;
     for (; s + kGrp <= T.ntr; s += kGrp) {
-      df q[kGrp];
-      float2 a[kGrp], u3[kGrp];
+      df q[kGrp], a[kGrp], u3[kGrp];
       double u0[kGrp];
 #pragma unroll
       for (int r = 0; r < kGrp; ++r) {
         const size_t x = (size_t)(s + r) * nc + c;
-        q[r] = df{T.qhi[x], T.qlo[x]};
-        a[r] = T.acc[x];
+        q[r] = mkdf(T.qhi[x], T.qlo[x]);
+        a[r] = mkdf(T.acc.h[x], T.acc.l[x]);
         u0[r] = STAGE >= 3 ? U[x] : 0.0;
-        u3[r] = STAGE == 4 ? u3p[x] : make_float2(0.0f, 0.0f);
+        u3[r] = STAGE == 4 ? mkdf(u3h[x], u3l[x]) : zero;
       }
 #pragma unroll
       for (int r = 0; r < kGrp; ++r) tracer(s + r, (size_t)(s + r) * nc + c, q[r], a[r], u0[r], u3[r]);
     }
     for (; s < T.ntr; ++s) {
       const size_t x = (size_t)s * nc + c;
-      tracer(s, x, df{T.qhi[x], T.qlo[x]}, T.acc[x], STAGE >= 3 ? U[x] : 0.0,
-             STAGE == 4 ? u3p[x] : make_float2(0.0f, 0.0f));
+      tracer(s, x, mkdf(T.qhi[x], T.qlo[x]), mkdf(T.acc.h[x], T.acc.l[x]), STAGE >= 3 ? U[x] : 0.0,
+             STAGE == 4 ? mkdf(u3h[x], u3l[x]) : zero);
     }
   }
   if (STAGE == 4) {
-    const double tot = block_tree256(0.25 * e, sm);
+    const double tot = block_tree256(0.25 * (e + df_to_d(ep)), sm);
     if (threadIdx.x == 0) B.partial[blockIdx.x] = tot;
   }
 }
@@ -1710,7 +1971,7 @@ __global__ void __launch_bounds__(kRedThreads) k_rhs_eval(DevTransport<double> T
     if (s < T.ntr) {
       double adv;
       if (T.mixed) {  // the kernels accumulated m dq/dt as a pair
-        adv = df_to_d(T.acc[x]) / m;
+        adv = -(g * df_to_d(mkdf(T.acc.h[x], T.acc.l[x]))) / m;
       } else {
 #if RS_STRICT
         double fw = T.fx[s * fxp + fxi], fe = T.fx[s * fxp + fxi + 1];
@@ -1839,7 +2100,6 @@ static void launch_flux_one(cudaStream_t st, const DevTransport<double>& T, cons
     }
   }
 }
-void launch_scale_fluxes(cudaStream_t, const DevTransport<double>&, double*, double*, double*) {}
 #else
 // Launch shape of the FP64 kernels.  Lat / vertical pencil blocks are (pencil width 8, 16 or 32) x
 // up to `rows` threads, at most 512; a line of n cells takes n + 5 entries per phase, dealt evenly
@@ -1936,12 +2196,13 @@ static void launch_flux_one(cudaStream_t st, const DevTransport<double>& T, cons
   else
     k_adv_x_cell<<<dim3((unsigned)(((size_t)T.nlon * T.nlat * T.nlev + 255) / 256), (unsigned)T.ntr), 256, 0, st>>>(T, sel);
 }
+#endif
+
 void launch_scale_fluxes(cudaStream_t st, const DevTransport<double>& T, double* mx6, double* myn6,
                          double* mys6) {
   const size_t n = (size_t)T.nlev * std::max((size_t)T.nlat * (T.nlon + 1), (size_t)(T.nlat + 1) * T.nlon);
   k_scale_fluxes<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(T, mx6, myn6, mys6);
 }
-#endif
 
 // Mixed-precision pencils: the staged hi / lo rows (four with the second set of the bulk-copy
 // staging), the pair rows of the differences and slopes, and the face fluxes as pairs.
@@ -2042,22 +2303,31 @@ static void launch_fluxes_mixed(cudaStream_t st, const DevTransport<double>& T, 
   const size_t shx = mixed_pencil_bytes(T.nlon, 1, tx), shy = mixed_pencil_bytes(T.nlat, pw, ty),
                shz = mixed_pencil_bytes(T.nlev, pw, tz);
   static const CUtensorMap kNoMap{};  // placeholder argument of the plain-load variants
-  // rs_create refuses mixed precision on grids whose pencils do not fit at width 16
-  if ((only_dir < 0 || only_dir == 0) && T.mstream_x) {
+  // rs_create refuses mixed precision on grids whose pencils do not fit at width 16; the streaming
+  // kernels count the cells and faces of a tracer in 32 bits
+  const bool small = (long long)(T.nlev + 2) * (T.nlat + 1) * (T.nlon + 1) < (1LL << 31);
+  if ((only_dir < 0 || only_dir == 0) && T.mstream_x && small) {
     const long long warps = (long long)((T.nlon + kSegX - 1) / kSegX) * T.nlat * T.nlev;
-    k_adv_x_stream<<<dim3((unsigned)((warps + 3) / 4), groups(sx)), 128, 0, st>>>(T, sel, sx);
+    const unsigned grid = (unsigned)((warps + 3) / 4) * groups(sx);
+    if (sx > 1) k_adv_x_stream<2><<<grid, 128, 0, st>>>(T, sel, sx);
+    else k_adv_x_stream<1><<<grid, 128, 0, st>>>(T, sel, sx);
   } else if (only_dir < 0 || only_dir == 0) {
     dim3 grid((unsigned)(T.nlat * T.nlev), groups(sx));
     if (tx) k_adv_x_mixed<true><<<grid, xt, shx, st>>>(T, sel, sx);
     else k_adv_x_mixed<false><<<grid, xt, shx, st>>>(T, sel, sx);
   }
-  if (T.mstream_yz) {
-    if (only_dir < 0 || only_dir == 1)
-      k_adv_yz_stream<1><<<dim3((unsigned)((T.nlon + 127) / 128) * (unsigned)T.nlev, groups(syz)),
-                           128, 0, st>>>(T, sel, syz);
-    if (only_dir < 0 || only_dir == 2)
-      k_adv_yz_stream<2><<<dim3((unsigned)((ncol + 127) / 128), groups(syz)), 128, 0, st>>>(
-          T, sel, syz);
+  if (T.mstream_yz && small) {
+    const size_t lines = (size_t)T.nlon * T.nlev;
+    const unsigned gy = (unsigned)((lines + kLine32 - 1) / kLine32) * groups(syz),
+                   gz = (unsigned)((ncol + kLine32 - 1) / kLine32) * groups(syz);
+    if (only_dir < 0 || only_dir == 1) {
+      if (syz > 1) k_adv_yz_stream<1, 2><<<gy, kLine32, 0, st>>>(T, sel, syz);
+      else k_adv_yz_stream<1, 1><<<gy, kLine32, 0, st>>>(T, sel, syz);
+    }
+    if (only_dir < 0 || only_dir == 2) {
+      if (syz > 1) k_adv_yz_stream<2, 2><<<gz, kLine32, 0, st>>>(T, sel, syz);
+      else k_adv_yz_stream<2, 1><<<gz, kLine32, 0, st>>>(T, sel, syz);
+    }
     return;
   }
   if (only_dir < 0 || only_dir == 1) {
