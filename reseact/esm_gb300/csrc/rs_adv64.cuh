@@ -410,15 +410,8 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
   }
   double e = 0.0;
   if (c < nc) {
-    const int i = (int)(c % T.nlon);
-    const int j = (int)((c / T.nlon) % T.nlat);
-    const int k = (int)(c / ((size_t)T.nlon * T.nlat));
-    const CellGeo G{T.gx[j], T.gylo[j], T.gyhi[j]};
-    const MassFluxes F = mass_fluxes(T, i, j, k, 1.0);
-    double hz, vz;
-    div_parts(F, G, hz, vz);
-    const double dmdt = T.mcorr ? -((g * hz + T.mcorr[c]) + g * vz) : -(g * (hz + vz));
-    const size_t col = (size_t)j * T.nlon + i, xm = (size_t)(T.nsp - 1) * nc + c;
+    const double dmdt = T.mcorr ? -fma(g, T.mdiv[c], T.mcorr[c]) : -(g * T.mdiv[c]);
+    const size_t col = c % ((size_t)T.nlon * T.nlat), xm = (size_t)(T.nsp - 1) * nc + c;
     const double m = Qin[xm];
     const double rmg = g * rcp_nr(m);  // m > 0
     const double sc = -dt_2 * rmg;     // the tracer increment is acc * sc without PBL mixing

@@ -422,7 +422,7 @@ struct rs_handle {
   // divergence correction on the device; the diagnosed Mz replaces the mz field
   std::vector<double> mx_host, my_host, gx_host, gylo_host, gyhi_host, dpsdt_host;
   bool fixer_on = false;
-  DevBuf<double> mcorr;
+  DevBuf<double> mcorr, mdiv;
   std::shared_ptr<rs::JitChem> jit;
   // straight-line forms of the table-walking kernel this handle's mode runs, for mechanisms too
   // large for jit (null: not built)
@@ -563,7 +563,8 @@ void make_flux_pairs(rs_handle* h) {
   CK(cudaGetLastError());
 }
 
-// The kernels' scaled fluxes (after every flux change).
+// The kernels' scaled fluxes and the air-mass divergence (after every flux change, including the
+// pressure fixer's diagnosed Mz).
 void scale_fluxes(rs_handle* h) {
   h->mx6.alloc(h->mx.n);
   h->myn6.alloc(h->my.n);
@@ -573,7 +574,10 @@ void scale_fluxes(rs_handle* h) {
   T.lat_bc = h->cfg.grid.lat_bc;
   T.gx = h->gx.p; T.gylo = h->gylo.p; T.gyhi = h->gyhi.p;
   T.mx = h->mx.p; T.my = h->my.p;
+  T.mz = h->mz.p;
   rs::launch_scale_fluxes(h->st, T, h->mx6.p, h->myn6.p, h->mys6.p);
+  h->mdiv.alloc(h->nc);
+  rs::launch_air_divergence(h->st, T, h->mdiv.p);
   CK(cudaGetLastError());
 }
 
@@ -663,6 +667,7 @@ void refresh_dt(rs_handle* h) {
   T.vsA = h->vsA.p; T.vsB = h->vsB.p; T.veAB = h->veAB.p; T.veC = h->veC.p; T.veD = h->veD.p;
   T.fx = h->fx.p; T.fy = h->fy.p; T.fz = h->fz.p;
   T.acc64 = h->fx.p;
+  T.mdiv = h->mdiv.p;
   T.mx6 = h->mx6.p; T.myn6 = h->myn6.p; T.mys6 = h->mys6.p;
   T.mixed = h->cfg.precision == RS_PREC_MIXED;
   T.qhi = h->qhi.p; T.qlo = h->qlo.p;
@@ -1127,7 +1132,7 @@ void rs_destroy(rs_handle* h) {
                             &h->mx, &h->my, &h->mz, &h->qw, &h->qe, &h->qs, &h->qn, &h->gx,
                             &h->gylo, &h->gyhi, &h->vsA, &h->vsB, &h->veAB, &h->veC, &h->veD,
                             &h->dtcell, &h->stepcell, &h->totals, &h->fsal[0], &h->fsal[1],
-                            &h->pbl_f, &h->pbl_w, &h->pbl_den, &h->pbl_qbar, &h->mcorr};
+                            &h->pbl_f, &h->pbl_w, &h->pbl_den, &h->pbl_qbar, &h->mcorr, &h->mdiv};
   for (auto* b : bufs) b->release();
   h->slot_row.release();
   h->slot_col.release();
@@ -1241,7 +1246,7 @@ rs_status rs_set_forcing(rs_handle* h, const rs_forcing* f) {
       if (pbl_inputs) build_pbl(h);
       if (f->dps_dt) h->dpsdt_host.assign(f->dps_dt, f->dps_dt + ncol);
       if (f->dps_dt || f->hyb_b || f->mx || f->my || f->mz || f->dp) build_fixer(h);
-      if (f->mx || f->my) scale_fluxes(h);
+      if (f->dps_dt || f->hyb_b || f->mx || f->my || f->mz || f->dp) scale_fluxes(h);
       if (h->cfg.precision == RS_PREC_MIXED) make_flux_pairs(h);
     }
     if (f->temperature) {

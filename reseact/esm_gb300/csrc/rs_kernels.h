@@ -70,6 +70,7 @@ struct DevTransport {
   const double* mx6;   // shape of mx
   const double* myn6;  // shape of my, as the cell south of the face sees it
   const double* mys6;  // and the cell north of it
+  const double* mdiv;  // [nc] the air-mass flux divergence at time factor 1
   // mixed precision (compensated FP32): the RHS input split into hi, lo planes [ntr][nc]
   // (hi + lo = q to 2^-47), the vertical coefficients (twice the slopes', half the edges' slope
   // terms) and the air-mass face fluxes as hi and lo planes (mx12 .. mys12: mx6 .. mys6 / 2), and
@@ -177,6 +178,8 @@ void launch_flux_dir(cudaStream_t st, const DevTransport<double>& T, const doubl
 // the scaled air-mass fluxes mx6, myn6, mys6 from mx, my
 void launch_scale_fluxes(cudaStream_t st, const DevTransport<double>& T, double* mx6, double* myn6,
                          double* mys6);
+// the air-mass flux divergence of every cell from mx, my, mz
+void launch_air_divergence(cudaStream_t st, const DevTransport<double>& T, double* mdiv);
 // scale times n doubles as hi and lo planes, dst[0..n) and dst[n..2n)
 void launch_make_pairs(cudaStream_t st, const double* src, double scale, float* dst, size_t n);
 void launch_flux_dir_mixed(cudaStream_t st, const DevTransport<double>& T, const double* Q, int dir,

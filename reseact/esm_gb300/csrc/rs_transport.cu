@@ -764,13 +764,21 @@ __device__ __forceinline__ bool upwind_lo(float M, int gs) { return (__float_as_
 // split a double into a pair: production build with integer operations (split_bits below,
 // truncating: hi + lo = v to 2^-47), strict build with conversions
 __device__ __forceinline__ df split_df(double v);
+// The conversions of values outside the integer forms' range are calls: as short branches they are
+// predicated, and an FP64-pipe instruction holds the pipe for its 64 cycles with no lane active too
+// (57 of the 88 such instructions of a cell's stage 4 with 12 tracers were of this kind).
+__device__ __noinline__ double f2d_convert(float x) { return (double)x; }
+__device__ __noinline__ float2 split_convert(double v) {
+  const float h = (float)v;
+  return make_float2(h, (float)(v - (double)h));
+}
 // float -> double by re-biasing the exponent in the integer pipes (exact; zero kept, subnormal,
 // inf and NaN convert)
 __device__ __forceinline__ double f2d_bits(float x) {
   const unsigned u = __float_as_uint(x);
   const unsigned fe = (u >> 23) & 0xffu;
   if ((u << 1) == 0u) return __hiloint2double((int)(u & 0x80000000u), 0);
-  if (fe == 0u || fe == 255u) return (double)x;
+  if (fe == 0u || fe == 255u) return f2d_convert(x);
   return __hiloint2double((int)((u & 0x80000000u) | ((fe + 896u) << 20) | ((u & 0x7fffffu) >> 3)),
                           (int)(u << 29));
 }
@@ -1487,9 +1495,9 @@ __device__ __forceinline__ void split_bits(double v, float& hi, float& lo) {
   const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
   const int e = (int)((h >> 20) & 0x7ff);
   if (e < 949 || e > 1150) {
-    // volatile: the compiler otherwise runs this branch's FP64 instructions on every value
-    asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(hi) : "d"(v));
-    lo = (float)(v - (double)hi);
+    const float2 p = split_convert(v);
+    hi = p.x;
+    lo = p.y;
     return;
   }
   const unsigned sign = h & 0x80000000u;
@@ -1620,6 +1628,20 @@ __device__ __forceinline__ void div_parts(const MassFluxes& F, const CellGeo& G,
 __device__ __forceinline__ void div_parts(const DevTransport<double>& T, int i, int j, int k,
                                           double g, const CellGeo& G, double& hz, double& vz) {
   div_parts(mass_fluxes(T, i, j, k, g), G, hz, vz);
+}
+// The air-mass flux divergence of every cell at time factor 1, once per forcing change: formed by the
+// stage kernels it was 16 of their 26 FP64 instructions per cell, four times per attempt.
+__global__ void k_air_divergence(DevTransport<double> T, double* __restrict__ mdiv) {
+  const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= (size_t)T.nlon * T.nlat * T.nlev) return;
+  const int i = (int)(c % T.nlon), j = (int)((c / T.nlon) % T.nlat);
+  double hz, vz;
+  div_parts(T, i, j, (int)(c / ((size_t)T.nlon * T.nlat)), 1.0, CellGeo{T.gx[j], T.gylo[j], T.gyhi[j]}, hz, vz);
+  mdiv[c] = hz + vz;
+}
+void launch_air_divergence(cudaStream_t st, const DevTransport<double>& T, double* mdiv) {
+  const size_t nc = (size_t)T.nlon * T.nlat * T.nlev;
+  k_air_divergence<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(T, mdiv);
 }
 #if RS_STRICT
 __device__ __forceinline__ double div_m(const DevTransport<double>& T, int i, int j, int k,
@@ -1795,7 +1817,8 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
 // error and the hairer norm are formed in pairs as well (relative error ~1e-13 after the one
 // cancellation, which the pairs of the states carry anyway; the FP64 form's one-step reciprocal has
 // 1e-12): eight FP64 instructions per cell and tracer, 64 cycles each, had made this stage five
-// times as long as the others (144x91x47: 211 us against 41; 360x181x72 with 30 tracers 3.47 ms).
+// times as long as the others (144x91x47: 211 us against 41, now 86; 360x181x72 with 30 tracers
+// 3.47 ms).  Stages 1-2 take 32 us there, close to the 30 us of their bytes.
 // The air-mass row is the FP64 scheme's, stage by stage (m in the air-mass planes of U, S1, S2, S3).
 //   1: P = U + dt/2 f(U)          2: P = P + dt/2 f(P)
 //   3: u3 = P + dt/2 f(P) -> S1 (pairs), P = u4 = U + (u3 - U) / 3
@@ -1814,8 +1837,8 @@ __device__ __forceinline__ df df_div(df a, df b) {
   const float rem = __fmaf_rn(-q, b.l.v, __fadd_rn(__fmaf_rn(-q, b.h.v, a.h.v), a.l.v));
   return df_renorm(df{{q}, {__fmul_rn(rem, r)}});
 }
-// one tracer's squared error ratio in FP64, for what is outside the pairs' range (and NaN).  A
-// call: inlined, its FP64 instructions ran (and were thrown away) on the ordinary path too.
+// one tracer's squared error ratio in FP64, for what is outside the pairs' range (and NaN); a call
+// for the reason given at f2d_convert
 __device__ __noinline__ double error_fp64(float dh, float dl, double am, double rtol, double atol) {
   const double at = df_to_d(mkdf(dh, dl)) * rcp_nr1(fma(am, rtol, atol));  // den >= atol > 0
   return at * at;
@@ -1844,14 +1867,7 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
   double e = 0.0;
   df ep = mkdf(0.0f, 0.0f);
   if (c < nc) {
-    const int i = (int)(c % T.nlon);
-    const int j = (int)((c / T.nlon) % T.nlat);
-    const int k = (int)(c / ((size_t)T.nlon * T.nlat));
-    const CellGeo G{T.gx[j], T.gylo[j], T.gyhi[j]};
-    const MassFluxes F = mass_fluxes(T, i, j, k, g);
-    double hz, vz;
-    div_parts(F, G, hz, vz);
-    const double dmdt = T.mcorr ? -((hz + T.mcorr[c]) + vz) : -(hz + vz);
+    const double dmdt = T.mcorr ? -fma(g, T.mdiv[c], T.mcorr[c]) : -(g * T.mdiv[c]);
     const size_t xm = (size_t)(T.nsp - 1) * nc + c;
     const double m = Qm[xm];
 #if RS_STRICT
@@ -1860,7 +1876,7 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
     const double rmg = g * rcp_nr(m);  // m > 0
 #endif
     const df sc = split_df(-dt_2 * rmg);  // the tracer increment is acc * sc
-    const size_t col = (size_t)j * T.nlon + i;
+    const size_t col = c % ((size_t)T.nlon * T.nlat);
     // the air-mass row, in FP64 as the FP64 scheme forms it
     const double mn = fma(dmdt, dt_2, m);
     if (STAGE == 1) B.S1[xm] = mn;
