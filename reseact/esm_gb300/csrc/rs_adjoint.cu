@@ -234,6 +234,7 @@ __device__ __forceinline__ void slope_form(double am, double a, double ap, doubl
     val = sg * ada;
   }
 }
+#if RS_STRICT
 // slope_form without branches: the same value and coefficients for every input.  Each
 // coefficient of a limited slope is an exact constant (0, +-1/2, +-2) or a sign flip of a
 // vertical coefficient, so the frozen branch is picked by integer compares of the magnitude
@@ -247,11 +248,7 @@ __device__ __forceinline__ void slope_form_bf(double am, double a, double ap, do
     slope_form(am, a, ap, sA, sB, uniform, val, c);
     return;
   }
-#if RS_STRICT
   const bool live = d1 * d0 > 0.0;
-#else
-  const bool live = sgn_same_nz(d0, d1);  // the forward kernels' test
-#endif
   const double da = uniform ? 0.5 * (ap - am) : sA * d1 + sB * d0;
   const int s0 = __double2hiint(d0), s1 = __double2hiint(d1), sd = __double2hiint(da);
   const unsigned h0 = (unsigned)s0 & 0x7fffffffu, l0 = (unsigned)__double2loint(d0);
@@ -281,6 +278,7 @@ __device__ __forceinline__ void slope_form_bf(double am, double a, double ap, do
   c[1] = live ? sel_d(binds, q1, u1) : 0.0;
   c[2] = live ? sel_d(binds, q2, u2) : 0.0;
 }
+#endif
 
 __device__ __forceinline__ void face_weights_lin(const double* v, bool right, bool uniform,
                                                  const double* sA, const double* sB,
@@ -516,7 +514,9 @@ __global__ void __launch_bounds__(256) k_adj_gather(DevTransport<double> T, cons
   }
 }
 
+#if RS_STRICT
 // ------------------------------------------------------------------ fused adjoint pencils
+// (strict build; the production build sweeps the forward kernels' advective form, rs_adj64.cuh)
 // One block per pencil (a lon row; or PW adjacent lat lines / vertical columns), looping over
 // the tracers.  The same arithmetic as face_weights_lin + the per-cell gather, reorganised:
 //   1. the tracer values (3-cell halo) and the cell adjoints g = fbar / m go to shared memory;
@@ -688,15 +688,6 @@ __global__ void __launch_bounds__(256) k_adj_pencil(DevTransport<double> T,
       const double dA = aRv - aLv;
       const double a6 = 6.0 * (a - 0.5 * (aLv + aRv));
       bool flat, stl, str;
-#if !RS_STRICT
-      if (!(tiny_operand(a) || tiny_operand(aLv) || tiny_operand(aRv))) {
-        const long long ka = ord_key(a), kl = ord_key(aLv), kr = ord_key(aRv);
-        flat = !((kr > ka && ka > kl) || (kr < ka && ka < kl));
-        const long long kd = ord_key(dA), k6 = ord_key(a6);
-        stl = (kd > 0 && k6 > kd) || (kd < 0 && k6 < kd);
-        str = !stl && ((kd > 0 && k6 < -kd) || (kd < 0 && k6 > -kd));
-      } else
-#endif
       {
         flat = (aRv - a) * (a - aLv) <= 0.0;
         stl = dA * a6 > dA * dA;                      // aL <- 3a - 2aR
@@ -789,26 +780,7 @@ __global__ void __launch_bounds__(256) k_adj_pencil(DevTransport<double> T,
 #undef AV
 }
 
-// ubar = (d f_T / du)^T fbar at stage state U (whose RHS value is F), time factor g
-// VJP of the PBL mixing term t_k = f_k (qbar - q_k) / tau with qbar = sum_j w_j q_j / den:
-// ubar_j += (w_j / den) * (sum_k fbar_k f_k) / tau - fbar_j f_j / tau, per tracer and column
-// (the term does not depend on the air mass).
-__global__ void k_pbl_vjp(DevTransport<double> T, const double* __restrict__ fbar,
-                          double* __restrict__ ubar) {
-  const size_t ncol = (size_t)T.nlon * T.nlat, nc = ncol * T.nlev;
-  const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= (size_t)T.ntr * ncol) return;
-  const size_t s = id / ncol, col = id % ncol;
-  const double* fb = fbar + s * nc + col;
-  double* ub = ubar + s * nc + col;
-  double a = 0.0;
-  for (int k = 0; k < T.nlev; ++k) a = a + fb[(size_t)k * ncol] * T.pbl_f[(size_t)k * ncol + col];
-  const double at = a / T.pbl_tau, den = T.pbl_den[col];
-  for (int k = 0; k < T.nlev; ++k) {
-    const size_t x = (size_t)k * ncol + col;
-    ub[(size_t)k * ncol] += (T.pbl_w[x] / den) * at - (fb[(size_t)k * ncol] * T.pbl_f[x]) / T.pbl_tau;
-  }
-}
+#include "rs_adj64.cuh"
 
 // The fused adjoint pencils for all three directions, or false (nothing launched) when a
 // direction's pencils do not fit in shared memory -- the caller then uses the face + gather
@@ -874,13 +846,43 @@ static bool launch_adj_pencils(cudaStream_t st, const DevTransport<double>& T, c
   return true;
 }
 
+#endif  // RS_STRICT
+#include "rs_adj64.cuh"
+
+// VJP of the PBL mixing term t_k = f_k (qbar - q_k) / tau with qbar = sum_j w_j q_j / den:
+// ubar_j += (w_j / den) * (sum_k fbar_k f_k) / tau - fbar_j f_j / tau, per tracer and column
+// (the term does not depend on the air mass).
+__global__ void k_pbl_vjp(DevTransport<double> T, const double* __restrict__ fbar,
+                          double* __restrict__ ubar) {
+  const size_t ncol = (size_t)T.nlon * T.nlat, nc = ncol * T.nlev;
+  const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= (size_t)T.ntr * ncol) return;
+  const size_t s = id / ncol, col = id % ncol;
+  const double* fb = fbar + s * nc + col;
+  double* ub = ubar + s * nc + col;
+  double a = 0.0;
+  for (int k = 0; k < T.nlev; ++k) a = a + fb[(size_t)k * ncol] * T.pbl_f[(size_t)k * ncol + col];
+  const double at = a / T.pbl_tau, den = T.pbl_den[col];
+  for (int k = 0; k < T.nlev; ++k) {
+    const size_t x = (size_t)k * ncol + col;
+    ub[(size_t)k * ncol] += (T.pbl_w[x] / den) * at - (fb[(size_t)k * ncol] * T.pbl_f[x]) / T.pbl_tau;
+  }
+}
+
+// ubar = (d f_T / du)^T fbar at stage state U (whose RHS value is F), time factor g
 void launch_transport_rhs_vjp(cudaStream_t st, const DevTransport<double>& T, const double* U,
                               const double* F, const double* fbar, double* ubar, double* G,
                               double* Cf, double g) {
   size_t nc = (size_t)T.nlon * T.nlat * T.nlev;
   unsigned nb = (unsigned)((nc + 255) / 256);
+#if !RS_STRICT
+  const bool done = launch_adj_dev(st, T, U, F, fbar, ubar, G, g);
+  if (!done) k_adj_cell<<<nb, 256, 0, st>>>(T, U, F, fbar, ubar, G, g);
+#else
   k_adj_cell<<<nb, 256, 0, st>>>(T, U, F, fbar, ubar, G, g);
-  if (!launch_adj_pencils(st, T, U, G, ubar, g)) {  // pencils too long for shared memory
+  const bool done = launch_adj_pencils(st, T, U, G, ubar, g);
+#endif
+  if (!done) {  // lines too long for shared memory
     long long nx = (long long)(T.nlon + 1) * T.nlat * T.nlev;
     long long ny = (long long)T.nlon * (T.nlat + 1) * T.nlev;
     long long nz = (long long)T.nlon * T.nlat * (T.nlev + 1);

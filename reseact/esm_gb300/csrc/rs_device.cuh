@@ -279,13 +279,6 @@ __device__ __forceinline__ void lu_solve(const DevMech& M, const double* W, cons
 // ------------------------------------------------------------------ integer-pipe FP64 helpers
 // Sign tests, magnitude compares and selects of doubles on their bit patterns (the integer
 // pipes; FP64 issues at ~2 lanes per SM per clock on this GPU).
-// d0, d1 nonzero with equal signs: d1*d0 > 0 unless the product underflows
-__device__ __forceinline__ bool sgn_same_nz(double a, double b) {
-  const int ha = __double2hiint(a), hb = __double2hiint(b);
-  const bool nza = ((ha & 0x7fffffff) | __double2loint(a)) != 0;
-  const bool nzb = ((hb & 0x7fffffff) | __double2loint(b)) != 0;
-  return ((ha ^ hb) >= 0) & nza & nzb;
-}
 constexpr long long kMagMask = 0x7fffffffffffffffLL, kSignBit = (long long)0x8000000000000000ULL,
                     kExpOne = 1LL << 52;
 __device__ __forceinline__ double sel_d(bool c, double x, double y) {
@@ -310,20 +303,6 @@ __device__ __forceinline__ bool prod_may_underflow(double d0, double d1) {
   const int e0 = bexp(d0), e1 = bexp(d1);
   return e0 == 0 || e1 == 0 || e0 + e1 < 980;
 }
-// Any nonzero difference of doubles >= 2^-484 in magnitude (or zero) is >= 2^-537, so
-// products of two such differences do not underflow; tiny operands use the FP form.
-__device__ __forceinline__ bool tiny_operand(double x) {
-  return !is_zero_d(x) && bexp(x) < 539;
-}
-// Order-preserving integer key of a finite double (-0 and +0 both map to 0, key(-x) = -key(x)):
-// the sign of the rounded difference x - y is the sign of key(x) - key(y) (gradual underflow
-// makes x - y == 0 exactly when x == y), so the limiter's sign tests need no subtraction.
-__device__ __forceinline__ long long ord_key(double x) {
-  const long long b = __double_as_longlong(x);
-  const long long sgn = b >> 63;  // 0 or -1
-  return (b ^ (sgn & kMagMask)) - sgn;
-}
-
 // ------------------------------------------------------------------ fixed-tree reductions
 // Pairwise tree over 256 lanes: v[t] += v[t+s] for s = 128 ... 1 (identical to the CPU
 // restatement's tree256).  Returns the total in thread 0.
