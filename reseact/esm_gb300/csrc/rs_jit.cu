@@ -245,6 +245,27 @@ struct Gen {
   // constant (kd_r = -dtg * K_r) before the partials at x are formed, so each Jacobian entry of
   // W is its plain sum of scaled partials (plus 1 on the diagonal): one multiply per reaction
   // instead of one per entry.
+  // the off-diagonal Jacobian entry whose terms are those of diagonal entry d, negated, or -1
+  int negated_entry(int d) const {
+    const int n = T.jac_ptr[d + 1] - T.jac_ptr[d];
+    for (int e = 0; e < T.njac; ++e) {
+      if (T.jac_diag[e] || n < 2 || T.jac_ptr[e + 1] - T.jac_ptr[e] != n) continue;
+      bool eq = true;
+      for (int t = 0; t < n && eq; ++t)
+        eq = T.jac_part[T.jac_ptr[e] + t] == T.jac_part[T.jac_ptr[d] + t] &&
+             T.jac_coef[T.jac_ptr[e] + t] == -T.jac_coef[T.jac_ptr[d] + t];
+      if (eq) return e;
+    }
+    return -1;
+  }
+  // pivot k is exactly 1: no Jacobian entry on its diagonal and no elimination update
+  bool unit_pivot(int k) const {
+    for (int e = 0; e < T.njac; ++e)
+      if (T.jac_diag[e] && T.jac_slot[e] == T.lu_diag[k] && T.jac_ptr[e + 1] > T.jac_ptr[e]) return false;
+    for (int dst : T.upd_dst)
+      if (dst == T.lu_diag[k]) return false;
+    return true;
+  }
   void build_w_scaled() {
     std::vector<char> used(T.nr, 0);
     for (int p = 0; p < T.npart; ++p) used[T.part_r[p]] = 1;
@@ -252,7 +273,8 @@ struct Gen {
     for (int r = 0; r < T.nr; ++r)
       if (used[r]) o << "  const double kd" << r << "_ = -dtg * K(" << r << ");\n";
     partials("x", "P", true);
-    std::vector<std::string> w(T.nlu, "0.0");
+    std::vector<std::string> w(T.nlu, "0.0"), tail(T.nlu);
+    std::vector<int> late;  // slots formed from another slot
     for (int i = 0; i < T.ns; ++i) w[T.lu_diag[i]] = "1.0";
     for (int e = 0; e < T.njac; ++e) {
       std::ostringstream acc;
@@ -262,9 +284,16 @@ struct Gen {
         first = false;
       }
       if (first) continue;
-      w[T.jac_slot[e]] = T.jac_diag[e] ? "1.0 + (" + acc.str() + ")" : acc.str();
+      // a loss that is another entry's production, term by term: one sum for both (negation is exact)
+      const int same = T.jac_diag[e] ? negated_entry(e) : -1;
+      if (same >= 0) w[T.jac_slot[e]] = "1.0 - WV(" + std::to_string(T.jac_slot[same]) + ")", late.push_back(T.jac_slot[e]);
+      else w[T.jac_slot[e]] = T.jac_diag[e] ? "1.0 + (" + acc.str() + ")" : acc.str();
     }
-    for (int e = 0; e < T.nlu; ++e) o << "  WV(" << e << ") = " << w[e] << ";\n";
+    for (int sl : late) std::swap(w[sl], tail[sl]);
+    for (int e = 0; e < T.nlu; ++e)
+      if (tail[e].empty()) o << "  WV(" << e << ") = " << w[e] << ";\n";
+    for (int e = 0; e < T.nlu; ++e)
+      if (!tail[e].empty()) o << "  WV(" << e << ") = " << tail[e] << ";\n";
     o << "  }\n";
   }
   // (eh, el) <- W^-1 (eh, el) in float pairs from the FP64 factors, split entry by entry
@@ -283,6 +312,8 @@ struct Gen {
     for (int k = 0; k < T.ns; ++k) {
       if (strict)
         o << "  pv[" << k << "] = 1.0 / WV(" << T.lu_diag[k] << ");\n";
+      else if (unit_pivot(k))
+        o << "  pv[" << k << "] = 1.0;\n";
       else
         o << "  pv[" << k << "] = rcp_nr(WV(" << T.lu_diag[k] << "));\n";
       for (int ii = T.elim_ptr[k]; ii < T.elim_ptr[k + 1]; ++ii, ++m) {
@@ -1605,17 +1636,17 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
 }
 
 // An FP64 warp instruction takes 64 cycles of its SM sub-partition, so a block's warps cost most
-// where they stack on few SMs or leave a coarse last wave: 64 threads while 128-cell blocks would
-// leave SMs idle (152 SMs; 36x18x10, 6,480 cells: 73 us per attempt at 256 threads, 40 at 64),
-// 128 above (314,900 cells: 609 -> 574 us; 155,664: 300 -> 295; 615,888: 1,075 -> 1,070), 256 from
-// 4 M cells on, where the last wave is nothing and the partial sums would outnumber the
+// where they stack on few SMs or leave a coarse last wave: 64 threads up to 2^17 cells (6,480 cells:
+// 73 us per attempt at 256 threads, 40 at 64; 29,160: 70 / 66 / 54 at 256 / 128 / 64; 111,555: 199 /
+// 194 / 194), 128 above (314,900 cells: 609 -> 574 us; 155,664: 300 -> 295; 615,888: 1,075 -> 1,070),
+// 256 from 4 M cells on, where the last wave is nothing and the partial sums would outnumber the
 // allocation-free attempt's scratch.  The strict build keeps the oracle's 256-cell partial sums.
 int jit_attempt_block(int nc) {
 #if RS_STRICT
   (void)nc;
   return kBlock;
 #else
-  return nc <= 152 * 128 ? 64 : (nc <= (1 << 22) ? 128 : kBlock);
+  return nc <= (1 << 17) ? 64 : (nc <= (1 << 22) ? 128 : kBlock);
 #endif
 }
 
