@@ -173,33 +173,73 @@ struct Gen {
       o << "  const double u" << r << "_ = " << h.str() << ";\n";
       last[r] = fac.empty() ? std::string() : std::string(x) + "[" + std::to_string(fac.back()) + "]";
     }
-    for (int sp = 0; sp < T.ns; ++sp) {
+    // Sums that two species have in common (one's loss is the other's production) are formed once:
+    // n shared terms cost n + 2 instructions instead of 2 n.  Rows are lists of (term, coefficient);
+    // term r < nr is reaction r, nr + k the k-th shared sum; the pair with the most in common first.
+    typedef std::vector<std::pair<int, double>> Row;
+    std::vector<Row> rows(T.ns);
+    for (int sp = 0; sp < T.ns; ++sp)
+      for (int t = T.rhs_ptr[sp]; t < T.rhs_ptr[sp + 1]; ++t) rows[sp].push_back({T.rhs_r[t], T.rhs_c[t]});
+    for (;;) {
+      size_t most = 2;
+      int bi = -1, bj = -1;
+      double brho = 1.0;
+      auto common = [&](int i, int j, double rho) {
+        Row v;
+        for (auto& x : rows[i])
+          for (auto& y : rows[j])
+            if (x.first == y.first && y.second == rho * x.second) v.push_back(x);
+        return v;
+      };
+      for (int i = 0; i < (int)rows.size(); ++i)
+        for (int j = i + 1; j < (int)rows.size(); ++j)
+          for (double rho : {1.0, -1.0}) {
+            const size_t n = common(i, j, rho).size();
+            if (n > most) most = n, bi = i, bj = j, brho = rho;
+          }
+      if (bi < 0) break;
+      const Row shared = common(bi, bj, brho);
+      for (int k : {bi, bj}) {
+        Row rest;
+        for (auto& x : rows[k])
+          if (std::none_of(shared.begin(), shared.end(), [&](const std::pair<int, double>& y) { return y.first == x.first; }))
+            rest.push_back(x);
+        rest.push_back({T.nr + (int)rows.size() - T.ns, k == bi ? 1.0 : brho});
+        rows[k] = rest;
+      }
+      rows.push_back(shared);
+    }
+    auto sum = [&](const Row& row) {
       std::string acc;
-      for (int t = T.rhs_ptr[sp]; t < T.rhs_ptr[sp + 1]; ++t) {
-        const int r = T.rhs_r[t];
-        const double cf = T.rhs_c[t];
-        const std::string u = "u" + std::to_string(r) + "_";
+      for (auto& tc : row) {
+        const int r = tc.first;
+        const double cf = tc.second;
+        const std::string u = r < T.nr ? "u" + std::to_string(r) + "_" : "g" + std::to_string(r - T.nr) + "_";
+        const std::string lf = r < T.nr ? last[r] : std::string();
         std::string term;  // the product c * v_r, for a first term
-        if (last[r].empty()) term = cf == 1.0 ? u : (cf == -1.0 ? "(-" + u + ")" : lit(cf) + "*" + u);
-        else if (cf == 1.0) term = u + "*" + last[r];
-        else if (cf == -1.0) term = "(-" + u + ")*" + last[r];
-        else term = lit(cf) + "*(" + u + "*" + last[r] + ")";
+        if (lf.empty()) term = cf == 1.0 ? u : (cf == -1.0 ? "(-" + u + ")" : lit(cf) + "*" + u);
+        else if (cf == 1.0) term = u + "*" + lf;
+        else if (cf == -1.0) term = "(-" + u + ")*" + lf;
+        else term = lit(cf) + "*(" + u + "*" + lf + ")";
         if (acc.empty()) {
           acc = term;
-        } else if (last[r].empty()) {
+        } else if (lf.empty()) {
           acc = cf == 1.0 ? acc + " + " + u : (cf == -1.0 ? acc + " - " + u : "RS_FMA(" + lit(cf) + ", " + u + ", " + acc + ")");
         } else if (cf == 1.0) {
-          acc = "RS_FMA(" + u + ", " + last[r] + ", " + acc + ")";
+          acc = "RS_FMA(" + u + ", " + lf + ", " + acc + ")";
         } else if (cf == -1.0) {
-          acc = "RS_FMA(-" + u + ", " + last[r] + ", " + acc + ")";
+          acc = "RS_FMA(-" + u + ", " + lf + ", " + acc + ")";
         } else {
-          acc = "RS_FMA(" + lit(cf) + ", " + u + "*" + last[r] + ", " + acc + ")";
+          acc = "RS_FMA(" + lit(cf) + ", " + u + "*" + lf + ", " + acc + ")";
         }
       }
-      if (acc.empty()) acc = "0.0";
-      o << "  { const double a_ = " << acc << "; " << f << "[" << sp << "] = HE ? a_ + EM(" << sp
+      return acc.empty() ? std::string("0.0") : acc;
+    };
+    for (int k = (int)rows.size() - 1; k >= T.ns; --k)  // a shared sum may hold later ones
+      o << "  const double g" << k - T.ns << "_ = " << sum(rows[k]) << ";\n";
+    for (int sp = 0; sp < T.ns; ++sp)
+      o << "  { const double a_ = " << sum(rows[sp]) << "; " << f << "[" << sp << "] = HE ? a_ + EM(" << sp
         << ") : a_; }\n";
-    }
     o << "  }\n";
   }
   // Partial derivatives dv_r/dx_q of the rates at xa; `scaled` forms them from kd<r>_ =
