@@ -561,6 +561,17 @@ __device__ __forceinline__ double quant_dt(double d) {
   return __longlong_as_double(__double_as_longlong(d) & ~((1ll << 48) - 1));
 }
 
+// The first wave's warps of one SM sub-partition (`depth` of them fit; 152 SMs with four each) start
+// apart, over the FP64 time of one warp (RS_WARP_NS).  Started together they stay in lock step: all
+// load, convert and miss the instruction cache at once and leave the FP64 pipe idle, and they
+// finish together, so that what is left over runs as a whole extra wave.  One warp alone keeps the
+// pipe busy, so the wait costs nothing once the grid has more than one wave (615,888 cells: 910 ->
+// 886 us per attempt, 314,496: 497 -> 479, 155,664: 271 -> 255, 111,555: 186 -> 178).
+__device__ __forceinline__ void stagger(unsigned depth) {
+  const unsigned wpb = blockDim.x >> 5, w = blockIdx.x * wpb / 608u;
+  if (w > 0u && w < depth && gridDim.x * wpb > depth * 608u) __nanosleep(w * RS_WARP_NS / (depth - 1u));
+}
+
 // block total of v in thread 0: strict build (256 threads), the oracle's pairwise tree v[t] +=
 // v[t+s] for s = 128 ... 1; production build, a shuffle tree per warp and the warps' sums in
 // order (whole warps, at most 8)
@@ -613,6 +624,11 @@ std::string generate(const MechTables& T, double ros_d, double ros_c32, bool str
     << offsetof(Ctl, kzcap) << "\n";
   // the kernels in units that compile side by side (RS_UNIT 0: all of them)
   o << "#ifndef RS_UNIT\n#define RS_UNIT 0\n#endif\n#define RS_IN(k) (RS_UNIT == 0 || RS_UNIT == (k))\n";
+  // about the FP64 instructions of an attempt (two right-hand sides, the Jacobian, W, its LU, two
+  // solves, the updates) at 64 cycles of 0.48 ns
+  const size_t ops = 2 * (T.rhs_r.size() + T.nr) + T.nr + T.npart + T.jac_part.size() + T.upd_dst.size() +
+                     T.elim_lik.size() + 2 * T.nlu + 11 * T.ns;
+  o << "#define RS_WARP_NS " << ops * 31 << "u\n";
   o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude;
   // Every multiply-add is written out: RS_FMA fuses in the production build and keeps the
   // multiply and the add separate in the strict build; both builds compile with --fmad=false,
@@ -809,7 +825,7 @@ __device__ __noinline__ double attempt_error_fp64(const double* __restrict__ U,
                                     nullptr, dt, dto2, dto6, dtg, rtol, atol, nullptr);
 }
 #endif
-template <bool HE, int MODE, bool PAIRS>
+template <bool HE, int MODE, bool PAIRS, int MINB>
 __device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ ctl,
     double* __restrict__ U0, double* __restrict__ U1, const double* __restrict__ kr,
     const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,
@@ -830,6 +846,9 @@ __device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ c
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const u64 N = (u64)nc;
   double e = 0.0;
+#if !RS_STRICT
+  stagger(2 * MINB);
+#endif
   if (c < nc) {
     double x[NS], xn[NS], f0[NS];
 #pragma unroll
@@ -955,7 +974,7 @@ __device__ __forceinline__ void per_cell_body(int nc, int nsp, double* __restric
       const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,         \
       double rtol, double atol, int clamp, double* __restrict__ F0,                         \
       double* __restrict__ F1) {                                                            \
-    attempt_body<HE, MODE, PAIRS>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
+    attempt_body<HE, MODE, PAIRS, MINB>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
                            F1);                                                             \
   }
 #define RS_PAIRS (!RS_STRICT)
@@ -1041,6 +1060,9 @@ __device__ __forceinline__ void vjp_body(int nc, int nsp, const double* __restri
     double* __restrict__ lam_out, const double* __restrict__ kr,
     const double* __restrict__ em, double* __restrict__ ebar, double dt, int clamp,
     const double* __restrict__ kzi) {
+#if !RS_STRICT
+  stagger(2);
+#endif
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
   const u64 N = (u64)nc;
