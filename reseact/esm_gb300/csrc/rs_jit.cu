@@ -561,17 +561,6 @@ __device__ __forceinline__ double quant_dt(double d) {
   return __longlong_as_double(__double_as_longlong(d) & ~((1ll << 48) - 1));
 }
 
-// The first wave's warps of one SM sub-partition (`depth` of them fit; 152 SMs with four each) start
-// apart, over the FP64 time of one warp (RS_WARP_NS).  Started together they stay in lock step: all
-// load, convert and miss the instruction cache at once and leave the FP64 pipe idle, and they
-// finish together, so that what is left over runs as a whole extra wave.  One warp alone keeps the
-// pipe busy, so the wait costs nothing once the grid has more than one wave (615,888 cells: 910 ->
-// 886 us per attempt, 314,496: 497 -> 479, 155,664: 271 -> 255, 111,555: 186 -> 178).
-__device__ __forceinline__ void stagger(unsigned depth) {
-  const unsigned wpb = blockDim.x >> 5, w = blockIdx.x * wpb / 608u;
-  if (w > 0u && w < depth && gridDim.x * wpb > depth * 608u) __nanosleep(w * RS_WARP_NS / (depth - 1u));
-}
-
 // block total of v in thread 0: strict build (256 threads), the oracle's pairwise tree v[t] +=
 // v[t+s] for s = 128 ... 1; production build, a shuffle tree per warp and the warps' sums in
 // order (whole warps, at most 8)
@@ -629,7 +618,18 @@ std::string generate(const MechTables& T, double ros_d, double ros_c32, bool str
   const size_t ops = 2 * (T.rhs_r.size() + T.nr) + T.nr + T.npart + T.jac_part.size() + T.upd_dst.size() +
                      T.elim_lik.size() + 2 * T.nlu + 11 * T.ns;
   o << "#define RS_WARP_NS " << ops * 31 << "u\n";
-  o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude;
+  o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude << R"(
+// The first wave's warps of one SM sub-partition (`depth` of them fit; 152 SMs with four each) start
+// apart, over the FP64 time of one warp (RS_WARP_NS).  Started together they stay in lock step: all
+// load, convert and miss the instruction cache at once and leave the FP64 pipe idle, and they
+// finish together, so that what is left over runs as a whole extra wave.  One warp alone keeps the
+// pipe busy, so the wait costs nothing once the grid has more than one wave (615,888 cells: 910 ->
+// 886 us per attempt, 314,496: 497 -> 479, 155,664: 271 -> 255, 111,555: 186 -> 178).
+__device__ __forceinline__ void stagger(unsigned depth) {
+  const unsigned wpb = blockDim.x >> 5, w = blockIdx.x * wpb / 608u;
+  if (w > 0u && w < depth && gridDim.x * wpb > depth * 608u) __nanosleep(w * RS_WARP_NS / (depth - 1u));
+}
+)";
   // Every multiply-add is written out: RS_FMA fuses in the production build and keeps the
   // multiply and the add separate in the strict build; both builds compile with --fmad=false,
   // so no compiler contraction decides anything and all variants compute the same bits.
