@@ -169,22 +169,47 @@ def ros23_flops_per_cell(mech, order=None):
     return 3 * (vel + rhs) + part + buildw + lu + 3 * solve + stage + err
 
 
+def shared_rows(rows, nr):
+    """The right-hand side's rows [(reaction, coefficient)] with the sums that two of them have in
+    common (up to sign) split off as rows of their own, nr + k standing for the k-th, as the
+    generator does: n shared terms cost n + 2 instructions instead of 2 n."""
+    rows, ns = [list(r) for r in rows], len(rows)
+    while True:
+        best = (2, None)
+        for i in range(len(rows)):
+            for j in range(i + 1, len(rows)):
+                for rho in (1.0, -1.0):
+                    com = [(r, c) for r, c in rows[i] if (r, rho * c) in rows[j]]
+                    if len(com) > best[0]:
+                        best = (len(com), (i, j, rho, com))
+        if best[1] is None:
+            return rows
+        i, j, rho, com = best[1]
+        gone = {r for r, _ in com}
+        new = nr + len(rows) - ns
+        for k, c in ((i, 1.0), (j, rho)):
+            rows[k] = [x for x in rows[k] if x[0] not in gone] + [(new, c)]
+        rows.append(com)
+
+
 def ros23_exec_counts(mech, order, evals, emissions=False):
     """(FP64 flops, FP64 instructions) per cell of one attempt of the mechanism-specialised ROS23
     kernel as generated (production build).  `evals` = 3 RHS evaluations, or 2 when the attempt
     reuses f(x).
 
-    Flops are the algorithm's: each rate product once per reaction and one multiply-add per
-    stoichiometric term (+-1 coefficients folded into adds), FMA = 2; the LU with a
-    third-order refined reciprocal per pivot (three FMAs), the solves, the stage algebra and
-    the error norm with one Newton step per reciprocal.  Instructions follow the fused RHS the generator emits: per
-    reaction one head u_r = K_r * (all factors but the last), each +-1 term one FMA of u_r with
-    the last factor (a multiply for a sum's first term), terms with other coefficients sharing
-    one product u_r * last.  The FMAs re-multiply u_r * last per term, so the executed flops
-    exceed these by the products that the rate-once form shares.  W = I - dtg*J is formed from
-    partials of kd_r = -dtg*K_r, and the error norm takes dto6^2 out of its sum.  Checked
-    against ncu's DADD/DMUL/DFMA counts of the kernel (3-evaluation attempt of SuperFast in the
-    minimum-fill order: 1,037 instructions counted here, 997.5 measured)."""
+    Flops are the algorithm's FP64 work: each rate product once per reaction and one multiply-add
+    per stoichiometric term (+-1 coefficients folded into adds), FMA = 2; the LU with a
+    third-order refined reciprocal per pivot (three FMAs), the two solves of the step and the stage
+    algebra.  The error estimate's solve and norm run in float pairs on the FP32 pipe and are not
+    counted.  Instructions follow the code the generator emits: per reaction one head u_r = K_r *
+    (all factors but the last), each +-1 term one FMA of u_r with the last factor (a multiply for a
+    sum's first term), terms with other coefficients sharing one product u_r * last, sums that two
+    species share formed once (shared_rows).  The FMAs re-multiply u_r * last per term, so the
+    executed flops exceed these by the products that the rate-once form shares.  W = I - dtg*J is
+    formed from partials of kd_r = -dtg*K_r; a loss that is another entry's production reuses its
+    sum, and a pivot of exactly 1 needs neither reciprocal nor scaling.  Checked against ncu's
+    DADD/DMUL/DFMA counts of the kernel (3-evaluation attempt of SuperFast in the minimum-fill
+    order: 812 instructions counted here, 821 measured)."""
     t = mech.tables()
     ns = mech.ns
 
@@ -204,11 +229,11 @@ def ros23_exec_counts(mech, order, evals, emissions=False):
         rf += terms(t["rhs_coef"][t["rhs_ptr"][sp]:t["rhs_ptr"][sp + 1]])[1]
     ri = sum(max(n - 1, 0) for n in nfac)  # the heads
     shared = set()  # reactions whose product u_r * last is formed once for non-unit terms
-    for sp in range(ns):
-        lo, hi = t["rhs_ptr"][sp], t["rhs_ptr"][sp + 1]
-        for k, (r, c) in enumerate(zip(t["rhs_reaction"][lo:hi], t["rhs_coef"][lo:hi])):
-            r = int(r)
-            if nfac[r] == 0:  # u_r is the rate itself
+    rows = [list(zip(t["rhs_reaction"][lo:hi].tolist(), t["rhs_coef"][lo:hi].tolist()))
+            for lo, hi in zip(t["rhs_ptr"][:-1], t["rhs_ptr"][1:])]
+    for row in shared_rows(rows, len(nfac)):
+        for k, (r, c) in enumerate(row):
+            if r >= len(nfac) or nfac[r] == 0:  # a shared sum, or the rate itself
                 ri += terms([c])[0] if k == 0 else 1
             else:
                 ri += 1
@@ -226,17 +251,23 @@ def ros23_exec_counts(mech, order, evals, emissions=False):
     # per reaction with partials, each entry its folded sum, plus 1 on the diagonal
     diag = set(int(x) for x in t["lu_diag"])
     wi = wf = len(set(int(r) for r in t["part_reaction"]))
-    for e in range(t["n_jac"]):
-        a, b = terms(t["jac_coef"][t["jac_ptr"][e]:t["jac_ptr"][e + 1]])
+    entry = [tuple(zip(t["jac_part"][t["jac_ptr"][e]:t["jac_ptr"][e + 1]].tolist(),
+                       t["jac_coef"][t["jac_ptr"][e]:t["jac_ptr"][e + 1]].tolist())) for e in range(t["n_jac"])]
+    off = set(v for e, v in enumerate(entry) if int(t["jac_slot"][e]) not in diag)
+    lossless = len(diag)  # pivots without a Jacobian entry (nothing updates those of SuperFast)
+    for e, v in enumerate(entry):
+        a, b = terms([c for _, c in v])
         d = int(t["jac_slot"][e]) in diag
+        lossless -= d and len(v) > 0
+        if d and len(v) >= 2 and tuple((p, -c) for p, c in v) in off:
+            a = 0  # the other entry's sum
         wi, wf = wi + a + d, wf + b + d
     _, n_mult, n_upd, n_low, n_up = mech.lu_counts(order)
-    lu_i, lu_f = 3 * ns + n_mult + n_upd, 6 * ns + n_mult + 2 * n_upd
-    sv_i, sv_f = n_low + n_up + ns, 2 * (n_low + n_up) + ns
-    stage_i, stage_f = 8 * ns, 12 * ns
-    norm_i, norm_f = 7 * ns + 2, 12 * ns + 2  # dto6^2 applied once to the sum
-    inst = evals * ri + part + wi + lu_i + 3 * sv_i + stage_i + norm_i
-    flops = evals * rf + part + wf + lu_f + 3 * sv_f + stage_f + norm_f
+    lu_i, lu_f = 3 * (ns - lossless) + n_mult + n_upd, 6 * (ns - lossless) + n_mult + 2 * n_upd
+    sv_i, sv_f = n_low + n_up + ns - lossless, 2 * (n_low + n_up) + ns - lossless
+    stage_i, stage_f = 8 * ns, 12 * ns  # with the right-hand side of the estimate
+    inst = evals * ri + part + wi + lu_i + 2 * sv_i + stage_i + 1
+    flops = evals * rf + part + wf + lu_f + 2 * sv_f + stage_f + 1
     return flops, inst
 
 
@@ -249,16 +280,15 @@ def ros23_rhs_flops_per_cell(mech):
 
 def transport_flops_per_cell(nsp):
     """FP64 flops of one SSPRK43 attempt per cell as the production kernels execute them
-    (counted from their source, FMA = 2): per stage and tracer the x and y pencils 16 each
-    (neighbour difference, slope span, edge, branch-free limiter, flux) and the dp-weighted
-    vertical pencil 19; the stage kernels 12 per tracer in stages 1-2, 15 in stage 3 and 26 in
-    stage 4 (embedded error and norm), plus ~35 per cell and stage for the air-mass divergence
-    and row.  ncu measures 19 / 19 / 22 per face for the pencils (halo cells and the
-    compiler's choice of DMUL+DADD over DFMA), so this is the lower figure."""
+    (counted from their source, FMA = 2): per stage and tracer the lon rows 12, the lat lines 13
+    (neighbour difference, slope span, slope difference, edge, left edge, the other face term, two
+    accumulating FMAs) and the dp-weighted vertical lines 15; the stage kernels 2 per tracer in
+    stages 1-2, 5 in stage 3 and 15 in stage 4 (embedded error and norm), plus ~12 per cell and
+    stage for the air-mass row.  Halo cells are not counted."""
     ntr = nsp - 1
-    pencils = 4 * ntr * (16 + 16 + 19)
-    stages = ntr * (12 + 12 + 15 + 26) + 4 * 35
-    return pencils + stages
+    lines = 4 * ntr * (12 + 13 + 15)
+    stages = ntr * (2 + 2 + 5 + 15) + 4 * 12
+    return lines + stages
 
 
 def transport_bytes_per_cell(nsp):
@@ -459,10 +489,10 @@ def run_gb300(args):
                     "bound": "fp64", "achieved": round(achieved, 4),
                     "peak": peak, "unit": "TFLOP/s", "frac": round(achieved / peak, 4) if peak else None,
                     # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
-                    # one ncu capture of each variant's first launch on this workload: the
-                    # 128-register variant 235.7 + 606.6 MB (mostly spill stores), the split
-                    # variant (part of W in shared memory) 204.5 + 265.1 MB; null otherwise
-                    "traffic": ({"regs2": 842.4e6, "split": 469.6e6}.get(kinfo.get("variant"))
+                    # one ncu capture of each variant's first launch on this workload: 255 registers
+                    # 197.2 + 46.4 MB, 128 registers 247.3 + 546.0 MB (mostly spill stores), the
+                    # split variant (part of W in shared memory) 197.3 + 71.0 MB; null otherwise
+                    "traffic": ({"regs": 243.6e6, "regs2": 793.3e6, "split": 268.3e6}.get(kinfo.get("variant"))
                                 if (kinfo.get("kind") == "specialized" and not args.small) else None),
                     "traffic_source": "ncu capture summarised in profiles/rs_jit_attempt_c2_144x91x47.md",
                     "flops_per_cell_attempt": round(f_exec, 1),

@@ -252,13 +252,16 @@ rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len);
 
 /* Set one launch shape that rs_autotune would choose, e.g. to replay an earlier tuning without
  * timing again (no reference counterpart).  Keys: "xthreads", "pencil", "rows",
- * "x_tracer_groups", "yz_tracer_groups" (FP64 pencils);
+ * "x_tracer_groups", "yz_tracer_groups" (FP64 lon rows and pencils), "yz_line" (1: one thread
+ * per lat / vertical line instead of the pencils); shapes neither set nor tuned follow the grid;
  * "mixed_xthreads", "mixed_x_tracers", "mixed_pencil", "mixed_rows", "mixed_yz_tracers",
  * "mixed_x_bulk", "mixed_yz_bulk" (mixed pencils); "mixed_x_stream", "mixed_yz_stream" (1: the
  * streaming forms of the mixed kernels instead of the pencils); "per_cell_threads",
  * "per_cell_blocks_per_sm", "per_cell_group" (per-cell chemistry; group 0 = one thread per
  * cell, 4 / 8 / 16 = lanes per cell, production build only), "per_cell_regcap" (1: the
- * table-walking per-cell kernel at 32 registers); "chem_attempt_variant" (0 "regs", 1 "smem",
+ * table-walking per-cell kernel at 32 registers), "per_cell_wide" (1: the straight-line per-cell
+ * kernel of a large mechanism, where built; the other per-cell keys select the table-walking
+ * kernels); "chem_attempt_variant" (0 "regs", 1 "smem",
  * 2 "regs2", 3 "split": how the specialised attempt kernel keeps W, where built).  Values outside a key's
  * candidates are RS_ERR_INVALID.  Every shape gives bit-identical results. */
 rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
@@ -269,8 +272,11 @@ rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
  *   straight-line CUDA at rs_create and compiled for the device with NVRTC (mechanisms of up
  *   to 32 species and 256 LU slots);
  * TABLE: one kernel for every mechanism that walks the sparse tables;
- * AUTO (the default): SPECIALIZED when it could be built, else TABLE.
- * Both compute the same arithmetic in the same order.  rs_set_chem_kernel returns
+ * AUTO (the default): SPECIALIZED when it could be built, else TABLE, for which the production
+ *   build also generates straight-line kernels (up to 64 species, 640 LU slots and 256 reactions;
+ *   the table kernels' bits; a table selected by name walks the tables).
+ * In the strict build both compute the same arithmetic in the same order; in the production build
+ * they agree to rounding.  rs_set_chem_kernel returns
  * RS_ERR_UNSUPPORTED for SPECIALIZED when it could not be built (reason in rs_last_error). */
 enum { RS_CHEM_KERNEL_AUTO = 0, RS_CHEM_KERNEL_TABLE = 1, RS_CHEM_KERNEL_SPECIALIZED = 2 };
 rs_status rs_set_chem_kernel(rs_handle* h, int32_t kind);
