@@ -1808,21 +1808,6 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
   }
 }
 #endif  // RS_STRICT
-#include "rs_adv64.cuh"
-
-// Compensated-FP32 stage kernel (mixed precision).  The tracers of stages 1-3 stay pairs:
-// the stage input is the (hi, lo) planes, the update q + dt/2 * (m dq/dt) / m is formed in pairs
-// and written back into those planes (in place: the update is pointwise), u3 is kept as hi and lo
-// planes in the tracer part of S1; stage 4 returns to FP64 with the candidate state.  Its embedded
-// error and the hairer norm are formed in pairs as well (relative error ~1e-13 after the one
-// cancellation, which the pairs of the states carry anyway; the FP64 form's one-step reciprocal has
-// 1e-12): eight FP64 instructions per cell and tracer, 64 cycles each, had made this stage five
-// times as long as the others (144x91x47: 211 us against 41, now 86; 360x181x72 with 30 tracers
-// 3.47 ms).  Stages 1-2 take 32 us there, close to the 30 us of their bytes.
-// The air-mass row is the FP64 scheme's, stage by stage (m in the air-mass planes of U, S1, S2, S3).
-//   1: P = U + dt/2 f(U)          2: P = P + dt/2 f(P)
-//   3: u3 = P + dt/2 f(P) -> S1 (pairs), P = u4 = U + (u3 - U) / 3
-//   4: unew = P + dt/2 f(P); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 constexpr float kThirdH = (float)(1.0 / 3.0);
 constexpr float kThirdL = (float)(1.0 / 3.0 - (double)(float)(1.0 / 3.0));
 __device__ __forceinline__ df df_abs(df a) {  // of a normalised pair
@@ -1843,6 +1828,47 @@ __device__ __noinline__ double error_fp64(float dh, float dl, double am, double 
   const double at = df_to_d(mkdf(dh, dl)) * rcp_nr1(fma(am, rtol, atol));  // den >= atol > 0
   return at * at;
 }
+// One tracer's error err against the tolerance of |u|: (err / (am rtol + atol))^2 added to the pair
+// ep on the FP32 pipe, or to e in FP64 where the pairs' range does not hold it.  The split is
+// branch-free: h the leading 24 bits, l the 29 below them rounded to 24 (fewer below 2^-74; 0 below
+// 2^-126).
+__device__ __forceinline__ df split_any(double v, unsigned& big) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mag = hi & 0x7fffffffu;
+  big = max(big, mag);
+  const unsigned f = (__funnelshift_l(lo, hi, 3) ^ 0x40000000u) & 0x7fffffffu;  // exponent - 896
+  const int sc = max((int)(f & 0x7f800000u) - (52 << 23), 0);
+  const float l = __fmul_rn(__int2float_rn((int)(lo & 0x1fffffffu)), __int_as_float(sc));
+  const unsigned sg = hi & 0x80000000u;
+  const bool z = mag < (898u << 20);
+  return mkdf(z ? 0.0f : __uint_as_float(f | sg), z ? 0.0f : __uint_as_float(__float_as_uint(l) ^ sg));
+}
+__device__ __noinline__ double error_term(double err, double am, double rtol, double atol) {
+  const double at = err * rcp_nr1(fma(am, rtol, atol));  // den >= atol > 0
+  return at * at;
+}
+__device__ __forceinline__ void add_error(double err, double am, double rtol, double atol, df rt, df at0,
+                                          bool pairs, df& ep, double& e) {
+  unsigned big = 0;
+  const df t = df_div(split_any(err, big), df_fma(split_any(am, big), rt, at0));
+  if (pairs && big < (1126u << 20) && fabsf(t.h.v) < 0x1p60f) ep = df_fma(t, t, ep);
+  else e += error_term(err, am, rtol, atol);
+}
+#include "rs_adv64.cuh"
+
+// Compensated-FP32 stage kernel (mixed precision).  The tracers of stages 1-3 stay pairs:
+// the stage input is the (hi, lo) planes, the update q + dt/2 * (m dq/dt) / m is formed in pairs
+// and written back into those planes (in place: the update is pointwise), u3 is kept as hi and lo
+// planes in the tracer part of S1; stage 4 returns to FP64 with the candidate state.  Its embedded
+// error and the hairer norm are formed in pairs as well (relative error ~1e-13 after the one
+// cancellation, which the pairs of the states carry anyway; the FP64 form's one-step reciprocal has
+// 1e-12): eight FP64 instructions per cell and tracer, 64 cycles each, had made this stage five
+// times as long as the others (144x91x47: 211 us against 41, now 86; 360x181x72 with 30 tracers
+// 3.47 ms).  Stages 1-2 take 32 us there, close to the 30 us of their bytes.
+// The air-mass row is the FP64 scheme's, stage by stage (m in the air-mass planes of U, S1, S2, S3).
+//   1: P = U + dt/2 f(U)          2: P = P + dt/2 f(P)
+//   3: u3 = P + dt/2 f(P) -> S1 (pairs), P = u4 = U + (u3 - U) / 3
+//   4: unew = P + dt/2 f(P); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double> T,
                                                              const Ctl* __restrict__ ctl,
