@@ -188,6 +188,10 @@ __global__ void __launch_bounds__(kRedThreads) k_finalize_graph(
     Ctl* __restrict__ c, const double* __restrict__ partial, int nparts,
     cudaGraphConditionalHandle loop) {
   __shared__ double sm[kRedThreads];
+#if !RS_STRICT
+  // launched while the attempt's last blocks still run; lets the next attempt be launched
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+#endif
   finalize_body(c, partial, nparts, sm);
   __syncthreads();
   if (threadIdx.x == 0) cudaGraphSetConditional(loop, c->done ? 0u : 1u);
@@ -280,7 +284,16 @@ void launch_finalize(cudaStream_t st, Ctl* ctl, const double* partial, int npart
 }
 void launch_finalize_graph(cudaStream_t st, Ctl* ctl, const double* partial, int nparts,
                            cudaGraphConditionalHandle loop) {
-  k_finalize_graph<<<1, kRedThreads, 0, st>>>(ctl, partial, nparts, loop);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(kRedThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = RS_STRICT ? 0 : 1;
+  cudaLaunchKernelEx(&cfg, k_finalize_graph, ctl, partial, nparts, loop);
 }
 void launch_ctl_init(cudaStream_t st, Ctl* ctl, const Ctl& init) {
   k_ctl_init<<<1, 1, 0, st>>>(ctl, init);
