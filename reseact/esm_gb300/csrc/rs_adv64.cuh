@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
                                                        TransportBufs B, double rtol,
                                                        double atol, int clamp) {
   __shared__ double sm[kRedThreads];
+  await_previous();
   if (ctl->done) return;
   const double g = ctl->g[STAGE - 1];
   const int cur = ctl->cur;

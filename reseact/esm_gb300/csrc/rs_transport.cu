@@ -161,7 +161,43 @@ struct StageSel {
   const double* Q;  // direct evaluation
   double g;
 };
+// Start of a kernel that `behind` launches: waits for the grid before it, lets the next one be launched.
+__device__ __forceinline__ void await_previous() {
+#if !RS_STRICT
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+#if !RS_STRICT
+// The kernels of an attempt depend on each other in a row.  Launched one by one from the host on a
+// small grid, each goes programmatically behind the one before, as soon as that one's blocks have
+// started, and waits in await_previous: the launches' latency is hidden (the hook calls of 36x18x10
+// 184 -> 173 us).  Not inside a graph, whose launches are already queued on the device, and not on
+// larger grids, where the waiting blocks take room from the running ones (180x91x72: 25.5 -> 25.8 ms).
+template <typename... P, typename... A>
+static void behind(const DevTransport<double>& T, void (*k)(P...), dim3 grid, dim3 block, size_t smem,
+                   cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if ((long long)T.nlon * T.nlat * T.nlev <= 152 * 128) cudaStreamIsCapturing(st, &cap);
+  cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, P(std::forward<A>(args))...);
+}
+#else
+template <typename... P, typename... A>
+static void behind(const DevTransport<double>&, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  k<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+}
+#endif
 __device__ __forceinline__ bool resolve_stage(const StageSel& s, const double*& Q, double& g) {
+  await_previous();
   if (!s.ctl) {
     Q = s.Q;
     g = s.g;
@@ -1573,6 +1609,7 @@ __global__ void __launch_bounds__(kRedThreads) k_split_input(DevTransport<double
                                                              const double* __restrict__ U1,
                                                              const double* __restrict__ Qd) {
   const double* U;
+  await_previous();
   if (ctl) {
     if (ctl->done) return;
     U = ctl->cur ? U1 : U0;
@@ -1875,6 +1912,7 @@ __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double
                                                              TransportBufs B, double rtol,
                                                              double atol, int clamp) {
   __shared__ double sm[kRedThreads];
+  await_previous();
   if (ctl->done) return;
   const double g = ctl->g[STAGE - 1];
   const int cur = ctl->cur;
@@ -2218,25 +2256,25 @@ static void launch_adv_yz(cudaStream_t st, const DevTransport<double>& T, const 
   const size_t ncol = (size_t)T.nlon * T.nlat;
   if (!(DIR == 1 ? f.fy : f.fz)) {
     const size_t lines = DIR == 1 ? (size_t)T.nlon * T.nlev : ncol;
-    k_adv_line<DIR><<<dim3((unsigned)((lines + kLineThreads - 1) / kLineThreads), (unsigned)T.ntr), kLineThreads, 0, st>>>(T, sel);
+    behind(T, k_adv_line<DIR>, dim3((unsigned)((lines + kLineThreads - 1) / kLineThreads), (unsigned)T.ntr), kLineThreads, 0, st, T, sel);
     return;
   }
   const unsigned tiles = DIR == 1 ? (unsigned)((T.nlon + f.pw - 1) / f.pw) * (unsigned)T.nlev
                                   : (unsigned)((ncol + f.pw - 1) / f.pw);
   const dim3 grid(tiles, (unsigned)f.gyz), block(f.pw, even_rows(DIR == 1 ? T.nlat : T.nlev, f.rows));
   const size_t sh = DIR == 1 ? f.shy : f.shz;
-  if (f.pw == 8) k_adv_pencil<DIR, 8><<<grid, block, sh, st>>>(T, sel);
-  else if (f.pw == 16) k_adv_pencil<DIR, 16><<<grid, block, sh, st>>>(T, sel);
-  else k_adv_pencil<DIR, 32><<<grid, block, sh, st>>>(T, sel);
+  if (f.pw == 8) behind(T, k_adv_pencil<DIR, 8>, grid, block, sh, st, T, sel);
+  else if (f.pw == 16) behind(T, k_adv_pencil<DIR, 16>, grid, block, sh, st, T, sel);
+  else behind(T, k_adv_pencil<DIR, 32>, grid, block, sh, st, T, sel);
 }
 static void launch_flux_one(cudaStream_t st, const DevTransport<double>& T, const StageSel& sel,
                             const FluxShape& f, int dir) {
   if (dir == 1) launch_adv_yz<1>(st, T, sel, f);
   else if (dir == 2) launch_adv_yz<2>(st, T, sel, f);
   else if (f.fx)
-    k_adv_x_rows<<<dim3((unsigned)((T.nlat * T.nlev + f.xr - 1) / f.xr), (unsigned)f.gx), f.xt, f.shx, st>>>(T, sel, f.xr);
+    behind(T, k_adv_x_rows, dim3((unsigned)((T.nlat * T.nlev + f.xr - 1) / f.xr), (unsigned)f.gx), f.xt, f.shx, st, T, sel, f.xr);
   else
-    k_adv_x_cell<<<dim3((unsigned)(((size_t)T.nlon * T.nlat * T.nlev + 255) / 256), (unsigned)T.ntr), 256, 0, st>>>(T, sel);
+    behind(T, k_adv_x_cell, dim3((unsigned)(((size_t)T.nlon * T.nlat * T.nlev + 255) / 256), (unsigned)T.ntr), 256, 0, st, T, sel);
 }
 #endif
 
@@ -2351,8 +2389,8 @@ static void launch_fluxes_mixed(cudaStream_t st, const DevTransport<double>& T, 
   if ((only_dir < 0 || only_dir == 0) && T.mstream_x && small) {
     const long long warps = (long long)((T.nlon + kSegX - 1) / kSegX) * T.nlat * T.nlev;
     const unsigned grid = (unsigned)((warps + 3) / 4) * groups(sx);
-    if (sx > 1) k_adv_x_stream<2><<<grid, 128, 0, st>>>(T, sel, sx);
-    else k_adv_x_stream<1><<<grid, 128, 0, st>>>(T, sel, sx);
+    if (sx > 1) behind(T, k_adv_x_stream<2>, grid, 128, 0, st, T, sel, sx);
+    else behind(T, k_adv_x_stream<1>, grid, 128, 0, st, T, sel, sx);
   } else if (only_dir < 0 || only_dir == 0) {
     dim3 grid((unsigned)(T.nlat * T.nlev), groups(sx));
     if (tx) k_adv_x_mixed<true><<<grid, xt, shx, st>>>(T, sel, sx);
@@ -2363,12 +2401,12 @@ static void launch_fluxes_mixed(cudaStream_t st, const DevTransport<double>& T, 
     const unsigned gy = (unsigned)((lines + kLine32 - 1) / kLine32) * groups(syz),
                    gz = (unsigned)((ncol + kLine32 - 1) / kLine32) * groups(syz);
     if (only_dir < 0 || only_dir == 1) {
-      if (syz > 1) k_adv_yz_stream<1, 2><<<gy, kLine32, 0, st>>>(T, sel, syz);
-      else k_adv_yz_stream<1, 1><<<gy, kLine32, 0, st>>>(T, sel, syz);
+      if (syz > 1) behind(T, k_adv_yz_stream<1, 2>, gy, kLine32, 0, st, T, sel, syz);
+      else behind(T, k_adv_yz_stream<1, 1>, gy, kLine32, 0, st, T, sel, syz);
     }
     if (only_dir < 0 || only_dir == 2) {
-      if (syz > 1) k_adv_yz_stream<2, 2><<<gz, kLine32, 0, st>>>(T, sel, syz);
-      else k_adv_yz_stream<2, 1><<<gz, kLine32, 0, st>>>(T, sel, syz);
+      if (syz > 1) behind(T, k_adv_yz_stream<2, 2>, gz, kLine32, 0, st, T, sel, syz);
+      else behind(T, k_adv_yz_stream<2, 1>, gz, kLine32, 0, st, T, sel, syz);
     }
     return;
   }
@@ -2444,36 +2482,36 @@ void launch_ssprk43_attempt(cudaStream_t st, const DevTransport<double>& T, cons
   if (T.mixed) {  // compensated FP32: the stages stay pairs until stage 4
     launch_fluxes(st, T, sel);
     if (T.pbl) launch_pbl_mean(st, T, sel);
-    k_stage_mixed<1><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+    behind(T, k_stage_mixed<1>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
     sel.stage = 2;
     launch_fluxes(st, T, sel);
     if (T.pbl) launch_pbl_mean(st, T, sel);
-    k_stage_mixed<2><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+    behind(T, k_stage_mixed<2>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
     sel.stage = 3;
     launch_fluxes(st, T, sel);
     if (T.pbl) launch_pbl_mean(st, T, sel);
-    k_stage_mixed<3><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+    behind(T, k_stage_mixed<3>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
     sel.stage = 4;
     launch_fluxes(st, T, sel);
     if (T.pbl) launch_pbl_mean(st, T, sel);
-    k_stage_mixed<4><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+    behind(T, k_stage_mixed<4>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
     return;
   }
   launch_fluxes(st, T, sel);
   if (T.pbl) launch_pbl_mean(st, T, sel);
-  k_stage<1><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+  behind(T, k_stage<1>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
   sel.stage = 2;
   launch_fluxes(st, T, sel);
   if (T.pbl) launch_pbl_mean(st, T, sel);
-  k_stage<2><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+  behind(T, k_stage<2>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
   sel.stage = 3;
   launch_fluxes(st, T, sel);
   if (T.pbl) launch_pbl_mean(st, T, sel);
-  k_stage<3><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+  behind(T, k_stage<3>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
   sel.stage = 4;
   launch_fluxes(st, T, sel);
   if (T.pbl) launch_pbl_mean(st, T, sel);
-  k_stage<4><<<nb, kRedThreads, 0, st>>>(T, ctl, B, rtol, atol, clamp);
+  behind(T, k_stage<4>, nb, kRedThreads, 0, st, T, ctl, B, rtol, atol, clamp);
 }
 
 void launch_transport_rhs(cudaStream_t st, const DevTransport<double>& T, const double* U,
