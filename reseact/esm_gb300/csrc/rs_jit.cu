@@ -204,7 +204,7 @@ struct Gen {
         for (auto& x : rows[k])
           if (std::none_of(shared.begin(), shared.end(), [&](const std::pair<int, double>& y) { return y.first == x.first; }))
             rest.push_back(x);
-        rest.push_back({T.nr + (int)rows.size() - T.ns, k == bi ? 1.0 : brho});
+        rest.insert(rest.begin(), {T.nr + (int)rows.size() - T.ns, k == bi ? 1.0 : brho});
         rows[k] = rest;
       }
       rows.push_back(shared);
