@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(128) k_adv_line(DevTransport<double> T, StageS
 __device__ __noinline__ double tendency(double a, double rmg) { return -a * rmg; }
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
-                                                       const Ctl* __restrict__ ctl,
+                                                       const Ctl* ctl,
                                                        TransportBufs B, double rtol,
                                                        double atol, int clamp) {
   __shared__ double sm[kRedThreads];

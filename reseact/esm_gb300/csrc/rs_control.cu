@@ -35,8 +35,7 @@ __device__ void prepare_next(Ctl* c) {
 }
 
 // One attempt's close-out (all threads of one 256-thread block); returns in every thread.
-__device__ void finalize_body(Ctl* __restrict__ c, const double* __restrict__ partial,
-                              int nparts, double* sm) {
+__device__ void finalize_body(Ctl* c, const double* partial, int nparts, double* sm) {
   if (c->done) return;
   double acc = 0.0;
   for (int q = threadIdx.x; q < nparts; q += kRedThreads) acc = acc + partial[q];
@@ -104,8 +103,7 @@ __device__ void stage_factors(Ctl* c) {
   if (w == 1) c->g[3] = v;
 }
 constexpr int kSumWarps = 6;
-__device__ void finalize_body(Ctl* __restrict__ c, const double* __restrict__ partial,
-                              int nparts, double* sm) {
+__device__ void finalize_body(Ctl* c, const double* partial, int nparts, double* sm) {
   if (c->done) return;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (w < kSumWarps) {
@@ -185,11 +183,11 @@ __global__ void __launch_bounds__(kRedThreads) k_finalize(Ctl* __restrict__ c,
 // the loop condition on EVERY path (0 once the controller is done), and the controller raises
 // done after at most maxiters attempts, so the graph loop always terminates.
 __global__ void __launch_bounds__(kRedThreads) k_finalize_graph(
-    Ctl* __restrict__ c, const double* __restrict__ partial, int nparts,
-    cudaGraphConditionalHandle loop) {
+    Ctl* c, const double* partial, int nparts, cudaGraphConditionalHandle loop) {
   __shared__ double sm[kRedThreads];
 #if !RS_STRICT
-  // launched while the attempt's last blocks still run; lets the next attempt be launched
+  // launched while the attempt's last blocks still run (they write partial, and c is read by them: no
+  // __restrict__ on either); lets the next attempt be launched
   asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 #endif
   finalize_body(c, partial, nparts, sm);

@@ -646,10 +646,16 @@ __device__ __forceinline__ void stagger(unsigned depth) {
   o << R"(
 // the stage-tape slot of the attempt a controller is running (null when it keeps no tape):
 // slot = the accepted count, [2][NS][N] doubles per slot, slots below the controller's kzcap
-__device__ __forceinline__ double* stage_slot(const unsigned char* __restrict__ ctl, u64 N) {
-  double* kz = *(double* const*)(ctl + OFF_KZ);
-  const int cap = *(const int*)(ctl + OFF_KZCAP);
-  const int slot = (int)*(const double*)(ctl + OFF_NACC);
+// a field of the controller record, which the grid before this one may still be writing until the
+// wait: a coherent load that stays in program order
+template <class V>
+__device__ __forceinline__ V ctl_field(const unsigned char* ctl, int off) {
+  return *(const volatile V*)(ctl + off);
+}
+__device__ __forceinline__ double* stage_slot(const unsigned char* ctl, u64 N) {
+  double* kz = ctl_field<double*>(ctl, OFF_KZ);
+  const int cap = ctl_field<int>(ctl, OFF_KZCAP);
+  const int slot = (int)ctl_field<double>(ctl, OFF_NACC);
   return (kz && slot >= 0 && slot < cap) ? kz + (u64)slot * 2 * NS * N : nullptr;
 }
 // SOL: the step's solution only (a replay along recorded accepted steps needs no error norm).
@@ -826,28 +832,28 @@ __device__ __noinline__ double attempt_error_fp64(const double* __restrict__ U,
 }
 #endif
 template <bool HE, int MODE, bool PAIRS, int MINB>
-__device__ __forceinline__ void attempt_body(const unsigned char* __restrict__ ctl,
-    double* __restrict__ U0, double* __restrict__ U1, const double* __restrict__ kr,
-    const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,
-    double rtol, double atol, int clamp, double* __restrict__ F0, double* __restrict__ F1) {
+__device__ __forceinline__ void attempt_body(const unsigned char* ctl, double* U0, double* U1,
+    const double* __restrict__ kr, const double* __restrict__ em, double* partial, int nc, int nsp,
+    double rtol, double atol, int clamp, double* F0, double* F1) {
   __shared__ double red[256];
 #if !RS_STRICT
   // Programmatic launch: this grid was launched while the controller before it still ran, and lets the
   // controller after it be launched now, which waits here in turn: the launches' latency is hidden
-  // (the 600 s window of 36x18x10: 7.71 -> 7.54 ms).
+  // (the 600 s window of 36x18x10: 7.71 -> 7.54 ms).  Until the wait the record, the states and F may
+  // still change, so none of them is a __restrict__ pointer; kr and em are written before any overlap.
   asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 #endif
-  if (*(const int*)(ctl + OFF_DONE)) return;
-  const double dt = *(const double*)(ctl + OFF_DTC);
-  const double dto2 = *(const double*)(ctl + OFF_DTO2);
-  const double dto6 = *(const double*)(ctl + OFF_DTO6);
-  const double dtg = *(const double*)(ctl + OFF_DTG);
-  const int cur = *(const int*)(ctl + OFF_CUR);
-  const double iters = *(const double*)(ctl + OFF_ITERS);
-  const double* __restrict__ U = cur ? U1 : U0;
-  double* __restrict__ Un = cur ? U0 : U1;
-  double* __restrict__ Fin = cur ? F1 : F0;
-  double* __restrict__ Fout = cur ? F0 : F1;
+  if (ctl_field<int>(ctl, OFF_DONE)) return;
+  const double dt = ctl_field<double>(ctl, OFF_DTC);
+  const double dto2 = ctl_field<double>(ctl, OFF_DTO2);
+  const double dto6 = ctl_field<double>(ctl, OFF_DTO6);
+  const double dtg = ctl_field<double>(ctl, OFF_DTG);
+  const int cur = ctl_field<int>(ctl, OFF_CUR);
+  const double iters = ctl_field<double>(ctl, OFF_ITERS);
+  const double* U = cur ? U1 : U0;
+  double* Un = cur ? U0 : U1;
+  double* Fin = cur ? F1 : F0;
+  double* Fout = cur ? F0 : F1;
   double* __restrict__ kzo = stage_slot(ctl, (u64)nc);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const u64 N = (u64)nc;
@@ -975,11 +981,9 @@ __device__ __forceinline__ void per_cell_body(int nc, int nsp, double* __restric
 
 #define RS_ATTEMPT(NAME, HE, MODE, MINB, PAIRS)                                                  \
   extern "C" __global__ void __launch_bounds__(256, MINB) NAME(                             \
-      const unsigned char* __restrict__ ctl, double* __restrict__ U0,                       \
-      double* __restrict__ U1, const double* __restrict__ kr,                               \
-      const double* __restrict__ em, double* __restrict__ partial, int nc, int nsp,         \
-      double rtol, double atol, int clamp, double* __restrict__ F0,                         \
-      double* __restrict__ F1) {                                                            \
+      const unsigned char* ctl, double* U0, double* U1, const double* __restrict__ kr,      \
+      const double* __restrict__ em, double* partial, int nc, int nsp, double rtol,         \
+      double atol, int clamp, double* F0, double* F1) {                                     \
     attempt_body<HE, MODE, PAIRS, MINB>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
                            F1);                                                             \
   }

@@ -162,6 +162,9 @@ struct StageSel {
   double g;
 };
 // Start of a kernel that `behind` launches: waits for the grid before it, lets the next one be launched.
+// What the grids before it write (the controller record, states, partial sums) may change until
+// then, so no kernel that calls this takes those by __restrict__ pointers: those promise memory that
+// is read-only for the whole kernel, and loads through them may move above the wait.
 __device__ __forceinline__ void await_previous() {
 #if !RS_STRICT
   asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
@@ -1604,10 +1607,8 @@ __global__ void k_scale_fluxes(DevTransport<double> T, double* __restrict__ mx6,
 
 // split the attempt's input state U[cur] (stage 1's RHS argument) into hi/lo planes
 __global__ void __launch_bounds__(kRedThreads) k_split_input(DevTransport<double> T,
-                                                             const Ctl* __restrict__ ctl,
-                                                             const double* __restrict__ U0,
-                                                             const double* __restrict__ U1,
-                                                             const double* __restrict__ Qd) {
+                                                             const Ctl* ctl, const double* U0,
+                                                             const double* U1, const double* Qd) {
   const double* U;
   await_previous();
   if (ctl) {
@@ -1742,7 +1743,7 @@ static void launch_pbl_mean(cudaStream_t st, const DevTransport<double>& T, cons
 //   4: unew = S3 + dt/2 f(S3); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage(DevTransport<double> T,
-                                                       const Ctl* __restrict__ ctl,
+                                                       const Ctl* ctl,
                                                        TransportBufs B, double rtol,
                                                        double atol, int clamp) {
   __shared__ double sm[kRedThreads];
@@ -1908,7 +1909,7 @@ __device__ __forceinline__ void add_error(double err, double am, double rtol, do
 //   4: unew = P + dt/2 f(P); err = 1/2 ((U - u3) / 3 + (u3 - unew)); candidate = clamp(unew)
 template <int STAGE>
 __global__ void __launch_bounds__(kRedThreads) k_stage_mixed(DevTransport<double> T,
-                                                             const Ctl* __restrict__ ctl,
+                                                             const Ctl* ctl,
                                                              TransportBufs B, double rtol,
                                                              double atol, int clamp) {
   __shared__ double sm[kRedThreads];
