@@ -72,7 +72,7 @@ struct DevTransport {
   const double* mys6;  // and the cell north of it
   const double* mdiv;  // [nc] the air-mass flux divergence at time factor 1
   // mixed precision (compensated FP32): the RHS input split into hi, lo planes [ntr][nc]
-  // (hi + lo = q to 2^-47), the vertical coefficients (twice the slopes', half the edges' slope
+  // (hi + lo = q to 2^-49), the vertical coefficients (twice the slopes', half the edges' slope
   // terms) and the air-mass face fluxes as hi and lo planes (mx12 .. mys12: mx6 .. mys6 / 2), and
   // the accumulator of -m dq/dt / g per cell
   float* qhi;
