@@ -781,7 +781,7 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
     fits = fits && fabsf(q.h) < 0x1p60f;
     sum = pair_add(sum, pair_mul(q, q));
   }
-  return fits && big < kPairBig && at0.h >= 0x1p-100f ? pair_to_d(sum) * (dto6 * dto6) : -1.0;
+  return fits && big < kPairBig ? pair_to_d(sum) * (dto6 * dto6) : -1.0;
   } else {
 )" << store_un;
     g.lu_solve("b");
@@ -1733,18 +1733,23 @@ int jit_attempt_block(int nc) {
 // us on 111,555).
 int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.attempt[2][0] ? 2 : 0; }
 
-// Up to one warp per SM sub-partition (152 SMs, four each) the attempt's time is its FP64 chain: W in
-// registers and the FP64 norm, whatever variant is set (6,480 cells: 40 us per attempt, 45 with the
-// float-pair norm).  Beyond, the pairs win (615,888 cells: 1,070 us with the FP64 norm, 981 with
-// pairs, both with 128 registers).
-static bool attempt_fp64_norm(int nc) { return nc <= 152 * 128; }
+// Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set:
+// - up to one warp per SM sub-partition (152 SMs, four each), where its time is its FP64 chain (6,480
+//   cells: 40 us per attempt, 45 with the float-pair norm); beyond, the pairs win (615,888 cells:
+//   1,070 us with the FP64 norm, 981 with pairs, both with 128 registers);
+// - at tolerances that the pairs do not resolve: the split of values below 2^-74 keeps 24 bits, which
+//   is out of sight only while such an error is far below atol; outside these bounds the pairs would
+//   also send cell after cell to the FP64 form, the attempt twice.
+static bool attempt_fp64_norm(int nc, double rtol, double atol) {
+  return nc <= 152 * 128 || !(atol >= 0x1p-40 && atol <= 0x1p100 && rtol >= 0x1p-60 && rtol <= 0x1p60);
+}
 
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                         double* U0, double* U1, const double* kr, const double* em,
                         double* part, double rtol, double atol, int clamp, double* F0,
                         double* F1) {
   const int v = J.attempt[J.variant][0] ? J.variant : 0;
-  const bool small = attempt_fp64_norm(nc);
+  const bool small = attempt_fp64_norm(nc, rtol, atol);
   cudaKernel_t k = small ? J.small[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
   if (!F0 || !F1) F0 = F1 = nullptr;

@@ -1,7 +1,8 @@
 """The float-pair error estimate of a chemistry attempt at the edges of its range, against the table
 kernels' FP64 estimate of the same attempt (same bound as in the middle of the range: 1e-11 relative
 and 2^-45 of the norm of dt f, what the cancelling FP64 sum itself loses).  Quotients above 2^64,
-whose squares are beyond FP32, come from a tolerance far below the error."""
+whose squares are beyond FP32, come from a tolerance far below the error; states and absolute
+tolerances of some 1e-27 lie where a pair's low part runs out of FP32's exponents."""
 import numpy as np
 import pytest
 
@@ -38,3 +39,9 @@ def _check(scale, dt, rtol, atol):
 @pytest.mark.parametrize("dt", [60.0, 300.0])
 def test_quotients_beyond_fp32_squares(rtol, atol, dt):
     assert _check(1.0, dt, rtol, atol) > 2.0 ** 64
+
+
+@pytest.mark.parametrize("scale,atol", [(1e-15, 1e-24), (1e-18, 1e-27), (1e-20, 1e-29), (1e-16, 1e-35)])
+@pytest.mark.parametrize("dt", [1.0, 60.0])
+def test_small_states_and_tolerances(scale, atol, dt):
+    _check(scale, dt, 1e-4, atol)
