@@ -398,6 +398,7 @@ rs_status rs_adjoint_reset_grad(rs_handle* h);
 /* One unclamped Rosenbrock23 attempt of step dt over all cells, reading d_u_in and writing
  * d_u_out (DEVICE pointers, the grid-SoA layout of rs_state_device_ptr, n = the handle's
  * state size), returning the hairer error estimate in *eest (host pointer, may be NULL).
+ * d_u_out may be d_u_in (the attempt in place); buffers that overlap otherwise may not be passed.
  * No counterpart in the reference.  It allocates nothing, for callers that cannot allocate
  * device memory when they step (a host whose own memory pool owns the device, or a loop that
  * must not synchronise on an allocation): its scratch is a 524,800-byte array fixed in the

@@ -1415,7 +1415,7 @@ std::string generate_wide(const MechTables& T, double ros_d, double ros_c32, boo
   if (!per_cell) {
     o << R"(#define LDK(r) double K##r; asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(K##r) : "l"(kr + (u64)(r) * N + c));
 extern "C" __global__ void __launch_bounds__(256, 1) rs_wide_attempt(
-    const unsigned char* __restrict__ ctl, double* __restrict__ U0, double* __restrict__ U1,
+    const unsigned char* __restrict__ ctl, double* U0, double* U1,
     const double* __restrict__ kr, const double* __restrict__ em, double* __restrict__ partial,
     int nc, int nsp, double rtol, double atol, int clamp) {
   extern __shared__ double wsm[];
@@ -1425,8 +1425,8 @@ extern "C" __global__ void __launch_bounds__(256, 1) rs_wide_attempt(
   const double dt = *(const double*)(ctl + OFF_DTC), dto2 = *(const double*)(ctl + OFF_DTO2);
   const double dto6 = *(const double*)(ctl + OFF_DTO6), dtg = *(const double*)(ctl + OFF_DTG);
   const int cur = *(const int*)(ctl + OFF_CUR);
-  const double* __restrict__ U = cur ? U1 : U0;
-  double* __restrict__ Un = cur ? U0 : U1;
+  const double* U = cur ? U1 : U0;
+  double* Un = cur ? U0 : U1;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const u64 N = (u64)nc;
   double e = 0.0;
@@ -1739,7 +1739,9 @@ int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.a
 //   1,070 us with the FP64 norm, 981 with pairs, both with 128 registers);
 // - at tolerances that the pairs do not resolve: the split of values below 2^-74 keeps 24 bits, which
 //   is out of sight only while such an error is far below atol; outside these bounds the pairs would
-//   also send cell after cell to the FP64 form, the attempt twice.
+//   also send cell after cell to the FP64 form, the attempt twice;
+// - in place (one buffer for both states): a cell whose values leave the pairs' range reads its input
+//   again, after its new state is stored.
 static bool attempt_fp64_norm(int nc, double rtol, double atol) {
   return nc <= 152 * 128 || !(atol >= 0x1p-40 && atol <= 0x1p100 && rtol >= 0x1p-60 && rtol <= 0x1p60);
 }
@@ -1749,7 +1751,7 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
                         double* part, double rtol, double atol, int clamp, double* F0,
                         double* F1) {
   const int v = J.attempt[J.variant][0] ? J.variant : 0;
-  const bool small = attempt_fp64_norm(nc, rtol, atol);
+  const bool small = attempt_fp64_norm(nc, rtol, atol) || U0 == U1;
   cudaKernel_t k = small ? J.small[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
   if (!F0 || !F1) F0 = F1 = nullptr;
