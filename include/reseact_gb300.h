@@ -262,7 +262,9 @@ rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len);
  * table-walking per-cell kernel at 32 registers), "per_cell_wide" (1: the straight-line per-cell
  * kernel of a large mechanism, where built; the other per-cell keys select the table-walking
  * kernels); "chem_attempt_variant" (0 "regs", 1 "smem",
- * 2 "regs2", 3 "split": how the specialised attempt kernel keeps W, where built).  Values outside a key's
+ * 2 "regs2", 3 "split": how the specialised attempt kernel keeps W, where built; in the production build
+ * the choice counts for grids above 19,456 cells and tolerances atol_C 2^-40 .. 2^100, rtol_C 2^-60 .. 2^60, and
+ * all others run one form with an FP64 error norm, "fp64_norm").  Values outside a key's
  * candidates are RS_ERR_INVALID.  Every shape gives bit-identical results. */
 rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
 
@@ -280,7 +282,8 @@ rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
  * RS_ERR_UNSUPPORTED for SPECIALIZED when it could not be built (reason in rs_last_error). */
 enum { RS_CHEM_KERNEL_AUTO = 0, RS_CHEM_KERNEL_TABLE = 1, RS_CHEM_KERNEL_SPECIALIZED = 2 };
 rs_status rs_set_chem_kernel(rs_handle* h, int32_t kind);
-/* The kernel kind in use (TABLE or SPECIALIZED) and a one-line JSON description of it. */
+/* The kernel kind in use (TABLE or SPECIALIZED) and a one-line JSON description of it: of a specialised
+ * kernel the variant that is set ("variant") and the form that attempts run ("runs", "runs_regs"). */
 rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info, size_t info_len);
 /* Staging of the mixed-precision transport pencils (no reference counterpart).  Beside the
  * pencils, the mixed transport has streaming forms without shared memory (a warp of shuffles

@@ -2079,14 +2079,19 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
       for (char& ch : why)
         if (ch == '"' || ch == '\\' || ch == '\n') ch = ' ';
       char line[768];
-      if (h->jit)
+      if (h->jit) {
+        const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
+        const int v = h->jit->variant;
         std::snprintf(line, sizeof line,
-                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"regs\": [%d, %d, %d, %d], "
+                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"runs\": \"%s\", \"runs_regs\": %d, "
+                      "\"regs\": [%d, %d, %d, %d], "
                       "\"smem_bytes\": %zu, \"split_smem_bytes\": %zu, \"compile_ms\": %.1f}",
-                      spec ? "specialized" : "table", rs::kJitVariantNames[h->jit->variant],
+                      spec ? "specialized" : "table", rs::kJitVariantNames[v],
+                      !spec ? "table" : (f64 ? "fp64_norm" : rs::kJitVariantNames[v]),
+                      !spec ? 0 : (f64 ? h->jit->fp64_norm_regs : h->jit->regs[v]),
                       h->jit->regs[0], h->jit->regs[1], h->jit->regs[2], h->jit->regs[3],
                       h->jit->attempt_smem[1], h->jit->attempt_smem[3], h->jit->compile_ms);
-      else
+      } else
         std::snprintf(line, sizeof line, "{\"kind\": \"table\", \"wide\": %s, \"why\": \"%.600s\"}",
                       h->lc.wide ? "true" : "false", why.c_str());
       std::strncpy(info, line, info_len - 1);
@@ -2558,28 +2563,33 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
     }
     if (h->cfg.do_chemistry && h->cfg.chem_mode == RS_CHEM_GLOBAL_DT && h->lc.jit) {
       // variants of the specialised attempt kernel: one attempt from the accepted state into
-      // the candidate buffer (the accepted state is untouched)
+      // the candidate buffer (the accepted state is untouched).  Where the form with the FP64 norm
+      // runs whatever is set, there is nothing to choose: its one time stands for all of them.
+      const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
+      const int was = h->jit->variant;
       Ctl init = make_ctl(h, 0.0, 600.0, 60.0, h->cfg.ctrl_C, (double)h->nc * h->nsp);
       init.cur = h->cur;
       Ctl* c = h->ctl.p + 2;
       rs::launch_ctl_init(h->st, c, init);
-      float best = 1e30f;
-      int pick = 0;
+      float best = 1e30f, ms = 0.0f;
+      int pick = was;
       bool first = true;
       rep += std::string(rep.size() > 1 ? ", " : "") + "\"chem_attempt\": [";
       for (int v = 0; v < rs::kJitVariants; ++v) {
         if (!h->jit->attempt[v][0]) continue;
         h->jit->variant = v;
-        float ms = time_min(h->st, 3, [&] {
-          rs::launch_ros23_attempt(h->lc, c, h->U[0].p, h->U[1].p, h->krates.p,
-                                   h->have_emis ? h->emis.p : nullptr, h->partial.p,
-                                   h->cfg.rtol_C, h->cfg.atol_C, h->cfg.clamp_nonneg);
-        });
-        std::snprintf(line, sizeof line, "%s{\"variant\": \"%s\", \"regs\": %d, \"ms\": %.4f}",
-                      first ? "" : ", ", rs::kJitVariantNames[v], h->jit->regs[v], ms);
+        if (first || !f64)
+          ms = time_min(h->st, 3, [&] {
+            rs::launch_ros23_attempt(h->lc, c, h->U[0].p, h->U[1].p, h->krates.p,
+                                     h->have_emis ? h->emis.p : nullptr, h->partial.p,
+                                     h->cfg.rtol_C, h->cfg.atol_C, h->cfg.clamp_nonneg);
+          });
+        std::snprintf(line, sizeof line, "%s{\"variant\": \"%s\", \"regs\": %d, \"runs\": \"%s\", \"ms\": %.4f}",
+                      first ? "" : ", ", rs::kJitVariantNames[v], f64 ? h->jit->fp64_norm_regs : h->jit->regs[v],
+                      f64 ? "fp64_norm" : rs::kJitVariantNames[v], ms);
         rep += line;
         first = false;
-        if (ms < best) {
+        if (!f64 && ms < best) {
           best = ms;
           pick = v;
         }

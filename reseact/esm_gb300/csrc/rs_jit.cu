@@ -990,7 +990,7 @@ __device__ __forceinline__ void per_cell_body(int nc, int nsp, double* __restric
                            F1);                                                             \
   }
 #define RS_PAIRS (!RS_STRICT)
-#if RS_IN(1)
+#if RS_IN(1) && !RS_STRICT
 RS_ATTEMPT(rs_jit_attempt_l0, false, 0, 1, false)
 RS_ATTEMPT(rs_jit_attempt_l1, true, 0, 1, false)
 #endif
@@ -1669,7 +1669,7 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
       *why = std::string("cudaLibraryGetKernel(") + name + "): " + cudaGetErrorString(e);
     return e == cudaSuccess;
   };
-  bool ok = get(&J->small[0], "rs_jit_attempt_l0") && get(&J->small[1], "rs_jit_attempt_l1") &&
+  bool ok = (strict || (get(&J->fp64_norm[0], "rs_jit_attempt_l0") && get(&J->fp64_norm[1], "rs_jit_attempt_l1"))) &&
             get(&J->attempt[0][0], "rs_jit_attempt_r0") && get(&J->attempt[0][1], "rs_jit_attempt_r1") &&
             get(&J->attempt[2][0], "rs_jit_attempt_q0") && get(&J->attempt[2][1], "rs_jit_attempt_q1") &&
             get(&J->per_cell[0], "rs_jit_per_cell_0") && get(&J->per_cell[1], "rs_jit_per_cell_1") &&
@@ -1708,6 +1708,9 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
     else
       cudaGetLastError();
   }
+  cudaFuncAttributes fa{};
+  if (J->fp64_norm[0] && cudaFuncGetAttributes(&fa, (const void*)J->fp64_norm[0]) == cudaSuccess)
+    J->fp64_norm_regs = fa.numRegs;
   why->clear();
   return J;
 }
@@ -1733,7 +1736,8 @@ int jit_attempt_block(int nc) {
 // us on 111,555).
 int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.attempt[2][0] ? 2 : 0; }
 
-// Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set:
+// Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set (the
+// strict build has no other norm and runs the variant that is set):
 // - up to one warp per SM sub-partition (152 SMs, four each), where its time is its FP64 chain (6,480
 //   cells: 40 us per attempt, 45 with the float-pair norm); beyond, the pairs win (615,888 cells:
 //   1,070 us with the FP64 norm, 981 with pairs, both with 128 registers);
@@ -1742,7 +1746,8 @@ int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.a
 //   also send cell after cell to the FP64 form, the attempt twice;
 // - in place (one buffer for both states): a cell whose values leave the pairs' range reads its input
 //   again, after its new state is stored.
-static bool attempt_fp64_norm(int nc, double rtol, double atol) {
+bool jit_fp64_norm(const JitChem& J, int nc, double rtol, double atol) {
+  if (!J.fp64_norm[0]) return false;
   return nc <= 152 * 128 || !(atol >= 0x1p-40 && atol <= 0x1p100 && rtol >= 0x1p-60 && rtol <= 0x1p60);
 }
 
@@ -1751,8 +1756,8 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
                         double* part, double rtol, double atol, int clamp, double* F0,
                         double* F1) {
   const int v = J.attempt[J.variant][0] ? J.variant : 0;
-  const bool small = attempt_fp64_norm(nc, rtol, atol) || U0 == U1;
-  cudaKernel_t k = small ? J.small[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
+  const bool fp64 = jit_fp64_norm(J, nc, rtol, atol) || (J.fp64_norm[0] && U0 == U1);
+  cudaKernel_t k = fp64 ? J.fp64_norm[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);
   if (!F0 || !F1) F0 = F1 = nullptr;
   void* args[] = {&c, &U0, &U1, &kr, &em, &part, &nc, &nsp, &rtol, &atol, &clamp, &F0, &F1};
@@ -1760,7 +1765,7 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((nc + block - 1) / block);
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = small ? 0 : J.attempt_smem[v];
+  cfg.dynamicSmemBytes = fp64 ? 0 : J.attempt_smem[v];
   cfg.stream = st;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

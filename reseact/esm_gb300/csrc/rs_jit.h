@@ -32,7 +32,8 @@ extern const char* const kJitVariantNames[kJitVariants];
 
 struct JitChem {
   cudaKernel_t attempt[kJitVariants][2] = {};  // [variant][has emission]; null: not built
-  cudaKernel_t small[2] = {};                  // grids of up to a warp per SM sub-partition
+  cudaKernel_t fp64_norm[2] = {};              // production build: the attempt of jit_fp64_norm
+  int fp64_norm_regs = 0;
   cudaKernel_t per_cell[2] = {};               // [has emission]
   cudaKernel_t rcp = nullptr;                  // elementwise production reciprocal
   cudaKernel_t vjp[2] = {};                    // ROS23 step VJP [has emission]
@@ -65,6 +66,8 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
 int jit_attempt_block(int nc);
 // The attempt variant for nc cells before the autotuner or the caller picks one.
 int jit_default_variant(const JitChem& J, int nc);
+// Whether attempts run the form with the FP64 norm, whatever variant is set.
+bool jit_fp64_norm(const JitChem& J, int nc, double rtol, double atol);
 
 // Same contracts as launch_ros23_attempt / launch_chem_per_cell in rs_kernels.h.
 void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
