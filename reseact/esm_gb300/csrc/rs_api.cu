@@ -2083,12 +2083,13 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
         const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
         const int v = h->jit->variant;
         std::snprintf(line, sizeof line,
-                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"runs\": \"%s\", \"runs_regs\": %d, "
+                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"runs\": \"%s\", \"runs_regs\": %d, \"runs_smem_bytes\": %zu, "
                       "\"regs\": [%d, %d, %d, %d], "
                       "\"smem_bytes\": %zu, \"split_smem_bytes\": %zu, \"compile_ms\": %.1f}",
                       spec ? "specialized" : "table", rs::kJitVariantNames[v],
                       !spec ? "table" : (f64 ? "fp64_norm" : rs::kJitVariantNames[v]),
                       !spec ? 0 : (f64 ? h->jit->fp64_norm_regs : h->jit->regs[v]),
+                      !spec || f64 ? (size_t)0 : rs::jit_attempt_smem(*h->jit, v, (int)h->nc),
                       h->jit->regs[0], h->jit->regs[1], h->jit->regs[2], h->jit->regs[3],
                       h->jit->attempt_smem[1], h->jit->attempt_smem[3], h->jit->compile_ms);
       } else

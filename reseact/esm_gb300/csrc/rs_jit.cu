@@ -660,8 +660,9 @@ __device__ __forceinline__ double* stage_slot(const unsigned char* ctl, u64 N) {
 }
 // SOL: the step's solution only (a replay along recorded accepted steps needs no error norm).
 // W storage: LU slots e < KR in the register array W, the others in shared memory at
-// WSM[(e - KR) * 256] (this thread's column of a [slot][thread] array); every slot index is a
-// compile-time constant, so each access resolves to one of the two when compiled.
+// WSM[(e - KR) * 64] (this thread's column of a [slot][thread] array per 64 threads of the block, see
+// w_column); every slot index is a compile-time constant, so each access resolves to one of the two
+// when compiled.
 // un, fin (may be null): where the clamped new state and, unless have_f0, f(x) go in global
 // memory -- written as soon as they are final, so that neither stays live through the error solve.
 // PAIRS: the error estimate in float pairs; returns a negative value where the pairs' range does
@@ -675,7 +676,7 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
     double* __restrict__ fin = nullptr) {
 #define K(r) __ldg(kr + (u64)(r) * N + c)
 #define EM(s) __ldg(em + (u64)(s) * N + c)
-#define WV(e) (*((e) < KR ? &W[(e)] : &WSM[((e) - KR) * 256]))
+#define WV(e) (*((e) < KR ? &W[(e)] : &WSM[((e) - KR) * 64]))
   RS_VDECL
   double P[NPA], k1[NS], f1[NS], k2[NS], b[NS], pv[NS];
   if (!have_f0) {
@@ -833,6 +834,11 @@ __device__ __noinline__ double attempt_error_fp64(const double* __restrict__ U,
                                     nullptr, dt, dto2, dto6, dtg, rtol, atol, nullptr);
 }
 #endif
+// a thread's column of the shared part of W: 64 threads to a [slot][thread] array, so that a warp's
+// accesses are contiguous, the strides constants and the shared memory that of the block's own threads
+__device__ __forceinline__ double* w_column(double* wsm, int slots) {
+  return wsm + (threadIdx.x >> 6) * (slots * 64) + (threadIdx.x & 63u);
+}
 template <bool HE, int MODE, bool PAIRS, int MINB>
 __device__ __forceinline__ void attempt_body(const unsigned char* ctl, double* U0, double* U1,
     const double* __restrict__ kr, const double* __restrict__ em, double* partial, int nc, int nsp,
@@ -875,13 +881,13 @@ __device__ __forceinline__ void attempt_body(const unsigned char* ctl, double* U
     }
     if constexpr (MODE == 1) {
       extern __shared__ double wsm[];
-      e = ros23_cell<HE, 0, false, false, PAIRS>(kr, em, N, c, x, xn, nullptr, wsm + threadIdx.x, f0, have,
+      e = ros23_cell<HE, 0, false, false, PAIRS>(kr, em, N, c, x, xn, nullptr, w_column(wsm, NLU), f0, have,
                                    F0 ? Fout : nullptr, clamp, nullptr, dt, dto2, dto6, dtg,
                                    rtol, atol, kzo, Un, F0 ? Fin : nullptr);
     } else if constexpr (MODE == 2) {
       extern __shared__ double wsm[];
       double W[NLU_R > 0 ? NLU_R : 1];
-      e = ros23_cell<HE, NLU_R, false, false, PAIRS>(kr, em, N, c, x, xn, W, wsm + threadIdx.x, f0, have,
+      e = ros23_cell<HE, NLU_R, false, false, PAIRS>(kr, em, N, c, x, xn, W, w_column(wsm, NLU - NLU_R), f0, have,
                                        F0 ? Fout : nullptr, clamp, nullptr, dt, dto2, dto6,
                                        dtg, rtol, atol, kzo, Un, F0 ? Fin : nullptr);
     } else {
@@ -1730,6 +1736,13 @@ int jit_attempt_block(int nc) {
 #endif
 }
 
+// The shared part of W of a block's own threads.  (Laid out for 256 threads in blocks of 64 or 128, it
+// left half to three quarters of an SM's shared memory unused: "smem" 351 -> 129 us on 76,183 cells and
+// 1,331 -> 967 on 615,888, "split" 182 -> 148 and 1,063 -> 943.)
+size_t jit_attempt_smem(const JitChem& J, int variant, int nc) {
+  return J.attempt_smem[variant] / kBlock * jit_attempt_block(nc);
+}
+
 // The attempt variant a handle starts with: 128 registers and 16 warps per SM ("regs2") hide the
 // spills' latency once the grid fills them (1,042 us per call against 1,145 with 255 registers on
 // 615,888 cells, 348 against 364 on 155,664); below, their last wave is too coarse (285 against 259
@@ -1765,7 +1778,7 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((nc + block - 1) / block);
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = fp64 ? 0 : J.attempt_smem[v];
+  cfg.dynamicSmemBytes = fp64 ? 0 : jit_attempt_smem(J, v, nc);
   cfg.stream = st;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -39,7 +39,7 @@ struct JitChem {
   cudaKernel_t vjp[2] = {};                    // ROS23 step VJP [has emission]
   cudaKernel_t step[2] = {};                   // accepted step, no error estimate [has emission]
   cudaKernel_t vjpk[2] = {};                   // step VJP reading k1, z2 from the stage tape
-  size_t attempt_smem[kJitVariants] = {};  // dynamic shared bytes of each attempt variant
+  size_t attempt_smem[kJitVariants] = {};  // dynamic shared bytes of each attempt variant, 256 threads
   int variant = 0;          // variant used for global-dt attempts
   double compile_ms = 0;    // NVRTC time (0 when the compiled image came from cache)
   int regs[kJitVariants] = {};  // registers per thread of each attempt variant
@@ -64,6 +64,8 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
 
 // Threads per block of the attempt kernels over nc cells (one partial sum per block).
 int jit_attempt_block(int nc);
+// Dynamic shared bytes per block of a variant over nc cells.
+size_t jit_attempt_smem(const JitChem& J, int variant, int nc);
 // The attempt variant for nc cells before the autotuner or the caller picks one.
 int jit_default_variant(const JitChem& J, int nc);
 // Whether attempts run the form with the FP64 norm, whatever variant is set.

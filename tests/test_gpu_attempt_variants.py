@@ -61,6 +61,16 @@ def test_autotuned_variant_is_bitwise_neutral(n):
     assert np.array_equal(res[0][0], res[1][0]) and res[0][1] == res[1][1]
 
 
+@pytest.mark.parametrize("n,threads", list(zip(LARGE, (64, 128))))
+def test_shared_memory_is_that_of_the_blocks_threads(n, threads):
+    s = Solver.for_workload(_work(n), do_transport=False)
+    for v, key in ((1, "smem_bytes"), (3, "split_smem_bytes")):
+        s.set_launch_shape(chem_attempt_variant=v)
+        info = s.chem_kernel()[1]
+        assert info["runs_smem_bytes"] == info[key] * threads // 256  # smem_bytes: 256 threads
+    s.close()
+
+
 def test_small_grid_says_what_runs():
     w = _work(SMALL)
     s = Solver.for_workload(w)
