@@ -29,12 +29,12 @@
 #include <mutex>
 #include <sstream>
 #include <string>
-#include <thread>
 #include <type_traits>
 #include <vector>
 
 #include "rs_jit.h"
 #include "rs_kernels.h"
+#include "rs_units.h"
 
 namespace rs {
 
@@ -1598,18 +1598,15 @@ bool compile_and_load(const std::string& src, bool strict, int units, Compiled* 
   auto t0 = std::chrono::steady_clock::now();
   const int n = std::max(1, units);
   std::vector<std::vector<char>> cubin(n);
-  std::vector<std::string> log(n);
+  std::vector<std::string> log(n), thrown;
   std::vector<char> ok(n, 0);
-  std::vector<std::thread> work;
-  for (int u = 1; u < n; ++u)
-    work.emplace_back([&, u] { ok[u] = jit_compile(src, strict, false, &cubin[u], &log[u], u + 1); });
-  ok[0] = jit_compile(src, strict, false, &cubin[0], &log[0], units ? 1 : 0);
-  for (auto& t : work) t.join();
-  for (int u = 0; u < n; ++u) {
+  run_units(n, [&](int u) { ok[u] = jit_compile(src, strict, false, &cubin[u], &log[u], units ? u + 1 : 0); }, &thrown);
+  for (int u = 0; u < n; ++u)
     if (!ok[u]) {
-      *why = log[u].substr(0, 4000);
+      *why = (thrown[u].empty() ? log[u] : "compiling a unit: " + thrown[u]).substr(0, 4000);
       return false;
     }
+  for (int u = 0; u < n; ++u) {
     cudaLibrary_t lib = nullptr;
     cudaError_t e = cudaLibraryLoadData(&lib, cubin[u].data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e != cudaSuccess) {
