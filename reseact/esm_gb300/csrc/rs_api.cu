@@ -1050,7 +1050,6 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
     h->lc = rs::LaunchCtx{h->st, h->dm, (int)h->nc, h->nsp, cls};
     h->jit = rs::jit_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32, RS_STRICT != 0, &h->jit_why);
     h->lc.jit = h->jit.get();
-    if (h->jit) h->jit->variant = rs::jit_default_variant(*h->jit, (int)h->nc);
     if (!h->jit && cfg->do_chemistry) {
       std::string why;
       h->wide = rs::wide_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32,

@@ -1740,12 +1740,6 @@ size_t jit_attempt_smem(const JitChem& J, int variant, int nc) {
   return J.attempt_smem[variant] / kBlock * jit_attempt_block(nc);
 }
 
-// The attempt variant a handle starts with: 128 registers and 16 warps per SM ("regs2") hide the
-// spills' latency once the grid fills them (1,042 us per call against 1,145 with 255 registers on
-// 615,888 cells, 348 against 364 on 155,664); below, their last wave is too coarse (285 against 259
-// us on 111,555).
-int jit_default_variant(const JitChem& J, int nc) { return nc > (1 << 17) && J.attempt[2][0] ? 2 : 0; }
-
 // Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set (the
 // strict build has no other norm and runs the variant that is set):
 // - up to one warp per SM sub-partition (152 SMs, four each), where its time is its FP64 chain (6,480

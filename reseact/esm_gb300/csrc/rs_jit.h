@@ -40,7 +40,11 @@ struct JitChem {
   cudaKernel_t step[2] = {};                   // accepted step, no error estimate [has emission]
   cudaKernel_t vjpk[2] = {};                   // step VJP reading k1, z2 from the stage tape
   size_t attempt_smem[kJitVariants] = {};  // dynamic shared bytes of each attempt variant, 256 threads
-  int variant = 0;          // variant used for global-dt attempts
+  // variant used for global-dt attempts: "regs" until the autotuner or the caller picks one.  It is
+  // the fastest or within 1 % of it on every grid (600 s of chemistry in ms, regs / smem / regs2 /
+  // split: 76,183 cells 2.90 / 2.89 / 3.07 / 3.58; 133,517: 4.43 / 4.37 / 4.96 / 4.67; 211,200: 6.64 /
+  // 6.72 / 7.10 / 6.85; 615,888: 17.08 / 17.08 / 17.45 / 17.06)
+  int variant = 0;
   double compile_ms = 0;    // NVRTC time (0 when the compiled image came from cache)
   int regs[kJitVariants] = {};  // registers per thread of each attempt variant
 };
@@ -66,8 +70,6 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
 int jit_attempt_block(int nc);
 // Dynamic shared bytes per block of a variant over nc cells.
 size_t jit_attempt_smem(const JitChem& J, int variant, int nc);
-// The attempt variant for nc cells before the autotuner or the caller picks one.
-int jit_default_variant(const JitChem& J, int nc);
 // Whether attempts run the form with the FP64 norm, whatever variant is set.
 bool jit_fp64_norm(const JitChem& J, int nc, double rtol, double atol);
 

@@ -71,6 +71,13 @@ def test_shared_memory_is_that_of_the_blocks_threads(n, threads):
     s.close()
 
 
+@pytest.mark.parametrize("n", LARGE)
+def test_a_handle_starts_with_w_in_registers(n):
+    s = Solver.for_workload(_work(n), do_transport=False)
+    assert s.chem_kernel()[1]["runs"] == "regs"
+    s.close()
+
+
 def test_small_grid_says_what_runs():
     w = _work(SMALL)
     s = Solver.for_workload(w)
