@@ -2547,10 +2547,16 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
                                    h->have_emis ? h->emis.p : nullptr, h->io.p, nullptr, h->queue.p,
                                    h->flag.p, a);
         });
-        // three attempts per cell fit the table-walking kernels, whose 2,048 threads per SM then
-        // all finish together; over a whole window with uneven step counts their warps run as
-        // long as their slowest cell, so the straight-line kernel is kept unless it is far behind
-        h->tune.pc_wide = ms < 2.0f * best;
+        // Three attempts of every cell show what a full device does; a window ends with its slowest
+        // cells, whose attempts several lanes finish sooner the emptier the device is (the
+        // straight-line kernel's last cell takes as long as its first).  So where lanes per cell win
+        // among the table-walking kernels, batches below 50 cells per SM keep them.  60 s windows of
+        // 30 / 44 / 64 species in ms, straight-line against lanes per cell: 1,024 cells 8.6 / 19.6 /
+        // 27.4 against 6.0 / 10.1 / 18.6, 4,096: 9.5 / 19.6 / 52.1 against 7.9 / 15.6 / 42.3; 8,192:
+        // 9.9 / 21.5 / 55.5 against 11.9 / 26.0 / 52.8, 16,384: 11.8 / 26.8 / 49.3 against 19.9 / 47.2 /
+        // 58.7.  At 262,144 cells 88 / 222 / 279 against 151 / 306 / 521 of the best table kernel.
+        const bool few = (long long)h->nc < 50LL * nsm && h->tune.pc_group > 0;
+        h->tune.pc_wide = !few && ms < best;
         std::snprintf(line, sizeof line, "], \"per_cell_wide\": [{\"ms\": %.4f}", ms);
         rep += line;
       }
