@@ -428,7 +428,7 @@ struct rs_handle {
   // large for jit (null: not built)
   std::shared_ptr<rs::WideChem> wide;
   DevBuf<double> fsal[2];  // f(U[b]) planes [ns][nc] for the specialised global-dt attempts
-  std::string jit_why;
+  std::string jit_why, wide_why;
   int chem_kernel = RS_CHEM_KERNEL_AUTO;
 };
 
@@ -1051,9 +1051,8 @@ rs_status rs_create(const rs_config* cfg, rs_handle** out) {
     h->jit = rs::jit_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32, RS_STRICT != 0, &h->jit_why);
     h->lc.jit = h->jit.get();
     if (!h->jit && cfg->do_chemistry) {
-      std::string why;
       h->wide = rs::wide_chem_build(h->mt, h->dm.ros_d, h->dm.ros_c32,
-                                    cfg->chem_mode == RS_CHEM_PER_CELL, &why);
+                                    cfg->chem_mode == RS_CHEM_PER_CELL, &h->wide_why);
       h->lc.wide = h->wide.get();
     }
     if (h->jit && cfg->do_chemistry && cfg->chem_mode == RS_CHEM_GLOBAL_DT) {
@@ -2074,10 +2073,11 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
     const bool spec = h->lc.jit != nullptr;
     if (kind) *kind = spec ? RS_CHEM_KERNEL_SPECIALIZED : RS_CHEM_KERNEL_TABLE;
     if (info && info_len) {
-      std::string why = h->jit_why;
-      for (char& ch : why)
-        if (ch == '"' || ch == '\\' || ch == '\n') ch = ' ';
-      char line[768];
+      std::string why = h->jit_why, wide_why = h->wide_why;
+      for (std::string* w : {&why, &wide_why})
+        for (char& ch : *w)
+          if (ch == '"' || ch == '\\' || (unsigned char)ch < 0x20) ch = ' ';
+      char line[1024];
       if (h->jit) {
         const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
         const int v = h->jit->variant;
@@ -2092,8 +2092,9 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
                       h->jit->regs[0], h->jit->regs[1], h->jit->regs[2], h->jit->regs[3],
                       h->jit->attempt_smem[1], h->jit->attempt_smem[3], h->jit->compile_ms);
       } else
-        std::snprintf(line, sizeof line, "{\"kind\": \"table\", \"wide\": %s, \"why\": \"%.600s\"}",
-                      h->lc.wide ? "true" : "false", why.c_str());
+        std::snprintf(line, sizeof line,
+                      "{\"kind\": \"table\", \"wide\": %s, \"wide_why\": \"%.300s\", \"why\": \"%.600s\"}",
+                      h->lc.wide ? "true" : "false", wide_why.c_str(), why.c_str());
       std::strncpy(info, line, info_len - 1);
       info[info_len - 1] = 0;
     }
