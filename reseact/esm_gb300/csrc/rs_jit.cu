@@ -100,6 +100,14 @@ constexpr int kBlock = 256;
 constexpr int kJitUnits = 8;  // RS_IN units of the generated source
 constexpr size_t kSmemCap = 227 * 1024 - kBlock * sizeof(double);
 
+// Whether the global-dt attempts form their error estimate in float pairs.  The pairs' splits and
+// sums take registers: beyond this many LU slots they spill more than the FP64 instructions they save
+// are worth.  Attempt in us, pairs / FP64 estimate (both with W in registers): 94 slots 132 / 136 on
+// 40,960 cells, 315 / 320 on 150,528, 1,126 / 1,181 on 614,400; 122 slots 169 / 171, 394 / 403, 1,616 /
+// 1,524; 162 slots 215 / 212, 535 / 509, 2,266 / 1,926; 242 slots 353 / 300, 886 / 732, 3,676 / 2,791.
+constexpr int kPairSlots = 108;
+bool jit_pairs(const MechTables& T, bool strict) { return !strict && T.nlu <= kPairSlots; }
+
 size_t smem_bytes(const MechTables& T) { return (size_t)T.nlu * kBlock * sizeof(double); }
 // "split" variant: the last split_slots(T) LU slots of W in shared memory, the others in
 // registers, two 256-thread blocks per SM (each block's shared part within half an SM's
@@ -618,7 +626,7 @@ std::string generate(const MechTables& T, double ros_d, double ros_c32, bool str
   const size_t ops = 2 * (T.rhs_r.size() + T.nr) + T.nr + T.npart + T.jac_part.size() + T.upd_dst.size() +
                      T.elim_lik.size() + 2 * T.nlu + 11 * T.ns;
   o << "#define RS_WARP_NS " << ops * 31 << "u\n";
-  o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n" << kPrelude << R"(
+  o << "#define RS_STRICT " << (strict ? 1 : 0) << "\n#define RS_PAIRS " << (jit_pairs(T, strict) ? 1 : 0) << "\n" << kPrelude << R"(
 // The first wave's warps of one SM sub-partition (`depth` of them fit; 152 SMs with four each) start
 // apart, over the FP64 time of one warp (RS_WARP_NS).  Started together they stay in lock step: all
 // load, convert and miss the instruction cache at once and leave the FP64 pipe idle, and they
@@ -995,8 +1003,7 @@ __device__ __forceinline__ void per_cell_body(int nc, int nsp, double* __restric
     attempt_body<HE, MODE, PAIRS, MINB>(ctl, U0, U1, kr, em, partial, nc, nsp, rtol, atol, clamp, F0,    \
                            F1);                                                             \
   }
-#define RS_PAIRS (!RS_STRICT)
-#if RS_IN(1) && !RS_STRICT
+#if RS_IN(1) && RS_PAIRS
 RS_ATTEMPT(rs_jit_attempt_l0, false, 0, 1, false)
 RS_ATTEMPT(rs_jit_attempt_l1, true, 0, 1, false)
 #endif
@@ -1672,7 +1679,7 @@ std::shared_ptr<JitChem> jit_chem_build(const MechTables& T, double ros_d, doubl
       *why = std::string("cudaLibraryGetKernel(") + name + "): " + cudaGetErrorString(e);
     return e == cudaSuccess;
   };
-  bool ok = (strict || (get(&J->fp64_norm[0], "rs_jit_attempt_l0") && get(&J->fp64_norm[1], "rs_jit_attempt_l1"))) &&
+  bool ok = (!jit_pairs(T, strict) || (get(&J->fp64_norm[0], "rs_jit_attempt_l0") && get(&J->fp64_norm[1], "rs_jit_attempt_l1"))) &&
             get(&J->attempt[0][0], "rs_jit_attempt_r0") && get(&J->attempt[0][1], "rs_jit_attempt_r1") &&
             get(&J->attempt[2][0], "rs_jit_attempt_q0") && get(&J->attempt[2][1], "rs_jit_attempt_q1") &&
             get(&J->per_cell[0], "rs_jit_per_cell_0") && get(&J->per_cell[1], "rs_jit_per_cell_1") &&

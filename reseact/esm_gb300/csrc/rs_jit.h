@@ -32,7 +32,7 @@ extern const char* const kJitVariantNames[kJitVariants];
 
 struct JitChem {
   cudaKernel_t attempt[kJitVariants][2] = {};  // [variant][has emission]; null: not built
-  cudaKernel_t fp64_norm[2] = {};              // production build: the attempt of jit_fp64_norm
+  cudaKernel_t fp64_norm[2] = {};              // the attempt of jit_fp64_norm, where the others use pairs
   int fp64_norm_regs = 0;
   cudaKernel_t per_cell[2] = {};               // [has emission]
   cudaKernel_t rcp = nullptr;                  // elementwise production reciprocal

@@ -103,13 +103,20 @@ def test_strict_build_runs_the_variant_that_is_set():
 
 @pytest.mark.parametrize("n,r", [(18, 40), (24, 50)])
 def test_mechanisms_between_the_shared_memory_and_the_straight_line_limits(n, r):
-    """More LU slots than fit in shared memory for 256 threads: no smem variant, still specialised."""
+    """More LU slots than fit in shared memory for 256 threads, and too many for float pairs: no smem
+    variant and no form beside the variants; the others give the same bits."""
     m = mechanism.synthetic(n_species=n, n_reactions=r)
-    w = workloads.c3(ncells=20000, mech=m)
-    s = Solver.for_workload(w, chem_mode=abi.RS_CHEM_GLOBAL_DT)
-    kind, info = s.chem_kernel()
-    assert kind == CHEM_KERNEL_SPECIALIZED, info
-    u = w.u0_cellmajor()
-    a, e = s.single_step(abi.RS_OP_CHEMISTRY, u, 0.0, 1e-3)
-    assert np.isfinite(a).all() and np.isfinite(e)
-    s.close()
+    for ncells in (1024, 20480):
+        w = workloads.c3(ncells=ncells, mech=m)
+        u = w.u0_cellmajor()
+        res = []
+        for v in (0, 2, 3):
+            s = Solver.for_workload(w, chem_mode=abi.RS_CHEM_GLOBAL_DT)
+            assert s.chem_kernel()[0] == CHEM_KERNEL_SPECIALIZED
+            s.set_launch_shape(chem_attempt_variant=v)
+            assert s.chem_kernel()[1]["runs"] == NAMES[v]
+            res.append(s.single_step(abi.RS_OP_CHEMISTRY, u, 0.0, 1e-3))
+            s.close()
+        assert np.isfinite(res[0][0]).all() and res[0][1] > 0.0
+        for a, e in res[1:]:
+            assert np.array_equal(res[0][0], a) and res[0][1] == e
