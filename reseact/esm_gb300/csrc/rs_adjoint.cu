@@ -780,8 +780,6 @@ __global__ void __launch_bounds__(256) k_adj_pencil(DevTransport<double> T,
 #undef AV
 }
 
-#include "rs_adj64.cuh"
-
 // The fused adjoint pencils for all three directions, or false (nothing launched) when a
 // direction's pencils do not fit in shared memory -- the caller then uses the face + gather
 // kernels, which compute the same bits.

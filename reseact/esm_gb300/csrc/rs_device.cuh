@@ -279,8 +279,6 @@ __device__ __forceinline__ void lu_solve(const DevMech& M, const double* W, cons
 // ------------------------------------------------------------------ integer-pipe FP64 helpers
 // Sign tests, magnitude compares and selects of doubles on their bit patterns (the integer
 // pipes; FP64 issues at ~2 lanes per SM per clock on this GPU).
-constexpr long long kMagMask = 0x7fffffffffffffffLL, kSignBit = (long long)0x8000000000000000ULL,
-                    kExpOne = 1LL << 52;
 __device__ __forceinline__ double sel_d(bool c, double x, double y) {
   return __longlong_as_double(c ? __double_as_longlong(x) : __double_as_longlong(y));
 }

@@ -1854,10 +1854,6 @@ std::shared_ptr<WideChem> wide_chem_build(const MechTables& T, double ros_d, dou
   return Wc;
 #endif
 }
-std::string wide_chem_source(const MechTables& T, bool per_cell) {
-  return wide_eligible(T) ? generate_wide(T, 1.0 / (2.0 + std::sqrt(2.0)), 6.0 + std::sqrt(2.0), per_cell)
-                          : std::string();
-}
 void wide_launch_attempt(const WideChem& Wc, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                          double* U0, double* U1, const double* kr, const double* em, double* part,
                          double rtol, double atol, int clamp) {

@@ -101,7 +101,6 @@ struct WideChem {
 // the one kernel asked for, or null and *why
 std::shared_ptr<WideChem> wide_chem_build(const MechTables& T, double ros_d, double ros_c32,
                                           bool per_cell, std::string* why);
-std::string wide_chem_source(const MechTables& T, bool per_cell);  // empty: not eligible
 void wide_launch_attempt(const WideChem& W, cudaStream_t st, int nc, int nsp, const Ctl* ctl,
                          double* U0, double* U1, const double* kr, const double* em, double* part,
                          double rtol, double atol, int clamp);
