@@ -283,8 +283,8 @@ rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
 enum { RS_CHEM_KERNEL_AUTO = 0, RS_CHEM_KERNEL_TABLE = 1, RS_CHEM_KERNEL_SPECIALIZED = 2 };
 rs_status rs_set_chem_kernel(rs_handle* h, int32_t kind);
 /* The kernel kind in use (TABLE or SPECIALIZED) and a one-line JSON description of it: of a specialised
- * kernel the variant that is set ("variant") and the form that attempts run ("runs", "runs_regs",
- * "runs_smem_bytes" per block); without one the reason ("why") and, where the straight-line
+ * kernel the variant that is set ("variant"), the form that attempts of the adaptive loop run ("runs", "runs_regs",
+ * "runs_smem_bytes" per block) and the one of single attempts ("runs_single"); without one the reason ("why") and, where the straight-line
  * kernels of a large mechanism are missing too, theirs ("wide_why"). */
 rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info, size_t info_len);
 /* Staging of the mixed-precision transport pencils (no reference counterpart).  Beside the

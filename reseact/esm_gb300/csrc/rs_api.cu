@@ -2080,13 +2080,15 @@ extern "C" rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info,
       char line[1024];
       if (h->jit) {
         const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
-        const int v = h->jit->variant;
+        const int v = rs::jit_variant(*h->jit, (int)h->nc, true), v1 = rs::jit_variant(*h->jit, (int)h->nc, false);
         std::snprintf(line, sizeof line,
-                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"runs\": \"%s\", \"runs_regs\": %d, \"runs_smem_bytes\": %zu, "
+                      "{\"kind\": \"%s\", \"variant\": \"%s\", \"runs\": \"%s\", \"runs_single\": \"%s\", "
+                      "\"runs_regs\": %d, \"runs_smem_bytes\": %zu, "
                       "\"regs\": [%d, %d, %d, %d], "
                       "\"smem_bytes\": %zu, \"split_smem_bytes\": %zu, \"compile_ms\": %.1f}",
                       spec ? "specialized" : "table", rs::kJitVariantNames[v],
                       !spec ? "table" : (f64 ? "fp64_norm" : rs::kJitVariantNames[v]),
+                      !spec ? "table" : (f64 ? "fp64_norm" : rs::kJitVariantNames[v1]),
                       !spec ? 0 : (f64 ? h->jit->fp64_norm_regs : h->jit->regs[v]),
                       !spec || f64 ? (size_t)0 : rs::jit_attempt_smem(*h->jit, v, (int)h->nc),
                       h->jit->regs[0], h->jit->regs[1], h->jit->regs[2], h->jit->regs[3],
@@ -2137,7 +2139,7 @@ extern "C" rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t 
     else if (k == "per_cell_wide") ok = in({0, 1}) && (value == 0 || (h->wide && h->wide->per_cell)) && (t.pc_wide = value, true);
     else if (k == "chem_attempt_variant") {  // the specialised attempt kernel's variant
       ok = value >= 0 && value < rs::kJitVariants && h->jit && h->jit->attempt[value][0];
-      if (ok) h->jit->variant = value;
+      if (ok) h->jit->variant = value, h->jit->chosen = true;
     }
     else if (k == "per_cell_group") {
       // G lanes per cell: the production build's (minimum-fill, descending back substitution)
@@ -2574,6 +2576,8 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
       // runs whatever is set, there is nothing to choose: its one time stands for all of them.
       const bool f64 = rs::jit_fp64_norm(*h->jit, (int)h->nc, h->cfg.rtol_C, h->cfg.atol_C);
       const int was = h->jit->variant;
+      const bool was_chosen = h->jit->chosen;
+      h->jit->chosen = true;  // the ones timed, then the one picked
       Ctl init = make_ctl(h, 0.0, 600.0, 60.0, h->cfg.ctrl_C, (double)h->nc * h->nsp);
       init.cur = h->cur;
       Ctl* c = h->ctl.p + 2;
@@ -2602,6 +2606,7 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
         }
       }
       h->jit->variant = pick;
+      h->jit->chosen = !f64 || was_chosen;
       std::snprintf(line, sizeof line, "], \"chem_choice\": \"%s\"", rs::kJitVariantNames[pick]);
       rep += line;
       invalidate_graphs(h);

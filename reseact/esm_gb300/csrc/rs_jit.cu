@@ -1747,6 +1747,17 @@ size_t jit_attempt_smem(const JitChem& J, int variant, int nc) {
   return J.attempt_smem[variant] / kBlock * jit_attempt_block(nc);
 }
 
+// Until a variant is picked, attempts of the loop keep W in registers: the fastest or within 1 % of it
+// on every grid (600 s of chemistry in ms, regs / smem / regs2 / split: 76,183 cells 2.90 / 2.89 /
+// 3.07 / 3.58; 133,517: 4.43 / 4.37 / 4.96 / 4.67; 211,200: 6.64 / 6.72 / 7.10 / 6.85; 615,888: 17.08 /
+// 17.08 / 17.45 / 17.06).  A single attempt evaluates f(x) as well and starts alone; above 2^18 cells
+// 128 registers and 16 warps per SM ("regs2") are faster there (us per call, regs / regs2: 211,200
+// cells 361 / 369, 294,840: 526 / 510, 437,710: 748 / 713, 615,888: 1,006 / 969, 960,000: 1,533 / 1,483).
+int jit_variant(const JitChem& J, int nc, bool reuse) {
+  if (J.chosen) return J.attempt[J.variant][0] ? J.variant : 0;
+  return !reuse && nc > (1 << 18) && J.attempt[2][0] ? 2 : 0;
+}
+
 // Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set (the
 // strict build has no other norm and runs the variant that is set):
 // - up to one warp per SM sub-partition (152 SMs, four each), where its time is its FP64 chain (6,480
@@ -1766,7 +1777,7 @@ void jit_launch_attempt(const JitChem& J, cudaStream_t st, int nc, int nsp, cons
                         double* U0, double* U1, const double* kr, const double* em,
                         double* part, double rtol, double atol, int clamp, double* F0,
                         double* F1) {
-  const int v = J.attempt[J.variant][0] ? J.variant : 0;
+  const int v = jit_variant(J, nc, F0 && F1);
   const bool fp64 = jit_fp64_norm(J, nc, rtol, atol) || (J.fp64_norm[0] && U0 == U1);
   cudaKernel_t k = fp64 ? J.fp64_norm[em ? 1 : 0] : J.attempt[v][em ? 1 : 0];
   const unsigned char* c = reinterpret_cast<const unsigned char*>(ctl);

@@ -40,11 +40,8 @@ struct JitChem {
   cudaKernel_t step[2] = {};                   // accepted step, no error estimate [has emission]
   cudaKernel_t vjpk[2] = {};                   // step VJP reading k1, z2 from the stage tape
   size_t attempt_smem[kJitVariants] = {};  // dynamic shared bytes of each attempt variant, 256 threads
-  // variant used for global-dt attempts: "regs" until the autotuner or the caller picks one.  It is
-  // the fastest or within 1 % of it on every grid (600 s of chemistry in ms, regs / smem / regs2 /
-  // split: 76,183 cells 2.90 / 2.89 / 3.07 / 3.58; 133,517: 4.43 / 4.37 / 4.96 / 4.67; 211,200: 6.64 /
-  // 6.72 / 7.10 / 6.85; 615,888: 17.08 / 17.08 / 17.45 / 17.06)
-  int variant = 0;
+  int variant = 0;      // variant used for global-dt attempts ...
+  bool chosen = false;  // ... where the autotuner or the caller picked it, else jit_variant's
   double compile_ms = 0;    // NVRTC time (0 when the compiled image came from cache)
   int regs[kJitVariants] = {};  // registers per thread of each attempt variant
 };
@@ -68,6 +65,9 @@ bool jit_compile(const std::string& src, bool strict, bool verbose, std::vector<
 
 // Threads per block of the attempt kernels over nc cells (one partial sum per block).
 int jit_attempt_block(int nc);
+// The variant that attempts over nc cells run: the picked one, or the grid's.  reuse: attempts of the
+// adaptive loop, which keep f(x) from one to the next; false: a single attempt.
+int jit_variant(const JitChem& J, int nc, bool reuse);
 // Dynamic shared bytes per block of a variant over nc cells.
 size_t jit_attempt_smem(const JitChem& J, int variant, int nc);
 // Whether attempts run the form with the FP64 norm, whatever variant is set.

@@ -78,6 +78,17 @@ def test_a_handle_starts_with_w_in_registers(n):
     s.close()
 
 
+@pytest.mark.parametrize("n,single", [((64, 64, 64), "regs"), ((72, 64, 64), "regs2")])
+def test_single_attempts_of_large_grids(n, single):
+    s = Solver.for_workload(_work(n), do_transport=False)
+    info = s.chem_kernel()[1]
+    assert info["runs"] == "regs" and info["runs_single"] == single
+    s.set_launch_shape(chem_attempt_variant=3)  # a picked variant serves both
+    info = s.chem_kernel()[1]
+    assert info["runs"] == info["runs_single"] == info["variant"] == "split"
+    s.close()
+
+
 def test_small_grid_says_what_runs():
     w = _work(SMALL)
     s = Solver.for_workload(w)
