@@ -2550,16 +2550,19 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
                                    h->have_emis ? h->emis.p : nullptr, h->io.p, nullptr, h->queue.p,
                                    h->flag.p, a);
         });
-        // Three attempts of every cell show what a full device does; a window ends with its slowest
-        // cells, whose attempts several lanes finish sooner the emptier the device is (the
-        // straight-line kernel's last cell takes as long as its first).  So where lanes per cell win
-        // among the table-walking kernels, batches below 50 cells per SM keep them.  60 s windows of
-        // 30 / 44 / 64 species in ms, straight-line against lanes per cell: 1,024 cells 8.6 / 19.6 /
-        // 27.4 against 6.0 / 10.1 / 18.6, 4,096: 9.5 / 19.6 / 52.1 against 7.9 / 15.6 / 42.3; 8,192:
-        // 9.9 / 21.5 / 55.5 against 11.9 / 26.0 / 52.8, 16,384: 11.8 / 26.8 / 49.3 against 19.9 / 47.2 /
-        // 58.7.  At 262,144 cells 88 / 222 / 279 against 151 / 306 / 521 of the best table kernel.
+        // Three attempts of every cell are not a window, whose cells take uneven numbers of steps, in two
+        // ways.  (1) A table-walking warp runs as long as its slowest cell, which the probe does not show:
+        // 60 s windows of 30 / 44 / 64 species, straight-line / best table kernel, 262,144 cells 88 / 149,
+        // 222 / 307, 280 / 529 ms (probe 5.8 / 7.1, 12.2 / 14.4, 10.6 / 12.6); 1,048,576 cells 306 / 407,
+        // 862 / 865, 931 / 1,060 (probe 27.9 / 27.7, 62.2 / 54.8, 55.0 / 47.4).  So the probe may be up to a
+        // quarter behind.  (2) The window ends with its slowest cells, whose attempts several lanes finish
+        // sooner the emptier the device is (the straight-line kernel's last cell takes as long as its
+        // first): where lanes per cell win among the table-walking kernels, batches below 50 cells per SM
+        // keep them.  1,024 cells 8.6 / 19.6 / 27.4 ms straight-line against 6.0 / 10.1 / 18.6 by lanes,
+        // 4,096: 9.5 / 19.6 / 52.1 against 7.9 / 15.6 / 42.3; 8,192: 9.9 / 21.5 / 55.5 against 11.9 / 26.0 /
+        // 52.8, 16,384: 11.8 / 26.8 / 49.3 against 19.9 / 47.2 / 58.7.
         const bool few = (long long)h->nc < 50LL * nsm && h->tune.pc_group > 0;
-        h->tune.pc_wide = !few && ms < best;
+        h->tune.pc_wide = !few && ms < 1.25f * best;
         std::snprintf(line, sizeof line, "], \"per_cell_wide\": [{\"ms\": %.4f}", ms);
         rep += line;
       }
@@ -2843,7 +2846,7 @@ extern "C" rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len) {
 // chemistry: a host that runs its own memory pool (a Julia CUDA.jl or PyTorch caching
 // allocator that has already reserved the device), or a latency-critical loop where an
 // allocation would synchronise the device.  rs_ros23_attempt_noalloc serves them: its
-// scratch (the 256-cell partial sums of the error norm and the controller record) lives in
+// scratch (the block partial sums of the error norm and the controller record) lives in
 // one file-scope device array that every GPU loading this library holds until exit.
 namespace {
 
