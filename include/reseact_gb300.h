@@ -64,8 +64,10 @@ typedef enum rs_status {
 /* lateral boundary kinds */
 enum { RS_BC_PERIODIC = 0, RS_BC_OPEN = 1, RS_BC_CLOSED = 2 };
 /* arithmetic of the transport half: FP64, or MIXED = compensated FP32 (the PPM reconstruction
- * and face terms in double-float pairs on the FP32 pipe, about 48 significant bits; the state,
- * air mass, stage updates and error norm in FP64) */
+ * and face terms, the stage updates and the error norm in double-float pairs on the FP32 pipe, about
+ * 48 significant bits; the state and the air mass in FP64).  The error norms of the FP64 forms are
+ * summed in such pairs too where their range holds the values, in FP64 elsewhere: they differ from the
+ * FP64 sum by less than 1e-11 and steer the step size only. */
 enum { RS_PREC_FP64 = 0, RS_PREC_MIXED = 1 };
 /* chemistry step-size control: one global dt (reference) or per-cell adaptive substeps */
 enum { RS_CHEM_GLOBAL_DT = 0, RS_CHEM_PER_CELL = 1 };
@@ -262,10 +264,10 @@ rs_status rs_autotune(rs_handle* h, char* buf, size_t buf_len);
  * table-walking per-cell kernel at 32 registers), "per_cell_wide" (1: the straight-line per-cell
  * kernel of a large mechanism, where built; the other per-cell keys select the table-walking
  * kernels); "chem_attempt_variant" (0 "regs", 1 "smem",
- * 2 "regs2", 3 "split": how the specialised attempt kernel keeps W, where built; in the production build
- * the choice counts for grids above 19,456 cells and tolerances atol_C 2^-40 .. 2^100, rtol_C 2^-60 .. 2^60, and
- * all others run one form with an FP64 error norm, "fp64_norm").  Values outside a key's
- * candidates are RS_ERR_INVALID.  Every shape gives bit-identical results. */
+ * 2 "regs2", 3 "split": how the specialised attempt kernel keeps W, where built; in the production build,
+ * mechanisms of up to 108 LU slots follow it on grids above 19,456 cells at tolerances atol_C 2^-40 ..
+ * 2^100 and rtol_C 2^-60 .. 2^60, and run one form with an FP64 error norm, "fp64_norm", elsewhere).
+ * Values outside a key's candidates are RS_ERR_INVALID.  Every shape gives bit-identical results. */
 rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
 
 /* Chemistry kernel selection (no reference counterpart; the reference compiles its RHS and
@@ -283,9 +285,10 @@ rs_status rs_set_launch_shape(rs_handle* h, const char* key, int32_t value);
 enum { RS_CHEM_KERNEL_AUTO = 0, RS_CHEM_KERNEL_TABLE = 1, RS_CHEM_KERNEL_SPECIALIZED = 2 };
 rs_status rs_set_chem_kernel(rs_handle* h, int32_t kind);
 /* The kernel kind in use (TABLE or SPECIALIZED) and a one-line JSON description of it: of a specialised
- * kernel the variant that is set ("variant"), the form that attempts of the adaptive loop run ("runs", "runs_regs",
- * "runs_smem_bytes" per block) and the one of single attempts ("runs_single"); without one the reason ("why") and, where the straight-line
- * kernels of a large mechanism are missing too, theirs ("wide_why"). */
+ * kernel the variant that is set ("variant"), the form that attempts of the adaptive loop run ("runs",
+ * "runs_regs", "runs_smem_bytes" per block) and the one of single attempts ("runs_single"); without
+ * one the reason ("why") and, where the straight-line kernels of a large mechanism are missing too,
+ * theirs ("wide_why"). */
 rs_status rs_get_chem_kernel(rs_handle* h, int32_t* kind, char* info, size_t info_len);
 /* Staging of the mixed-precision transport pencils (no reference counterpart).  Beside the
  * pencils, the mixed transport has streaming forms without shared memory (a warp of shuffles

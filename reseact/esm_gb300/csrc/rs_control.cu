@@ -1,6 +1,6 @@
 // rs_control.cu -- device-resident step-size control and layout kernels.
 //
-// k_finalize closes one attempt: level-2 fixed-tree sum of the 256-cell partials, the hairer
+// k_finalize closes one attempt: sum of the attempt's block partials in a fixed order, the hairer
 // norm EEst = sqrt(sse/N) (rx_traced_integrator.jl:347,398), then the PI controller exactly as
 // adaptive_solve's loop body (rx_traced_integrator.jl:480-505): NaN -> reject, q11 = EEst^b1,
 // q = q11/qold^b2 clamped to [1/qmax, 1/qmin] after /gamma, accept iff EEst <= 1 with the

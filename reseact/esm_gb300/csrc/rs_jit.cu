@@ -95,7 +95,7 @@ std::string lit(double v) {  // exact hex-float literal
   return std::signbit(v) ? "(" + std::string(b) + ")" : std::string(b);
 }
 
-// W storage: shared-memory variant only while NLU doubles per thread x 256 threads fit
+// W storage: shared-memory variant only while NLU doubles per thread fit for the largest block
 constexpr int kBlock = 256;
 constexpr int kJitUnits = 8;  // RS_IN units of the generated source
 constexpr size_t kSmemCap = 227 * 1024 - kBlock * sizeof(double);
@@ -1205,7 +1205,7 @@ extern "C" __global__ void rs_jit_rcp(const double* __restrict__ x, double* __re
 // What they gain is the table walk itself (an index load in front of every operand) and where the
 // work arrays live.  FP64 issues one warp instruction per 64 cycles and SM sub-partition, so two
 // warps per sub-partition (one 256-thread block per SM) are enough, and at that occupancy
-//   - the least-used LU slots of W, 112 of them, sit in shared memory ([slot][thread]) and the
+//   - the least-used LU slots of W, 111 of them, sit in shared memory ([slot][thread]) and the
 //     others in registers or their spills: volatile accesses and compiler barriers keep the
 //     compiler from promoting shared slots to registers and spilling those;
 //   - f, the partials and the Jacobian are formed reaction by reaction (each sum still adds its
@@ -1213,7 +1213,9 @@ extern "C" __global__ void rs_jit_rcp(const double* __restrict__ x, double* __re
 //   - rate constants are loaded in groups one group ahead.
 // 30 species, 60 reactions, 290 slots (3,400 FP64 instructions an attempt, 5.4 ns per cell at the
 // FP64 pipe's rate): 12.4 -> 6.8 ns per cell-attempt against k_ros23_attempt (128 threads per SM
-// with 226 shared slots: 7.4 ns; W in registers and spills alone: 8.4 ns).
+// with 226 shared slots: 7.4 ns; W in registers and spills alone: 8.4 ns).  It holds to the largest
+// accepted: 44 species 3.72 -> 1.99 ms per attempt on 155,648 cells, 64 species 3.26 -> 1.83, rs_create
+// 2.8 s.
 constexpr int kWideSlots = (int)((227 * 1024 - 2 * kBlock * sizeof(double)) / (kBlock * sizeof(double)));
 
 bool wide_eligible(const MechTables& T) {
@@ -1759,7 +1761,7 @@ int jit_variant(const JitChem& J, int nc, bool reuse) {
 }
 
 // Where the attempt forms its error norm in FP64, with W in registers, whatever variant is set (the
-// strict build has no other norm and runs the variant that is set):
+// strict build and mechanisms beyond kPairSlots have no other norm and run the variant that is set):
 // - up to one warp per SM sub-partition (152 SMs, four each), where its time is its FP64 chain (6,480
 //   cells: 40 us per attempt, 45 with the float-pair norm); beyond, the pairs win (615,888 cells:
 //   1,070 us with the FP64 norm, 981 with pairs, both with 128 registers);

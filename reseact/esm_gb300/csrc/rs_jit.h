@@ -22,11 +22,12 @@ namespace rs {
 struct PerCellArgs;
 
 // Variants of the global-dt attempt kernel (the autotuner picks one by timing):
-//   0 "regs"   W in registers (spilled by ptxas where needed), one 256-thread block per SM
+//   0 "regs"   W in registers (spilled by ptxas where needed), 256 threads per SM
 //   1 "smem"   W in dynamic shared memory, [slot][thread] so a warp's accesses are contiguous
-//   2 "regs2"  as 0 but capped at 128 registers for two blocks per SM
+//   2 "regs2"  as 0 but capped at 128 registers for 512 threads per SM
 //   3 "split"  the last half of W's LU slots (at most 55) in shared memory, the rest in
-//              registers, capped at 128 registers for two blocks per SM
+//              registers, capped at 128 registers for 512 threads per SM
+// in blocks of jit_attempt_block threads.
 constexpr int kJitVariants = 4;
 extern const char* const kJitVariantNames[kJitVariants];
 

@@ -383,8 +383,7 @@ __global__ void __launch_bounds__(256) k_flux_x_fused(DevTransport<double> T, St
   double* V = smx;            // V[p+3], p in [-3, n+2]
   double* Dd = smx + L;       // Dd[p+3] = v(p+1) - v(p), p in [-3, n+1]
   double* D = smx + 2 * L;    // D[p+3], slopes p in [-2, n+1]
-  double* E = smx + 3 * L;    // strict: E[f+3], edge between f-1 and f, f in [-1, n+1];
-                              // production: E[p+3] = 6 x right-edge deviation of cell p
+  double* E = smx + 3 * L;    // E[f+3], edge between f-1 and f, f in [-1, n+1]
   double* Mf = smx + 4 * L;   // Mf[f], the face's air-mass flux g*mx (shared by all tracers)
   const int row = blockIdx.x;  // (k, j)
   const int j = row % T.nlat, k = row / T.nlat;
@@ -584,8 +583,8 @@ __global__ void __launch_bounds__(512) k_flux_z_fused(DevTransport<double> T, St
 // (three FP32 operations), so they ride the FP32 pipe too.
 //
 // Each direction adds its part into a per-cell pair accumulator (x writes it, y and z add), and
-// the stage kernel turns it into the stage update.  The state, the air mass and the error
-// control stay FP64.
+// the stage kernel turns it into the stage update, whose error norm is formed in pairs as well.  The
+// state, the air mass and the step-size control stay FP64.
 //
 // What bounds it: issue slots and the FP32 / integer pipes.  Packed f32x2 operations do two
 // tracers per instruction at the scalar rate of flops, so the streaming kernels carry a pair of
@@ -1530,8 +1529,8 @@ __global__ void __launch_bounds__(kLine32, kLineBlocks) k_adv_yz_stream(DevTrans
 // hi + lo split without FP64-pipe conversions (production build): hi = v rounded to 24
 // significant bits, lo = the remainder rounded to 24 -- hi + lo = v to 2^-49 relative, without
 // bias, and |lo| <= ulp(hi) / 2 as the sums of pairs expect.  (Truncating both, the error of every
-// state had the sign of the state and lo was up to a whole ulp: one transport step 3.8e-15 rms and
-// 2.1e-14 at most, now 1.8e-15 and 1.3e-14.)  Values outside [2^-74, 2^126) (zero, subnormals, inf,
+// state had the sign of the state and lo was up to a whole ulp: one transport step was off by 5.3e-16
+// rms of a tracer's largest value and 2.7e-14 of each value at most, now 3.1e-16 and 1.4e-14.)  Values outside [2^-74, 2^126) (zero, subnormals, inf,
 // NaN included) convert.
 __device__ __forceinline__ void split_bits(double v, float& hi, float& lo) {
   const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
