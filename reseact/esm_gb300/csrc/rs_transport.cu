@@ -1530,8 +1530,8 @@ __global__ void __launch_bounds__(kLine32, kLineBlocks) k_adv_yz_stream(DevTrans
 // significant bits, lo = the remainder rounded to 24 -- hi + lo = v to 2^-49 relative, without
 // bias, and |lo| <= ulp(hi) / 2 as the sums of pairs expect.  (Truncating both, the error of every
 // state had the sign of the state and lo was up to a whole ulp: one transport step was off by 5.3e-16
-// rms of a tracer's largest value and 2.7e-14 of each value at most, now 3.1e-16 and 1.4e-14.)  Values outside [2^-74, 2^126) (zero, subnormals, inf,
-// NaN included) convert.
+// rms of a tracer's largest value and 2.7e-14 of each value at most, now 3.1e-16 and 1.4e-14.)
+// Values outside [2^-74, 2^126) (zero, subnormals, inf, NaN included) convert.
 __device__ __forceinline__ void split_bits(double v, float& hi, float& lo) {
   const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
   const int e = (int)((h >> 20) & 0x7ff);
