@@ -783,14 +783,13 @@ __device__ __forceinline__ double ros23_cell(const double* __restrict__ kr,
     o << R"(#undef pair_msub
 #undef pair_scale
   fp2 sum = {0.0f, 0.0f};
-  bool fits = true;  // no square beyond FP32, and no overflow on the way: that leaves a NaN here
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     const fp2 q = pair_div(fp2{eh[s], el[s]}, fp2{dh[s], dl[s]});
-    fits = fits && fabsf(q.h) < 0x1p60f;
     sum = pair_add(sum, pair_mul(q, q));
   }
-  return fits && big < kPairBig ? pair_to_d(sum) * (dto6 * dto6) : -1.0;
+  // a square beyond FP32, or an overflow on the way, leaves an infinity or a NaN in the sum
+  return fabsf(sum.h) < 0x1p126f && big < kPairBig ? pair_to_d(sum) * (dto6 * dto6) : -1.0;
   } else {
 )" << store_un;
     g.lu_solve("b");
